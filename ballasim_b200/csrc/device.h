@@ -102,6 +102,7 @@ struct EngineSensor {
   uint32_t width, height;
   uint32_t tiles_x, tiles_y;
   uint32_t tile0;      // first global tile of the sensor
+  uint32_t blob0;      // first of the sensor's blobs among all sensors' (the split engine's boxes)
   EventBuf ev;         // the sensor's own event buffer and counters
   unsigned long long* counters;
 };
@@ -168,16 +169,20 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
                    int32_t w0, int32_t w1, const SamplerRules& r, unsigned int* tile_counter, int blocks,
                    int warps_per_block, int stage, int tile_lw, int cascade, cudaStream_t stream);
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
-// The split engine (stage kStageSplit): window w as engine_window_kernel (blocks x warps_per_block warps, persistent
-// over the tiles) then engine_rest_kernel (rest_blocks x 128 threads) over the pixels the first posted to `rest`
-// (rest_capacity records of rest_record_bytes(); *rest_count and *tile_counter zero before the launch).
+// The split engine (stage kStageSplit): split_begin_kernel, then per window split_window_kernel (blocks x
+// warps_per_block warps over the tiles) and split_rest_kernel (rest_blocks x 128 threads) over the pixels that the first
+// posted to `rest` (rest_capacity records of split_record_bytes(); rest_counts: a word per window, zero before the
+// launch), and split_end_kernel. The state passes from S.in to S.out (carried_in to carried_out). tile0: the sensors'
+// first tiles (host memory); scratch: split_scratch_bytes(), 128-byte aligned.
 constexpr int kStageSplit = 1;
-void launch_engine_split(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
-                         int32_t w, const SamplerRules& r, unsigned int* tile_counter, void* rest, unsigned int* rest_count,
-                         unsigned int rest_capacity, int blocks, int warps_per_block, int tile_lw, int rest_blocks,
-                         cudaStream_t stream);
-size_t rest_record_bytes();
-int engine_rest_blocks_per_sm();
+size_t split_scratch_bytes(uint32_t total_tiles, uint32_t total_blobs);
+size_t split_record_bytes();
+void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,
+                         uint32_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
+                         void* rest, unsigned int* rest_counts, unsigned int rest_capacity, int blocks,
+                         int warps_per_block, int tile_lw, int rest_blocks, cudaStream_t stream);
+int split_window_blocks_per_sm(int warps_per_block);
+int split_rest_blocks_per_sm();
 // The fused engine with the learned step proposal (BF16 MLP operands and FP32 parameters in device memory):
 // the same tiles and pixel model, each window sampled by proposed power-of-two steps judged by the plain rule.
 // rec_samples / rec_steps (capacity 0: off) record every sample and every proposed step.

@@ -24,6 +24,10 @@ struct FieldDev {
   float base, amp, nx, ny, c, speed, width_px;
   int32_t n_blobs;
   const float* blobs;  // device memory, n_blobs x kBlobWords
+  // Set by field_bounds: no value of the field lies outside [lo, hi]; listable: at most 65,535 blobs, each term's
+  // exponent in [-80, 0].
+  float lo, hi;
+  int32_t listable;
 };
 
 // The candidate blobs of one warp and window (indices in blob order), or all blobs (idx null).
@@ -31,6 +35,41 @@ struct BlobList {
   const uint16_t* idx;
   int32_t n;
 };
+
+// Bounds of the field's values over all pixels and times, from the parameters and the blob table in host memory: the
+// base with every term of either sign, widened by the sums' rounding (a blob term lies between 0 and its
+// amplitude, tanh between -1 and 1). Parameters that are not finite give the widest bounds.
+inline void field_bounds(FieldDev& f, const float* blobs_host) {
+  double lo = f.base, hi = f.base, mag = lo < 0 ? -lo : lo;
+  const auto span = [&](double below, double above) {
+    lo -= below;
+    hi += above;
+    mag += below + above;
+  };
+  f.listable = f.n_blobs <= 65535 ? 1 : 0;
+  if (f.kind == kFieldTanhEdge) {
+    const double a = f.amp < 0 ? -f.amp : f.amp;
+    span(a, a);
+  } else {
+    bool negative = false;
+    for (int32_t k = 0; k < f.n_blobs; ++k) {
+      const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
+      negative = negative || !(b[0] >= 0.0f);
+      span(b[0] < 0.0f ? -b[0] : 0.0f, b[0] > 0.0f ? b[0] : 0.0f);
+      if (!(b[5] >= 0.0f && b[5] * b[6] <= 79.0f)) f.listable = 0;
+    }
+    if (!negative) mag = 0.0;  // adding terms >= 0 never rounds below the base
+  }
+  const double rounding = 1e-7 * (64.0 + f.n_blobs);  // each sum rounds by at most 2^-24 of the terms so far
+  lo -= rounding * mag;
+  hi += rounding * (mag + hi);
+  if (!(lo > -3e38 && hi < 3e38 && mag < 3e38)) {
+    lo = -3e38;
+    hi = 3e38;
+  }
+  f.lo = static_cast<float>(lo);
+  f.hi = static_cast<float>(hi);
+}
 
 BS_HD float t_seconds(int64_t t_ns) { return static_cast<float>(static_cast<double>(t_ns) * 1e-9); }
 

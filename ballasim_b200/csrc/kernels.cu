@@ -6,155 +6,11 @@
 //
 // Events leave through warp-aggregated atomics: the lanes that emit together take one slot range with one atomic
 // (coalesced group rank), and a call whose events exceed the buffer is re-run from its unchanged input state.
-#include <cooperative_groups.h>
-
-#include "device.h"
-
-namespace cg = cooperative_groups;
+#include "engine_dev.cuh"
 
 namespace bs {
 
 namespace {
-
-// Appends events to one sensor's buffer; the lanes of a warp that push together share one atomic, so every lane of
-// the warp must push to the same buffer (a warp works on one tile of one sensor).
-struct GlobalSink {
-  EventBuf ev;
-  unsigned long long* count;
-  __device__ __forceinline__ void push(const RawEvent& e) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(count, static_cast<unsigned long long>(g.size()));
-    base = g.shfl(base, 0);
-    const unsigned long long i = base + g.thread_rank();
-    if (i < ev.capacity) {
-      const uint4* src = reinterpret_cast<const uint4*>(&e);
-      uint4* dst = reinterpret_cast<uint4*>(ev.data + i);
-      dst[0] = src[0];
-      dst[1] = src[1];
-    }
-  }
-};
-
-// Appends each event with the pushing thread's own atomic: for a kernel whose lanes serve pixels of different
-// sensors (engine_rest_kernel).
-struct ThreadSink {
-  EventBuf ev;
-  unsigned long long* count;
-  __device__ __forceinline__ void push(const RawEvent& e) {
-    const unsigned long long i = atomicAdd(count, 1ull);
-    if (i < ev.capacity) {
-      const uint4* src = reinterpret_cast<const uint4*>(&e);
-      uint4* dst = reinterpret_cast<uint4*>(ev.data + i);
-      dst[0] = src[0];
-      dst[1] = src[1];
-    }
-  }
-};
-
-__device__ __forceinline__ void load_state(const StateSoA& a, uint32_t p, bool noise, PixelRegs& s) {
-  s.t_ref = a.t_ref[p];
-  s.t_search = a.t_search[p];
-  s.blind_until = a.blind_until[p];
-  s.s3_ref = a.s3_ref[p];
-  s.n3_ref = a.n3_ref[p];
-  s.dr_ref = a.dr_ref[p];
-  s.i_scale = a.i_scale[p];
-  s.held = a.held[p];
-  s.flags = a.flags[p];
-  if (noise) {
-    s.t_shot = a.t_shot[p];
-    s.t_ba = a.t_ba[p];
-    s.n_shot = a.n_shot[p];
-    s.n_ba = a.n_ba[p];
-  } else {
-    s.t_shot = s.t_ba = kForever;
-    s.n_shot = s.n_ba = 0;
-  }
-}
-
-__device__ __forceinline__ void store_state(const StateSoA& a, uint32_t p, bool noise, const PixelRegs& s) {
-  a.t_ref[p] = s.t_ref;
-  a.t_search[p] = s.t_search;
-  a.blind_until[p] = s.blind_until;
-  a.s3_ref[p] = s.s3_ref;
-  a.n3_ref[p] = s.n3_ref;
-  a.dr_ref[p] = s.dr_ref;
-  a.i_scale[p] = s.i_scale;
-  a.held[p] = s.held;
-  a.flags[p] = s.flags;
-  if (noise) {
-    a.t_shot[p] = s.t_shot;
-    a.t_ba[p] = s.t_ba;
-    a.n_shot[p] = s.n_shot;
-    a.n_ba[p] = s.n_ba;
-  }
-}
-
-__device__ __forceinline__ void load_cascade(const StateSoA& a, uint32_t p, CascadeRegs& q) {
-  q.z = a.z[p];
-  q.x1 = a.x1[p];
-  q.s2 = a.s2[p];
-  q.s3 = a.s3[p];
-  q.tv = a.tv[p];
-}
-
-__device__ __forceinline__ void store_cascade(const StateSoA& a, uint32_t p, const CascadeRegs& q) {
-  a.z[p] = q.z;
-  a.x1[p] = q.x1;
-  a.s2[p] = q.s2;
-  a.s3[p] = q.s3;
-  a.tv[p] = q.tv;
-}
-
-__device__ __forceinline__ void load_lattice(const StateSoA& a, uint32_t p, uint32_t n, LatticeRegs& L) {
-  for (int i = 0; i < 3; ++i) {
-    L.nk[i] = a.lat[static_cast<size_t>(i) * n + p];
-    L.nk1[i] = a.lat[static_cast<size_t>(3 + i) * n + p];
-  }
-  L.ln_a1 = a.lat[static_cast<size_t>(6) * n + p];
-  L.rho = a.lat[static_cast<size_t>(7) * n + p];
-  L.cell = a.cell[p];
-  L.have_k1 = a.have_k1[p];
-}
-
-__device__ __forceinline__ void store_lattice(const StateSoA& a, uint32_t p, uint32_t n, const LatticeRegs& L) {
-  for (int i = 0; i < 3; ++i) {
-    a.lat[static_cast<size_t>(i) * n + p] = L.nk[i];
-    a.lat[static_cast<size_t>(3 + i) * n + p] = L.nk1[i];
-  }
-  a.lat[static_cast<size_t>(6) * n + p] = L.ln_a1;
-  a.lat[static_cast<size_t>(7) * n + p] = L.rho;
-  a.cell[p] = L.cell;
-  a.have_k1[p] = L.have_k1;
-}
-
-// Drops events (the init of the noise lattice fires nothing).
-struct NullSink {
-  __device__ void push(const RawEvent&) {}
-};
-
-__device__ __forceinline__ void load_map(const MapSoA& m, uint32_t p, PixelMapRegs& r) {
-  r.theta_on = m.theta_on[p];
-  r.theta_off = m.theta_off[p];
-  r.leak = m.leak[p];
-  r.dark = m.dark[p];
-  r.scale = m.scale[p];
-  r.ba_rate_hz = m.ba_rate[p];
-  r.shot_max_hz = m.shot_max[p];
-}
-
-// Sums a value over the warp and adds it to a counter from lane 0 (all 32 lanes must call).
-__device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0 && v != 0ull) atomicAdd(dst, v);
-}
-__device__ __forceinline__ void warp_or(unsigned long long* dst, unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0 && v != 0ull) atomicOr(dst, v);
-}
 
 // ---------------------------------------------------------------------------------------------
 // init
@@ -406,185 +262,6 @@ __device__ __forceinline__ PixelMapRegs shfl_map(const PixelMapRegs& m, int src)
   o.ba_rate_hz = __shfl_sync(full, m.ba_rate_hz, src);
   o.shot_max_hz = __shfl_sync(full, m.shot_max_hz, src);
   return o;
-}
-
-// Would PixelProc::segment_fast pass segment [t0, e) with nothing but its clean effects (the piece counted, the
-// search moved to e, a node counted when e - t0 > 2)? Only where it takes that branch: one 2^23 ns piece, the pixel
-// not blind, its search armed at or before t0, no noise candidate before e, Delta(t0) below both levels, and the
-// node (t0, e - 1] a single integer or excluded. Inline code on the caller's registers.
-__device__ __forceinline__ bool clean_segment(const PixelRegs& s, const PixelMapRegs& m, const SensorConsts& k,
-                                              int64_t t0, int64_t e, float v0, float v1, float x0, float x1) {
-  if (((e - 1) >> kWindowLog2) != (t0 >> kWindowLog2)) return false;
-  if (s.blind_until != kNotBlind || s.t_search > t0) return false;
-  const int64_t tn = k.noise ? mini(s.t_shot, s.t_ba) : kForever;
-  if (tn < e) return false;
-  NullSink ns;
-  PixelCounters nc;
-  const PixelProc<NullSink> hp{const_cast<PixelRegs&>(s), m, k, 0u, ns, nc};
-  const float D0 = hp.delta(t0, x0);
-  if (D0 >= m.theta_on || D0 <= -m.theta_off) return false;
-  if (e - t0 == 1) return true;
-  return hp.excluded(Segment{t0, e, v0, v1}, t0, e, x0, x1);
-}
-
-// clean_segment's other case, for a segment it refused: the search armed after t0 (the first segment after init, or
-// the segment of an event), where PixelProc::piece searches [t_search, e) alone, without Delta(t0); clean when
-// nothing is left to search or the node (t0, e - 1] around it is excluded (the same effects).
-__device__ __forceinline__ bool clean_after_start(const PixelRegs& s, const PixelMapRegs& m, const SensorConsts& k,
-                                                  int64_t t0, int64_t e, float v0, float v1, float x0, float x1) {
-  if (((e - 1) >> kWindowLog2) != (t0 >> kWindowLog2)) return false;
-  if (s.blind_until != kNotBlind || s.t_search <= t0) return false;
-  const int64_t tn = k.noise ? mini(s.t_shot, s.t_ba) : kForever;
-  if (tn < e) return false;
-  if (s.t_search >= e) return true;
-  NullSink ns;
-  PixelCounters nc;
-  const PixelProc<NullSink> hp{const_cast<PixelRegs&>(s), m, k, 0u, ns, nc};
-  return hp.excluded(Segment{t0, e, v0, v1}, t0, e, x0, x1);
-}
-
-// The noise candidates of a stretch [t_from, t_end) of every lane's pixel, computed with all 32 lanes together.
-// A candidate that thinning rejects changes nothing but its chain (PixelProc::noise_candidate), and its acceptance
-// depends only on its draw and the irradiance at its time, which the stretch's samples give: so each lane's chains
-// move past their rejected candidates here, and stop at their first accepted candidate in the stretch (or at their
-// first candidate after it). The pixel model then meets only accepted candidates, at which it runs its own noise
-// path (the draw and the thinning test again, the refractory drop, the event) and follows the chains from there as
-// usual. Events and the chains' end state are those of the pixel model meeting every candidate; only the count of
-// the crossing search's nodes differs, since the search is no longer cut at rejected candidates (the first crossing
-// is the same: a time-ordered search over [lo, e) finds what searches over [lo, tn) then [tn, e) find).
-// active: this lane's stretch is in `run` (run.n samples after the one held at t_from, run.t(j) / run.v_at(j), raw
-// values clamped here as the pixel model clamps them). All lanes of the warp call it.
-template <class Run>
-__device__ __forceinline__ void noise_ahead(PixelRegs& s, const PixelMapRegs& m, const SensorConsts& k,
-                                            uint32_t pixel, bool active, int64_t t_from, float v_held,
-                                            int64_t t_end, const Run& run, PixelCounters& c) {
-  bool done_shot = !active, done_ba = !active;
-  for (;;) {
-    const bool p_shot = !done_shot && s.t_shot < t_end, p_ba = !done_ba && s.t_ba < t_end;
-    if (!__any_sync(0xffffffffu, p_shot || p_ba)) break;
-    if (!(p_shot || p_ba)) continue;
-    const bool shot = p_shot && (!p_ba || s.t_shot <= s.t_ba);
-    const int64_t tn = shot ? s.t_shot : s.t_ba;
-    const uint32_t purpose = shot ? kPurposeShot : kPurposeBackground;
-    const uint32_t nidx = shot ? s.n_shot : s.n_ba;
-    // The segment holding tn: [t_a, t_b) between consecutive samples, or held after the last one.
-    int64_t ta = t_from;
-    float va = v_held;
-    int64_t tb = kForever;
-    float vb = va;
-    for (int j = 0; j < run.n; ++j) {
-      const int64_t tj = run.t(j);
-      const float vj = clamp_irr(run.v_at(j), k.irr_max);
-      if (tj > tn) {
-        tb = tj;
-        vb = vj;
-        break;
-      }
-      ta = tj;
-      va = vj;
-    }
-    if (tb == kForever) vb = va;
-    const U4 w = draw(k.seed, purpose, k.camera, pixel, nidx);
-    NullSink ns;
-    PixelCounters nc;
-    const PixelProc<NullSink> hp{s, m, k, pixel, ns, nc};
-    const float I = hp.current(Segment{ta, tb, va, vb}, tn);
-    const double accept = shot ? sqrt(static_cast<double>(m.dark) / static_cast<double>(I)) : 1.0;
-    if (open_uniform_d(w.v[1]) < accept) {
-      if (shot) done_shot = true;
-      else done_ba = true;
-      continue;
-    }
-    ++c.noise_candidates;
-    const int64_t next = noise_next(k.seed, purpose, k.camera, pixel, nidx + 1, tn, shot ? m.shot_max_hz : m.ba_rate_hz);
-    if (shot) {
-      s.n_shot = nidx + 1;
-      s.t_shot = next;
-    } else {
-      s.n_ba = nidx + 1;
-      s.t_ba = next;
-    }
-  }
-}
-
-// A lane's window staged in shared memory (dt / v strided by 32 lanes) as noise_ahead's run.
-struct StagedRun {
-  int64_t t_w;
-  const uint32_t* dt;
-  const float* v;
-  int n;
-  __device__ __forceinline__ int64_t t(int j) const { return t_w + dt[j * 32]; }
-  __device__ __forceinline__ float v_at(int j) const { return v[j * 32]; }
-};
-// A CSR run in device memory as noise_ahead's run.
-struct GlobalRun {
-  const int64_t* tp;
-  const float* vp;
-  int n;
-  __device__ __forceinline__ int64_t t(int j) const { return __ldg(tp + j); }
-  __device__ __forceinline__ float v_at(int j) const { return __ldg(vp + j); }
-};
-
-// x = ln(I / i_scale) at a sample of value v (PixelProc::x_at_sample on the caller's registers).
-__device__ __forceinline__ float x_sample(const PixelRegs& s, const PixelMapRegs& m, float v) {
-  return log_f((m.dark + m.scale * v) / s.i_scale);
-}
-
-// The pixel model's full path on a state in memory, out of line: the hot loops keep the state in registers and copy
-// it here only for a segment that is not clean. fast: PixelProc::segment_fast with x at both ends; else
-// PixelProc::segment over [from, to).
-// kFlat: the processor's rare paths inline here, on copies the compiler can keep in registers (one large function:
-// the CSR kernel and the streaming engine); else they stay separate out-of-line functions working on the state in
-// memory (smaller code: the staged engine, whose instruction footprint sets its speed).
-template <class Sink, bool kFlat>
-__device__ __noinline__ void cold_segment(PixelRegs* s, const PixelMapRegs* m, const SensorConsts* k, uint32_t pixel,
-                                          Sink sink, PixelCounters* c, Segment g, int64_t from, int64_t to, bool fast,
-                                          float x0, float x1) {
-  PixelRegs sl = *s;
-  const PixelMapRegs ml = *m;
-  PixelCounters cl = *c;
-  PixelProc<Sink, kFlat> proc{sl, ml, *k, pixel, sink, cl};
-  if (fast) proc.segment_fast(g, x0, x1);
-  else proc.segment(g, from, to);
-  *s = sl;
-  *c = cl;
-}
-
-// One segment [t0, t1) of a pixel whose state is in registers: the clean outcome in place, anything else out of line.
-template <bool kFlat = true, class Sink>
-__device__ __forceinline__ void feed_segment(PixelRegs& s, const PixelMapRegs& m, const SensorConsts& k,
-                                             const SensorConsts* kd, uint32_t pixel, const Sink& sink,
-                                             PixelCounters& c, int64_t t0, int64_t t1, float v0, float v1, float x0,
-                                             float x1) {
-  if (clean_segment(s, m, k, t0, t1, v0, v1, x0, x1)) {
-    ++c.pieces;
-    if (t1 - t0 > 2) ++c.leaves;
-    s.t_search = maxi(s.t_search, t1);
-    return;
-  }
-  const Segment g{t0, t1, v0, v1};
-  const bool fast = ((t1 - 1) >> kWindowLog2) == (t0 >> kWindowLog2);
-  PixelRegs ts = s;
-  PixelMapRegs tm = m;
-  PixelCounters tc = c;
-  cold_segment<Sink, kFlat>(&ts, &tm, kd, pixel, sink, &tc, g, t0, t1, fast, x0, x1);
-  s = ts;
-  c = tc;
-}
-
-// The held sample from t_from to t_end (the end of a call), out of line where there is such a stretch.
-template <class Sink>
-__device__ __forceinline__ void feed_held(PixelRegs& s, const PixelMapRegs& m, const SensorConsts* kd, uint32_t pixel,
-                                          const Sink& sink, PixelCounters& c, int64_t t_from, float v,
-                                          int64_t t_end) {
-  if (t_from >= t_end) return;
-  PixelRegs ts = s;
-  PixelMapRegs tm = m;
-  PixelCounters tc = c;
-  cold_segment<Sink, true>(&ts, &tm, kd, pixel, sink, &tc, Segment{t_from, kForever, v, v}, t_from, t_end, false, 0.0f,
-                           0.0f);
-  s = ts;
-  c = tc;
 }
 
 // The warp-cooperative walk of one run (cnt samples at tp / vp) of a pixel whose state u every lane holds alike.
@@ -1434,85 +1111,6 @@ __global__ void scan_fix_kernel(int64_t* out, uint32_t n, const int64_t* block_s
 // ---------------------------------------------------------------------------------------------
 // The fused engine
 // ---------------------------------------------------------------------------------------------
-struct EngineArgs {
-  const EngineSensor* sensors;
-  int n_sensors;
-  uint32_t total_tiles;
-  const int64_t* t0;  // the model time, in device memory (a captured launch replays at any time)
-  int32_t w0, w1;
-  SamplerRules r;
-  unsigned int* tile_counter;
-  uint32_t tile_lw;   // log2 of the tile width: tiles of 2^lw x 2^(5 - lw) pixels, one warp each
-};
-
-// The pixel of `lane` in tile `local` of a sensor with tiles_x tiles per row.
-__device__ __forceinline__ void tile_xy(uint32_t local, uint32_t tiles_x, uint32_t lw, uint32_t lane, uint32_t& x,
-                                        uint32_t& y) {
-  x = (local % tiles_x) * (1u << lw) + (lane & ((1u << lw) - 1u));
-  y = (local / tiles_x) * (32u >> lw) + (lane >> lw);
-}
-
-// Feeds a window's samples, in time order, to the pixel model: every segment lies inside the window, so each
-// takes the fast path with x at both ends, each x computed once.
-struct WindowFeed {
-  PixelProc<GlobalSink>* proc;
-  int64_t t_w;
-  float irr_max;
-  int64_t prev_t;
-  float prev_v;
-  float last_raw;
-  float x_prev;
-  // Slot 0, the carried sample, sits at the model time: it replaces the held one.
-  __device__ __forceinline__ void start(float carried) {
-    last_raw = carried;
-    prev_v = clamp_irr(carried, irr_max);
-    x_prev = proc->x_at_sample(prev_v);
-  }
-  __device__ __forceinline__ void operator()(uint32_t dt, float v) {
-    last_raw = v;
-    const float vc = clamp_irr(v, irr_max);
-    const int64_t t = t_w + dt;
-    const float x1 = proc->x_at_sample(vc);
-    proc->segment_fast(Segment{prev_t, t, prev_v, vc}, x_prev, x1);
-    prev_t = t;
-    prev_v = vc;
-    x_prev = x1;
-  }
-};
-
-// WindowFeed for a pixel whose state stays in the caller's registers (s, m, c): each segment's clean outcome is taken
-// in place, anything else out of line (feed_segment<kFlat>); the same samples and state as WindowFeed's.
-template <bool kFlat, class Sink = GlobalSink>
-struct RegFeed {
-  PixelRegs& s;
-  const PixelMapRegs& m;
-  PixelCounters& c;
-  const SensorConsts& k;
-  const SensorConsts* kd;
-  uint32_t pixel;
-  Sink sink;
-  int64_t t_w;
-  int64_t prev_t;
-  float prev_v;
-  float last_raw;
-  float x_prev;
-  __device__ __forceinline__ void start(float carried) {
-    last_raw = carried;
-    prev_v = clamp_irr(carried, k.irr_max);
-    x_prev = x_sample(s, m, prev_v);
-  }
-  __device__ __forceinline__ void operator()(uint32_t dt, float v) {
-    last_raw = v;
-    const float vc = clamp_irr(v, k.irr_max);
-    const int64_t t = t_w + dt;
-    const float x1 = x_sample(s, m, vc);
-    feed_segment<kFlat>(s, m, k, kd, pixel, sink, c, prev_t, t, prev_v, vc, x_prev, x1);
-    prev_t = t;
-    prev_v = vc;
-    x_prev = x1;
-  }
-};
-
 // At most 128 registers (168 uncapped): 7.79 against 7.93 ms per step on 346x260 (102 registers: 8.58).
 __global__ void __launch_bounds__(128, 4) engine_kernel(EngineArgs a) {
   const uint32_t lane = threadIdx.x & 31u;
@@ -2061,259 +1659,6 @@ __global__ void __launch_bounds__(128) engine_kernel_staged(EngineArgs a) {
     warp_add(&S.counters[kCntLeaves], c.leaves);
     warp_add(&S.counters[kCntSamples], samples);
     warp_add(&S.counters[kCntNoise], c.noise_candidates);
-  }
-}
-
-// ---------------------------------------------------------------------------------------------
-// The split engine: per window, the common path in one kernel and the rare one in another
-// ---------------------------------------------------------------------------------------------
-// A pixel's rare paths (a segment where a crossing may occur, an accepted noise candidate, the refractory interval,
-// the first segment after the start) run one or two lanes at a time while the rest of the warp waits, and their code
-// competes with the hot loop's for the instruction cache: on the six sensors they took most of the staged engine's
-// time. Here each window is two launches. engine_window_kernel runs the staged engine's phases for every pixel (the
-// walk with its first kSplitStage samples staged, the noise pass, the pixel model's clean segments in registers)
-// and, at a pixel's first segment that is not clean, stops that pixel and posts it (its state, its feed and the
-// staged samples left) to a list; a window that overflows the stage is posted whole. engine_rest_kernel then
-// finishes the posted pixels' windows, one thread per pixel, through the full pixel model, so its lanes all run the
-// rare paths together. A pixel's samples are fed in the same order to the same state either way, so events and
-// state are the staged engine's; the state passes from one window to the next through HBM.
-constexpr int kSplitStage = 16;
-constexpr uint32_t kRestWhole = 0xFF;  // the samples left of a window that overflowed the stage
-
-// The posted pixels, as planes (structure of arrays): field k of record i at plane k, entry i, so that the window
-// kernel's posting lanes (consecutive records) store and the rest kernel's threads load with coalesced accesses.
-// Per record: the state where the pixel stopped (after the noise pass and its clean segments); the feed (the last
-// sample fed: time, clamped value, x; the last raw value); the pixel, its sensor, the samples left in dt / v
-// (kRestWhole: the window from its start, the carried sample in last_raw) and the window's lattice level (for a
-// whole window); the staged samples left.
-enum : int { kR64TRef, kR64TSearch, kR64Blind, kR64TShot, kR64TBa, kR64PrevT, kRest64 };
-enum : int {
-  kR32S3Ref, kR32N3Ref, kR32DrRef, kR32IScale, kR32Held, kR32Flags, kR32NShot, kR32NBa, kR32PrevV, kR32XPrev,
-  kR32LastRaw, kR32Pixel, kR32Tag, kR32Dt, kR32V = kR32Dt + kSplitStage, kRest32 = kR32V + kSplitStage
-};
-constexpr size_t kRestRecordBytes = kRest64 * 8 + kRest32 * 4;
-
-struct RestList {
-  unsigned char* base;  // kRest64 planes of 8 bytes, then kRest32 planes of 4, each `capacity` entries
-  unsigned int* count;
-  unsigned int capacity;
-  __device__ __forceinline__ int64_t* p64(int k) const {
-    return reinterpret_cast<int64_t*>(base) + static_cast<size_t>(k) * capacity;
-  }
-  __device__ __forceinline__ uint32_t* p32(int k) const {
-    return reinterpret_cast<uint32_t*>(base + static_cast<size_t>(kRest64) * 8 * capacity) +
-           static_cast<size_t>(k) * capacity;
-  }
-  __device__ __forceinline__ void put_state(unsigned int i, const PixelRegs& s) const {
-    p64(kR64TRef)[i] = s.t_ref;
-    p64(kR64TSearch)[i] = s.t_search;
-    p64(kR64Blind)[i] = s.blind_until;
-    p64(kR64TShot)[i] = s.t_shot;
-    p64(kR64TBa)[i] = s.t_ba;
-    p32(kR32S3Ref)[i] = __float_as_uint(s.s3_ref);
-    p32(kR32N3Ref)[i] = __float_as_uint(s.n3_ref);
-    p32(kR32DrRef)[i] = __float_as_uint(s.dr_ref);
-    p32(kR32IScale)[i] = __float_as_uint(s.i_scale);
-    p32(kR32Held)[i] = __float_as_uint(s.held);
-    p32(kR32Flags)[i] = s.flags;
-    p32(kR32NShot)[i] = s.n_shot;
-    p32(kR32NBa)[i] = s.n_ba;
-  }
-  __device__ __forceinline__ PixelRegs state(unsigned int i) const {
-    PixelRegs s;
-    s.t_ref = p64(kR64TRef)[i];
-    s.t_search = p64(kR64TSearch)[i];
-    s.blind_until = p64(kR64Blind)[i];
-    s.t_shot = p64(kR64TShot)[i];
-    s.t_ba = p64(kR64TBa)[i];
-    s.s3_ref = __uint_as_float(p32(kR32S3Ref)[i]);
-    s.n3_ref = __uint_as_float(p32(kR32N3Ref)[i]);
-    s.dr_ref = __uint_as_float(p32(kR32DrRef)[i]);
-    s.i_scale = __uint_as_float(p32(kR32IScale)[i]);
-    s.held = __uint_as_float(p32(kR32Held)[i]);
-    s.flags = p32(kR32Flags)[i];
-    s.n_shot = p32(kR32NShot)[i];
-    s.n_ba = p32(kR32NBa)[i];
-    return s;
-  }
-};
-
-// Window a.w0 of every tile (a.t0 the model time at the call's start). kFirst: the call's first window, where the
-// pixels' searches can be armed after their first segment's start (after init): such a segment is also taken in
-// place when clean (clean_after_start), instead of being posted; the other windows' kernel leaves that test out (in
-// the hot loop it cost more than it saves there).
-template <bool kFirst>
-__global__ void __launch_bounds__(128) engine_window_kernel(EngineArgs a, RestList rl) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const int64_t t_w = *a.t0 + static_cast<int64_t>(a.w0) * kWindowNs;
-  __shared__ uint16_t lists[4][kMaxListed];
-  __shared__ uint32_t st_dt[4][kSplitStage][32];
-  __shared__ float st_v[4][kSplitStage][32];
-  uint16_t* my_list = lists[warp];
-  for (;;) {
-    uint32_t tile = 0;
-    if (lane == 0) tile = atomicAdd(a.tile_counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if (tile >= a.total_tiles) break;
-    int si = 0;
-    while (si + 1 < a.n_sensors && a.sensors[si + 1].tile0 <= tile) ++si;
-    const EngineSensor& S = a.sensors[si];
-    const uint32_t local = tile - S.tile0;
-    uint32_t x, y;
-    tile_xy(local, S.tiles_x, a.tile_lw, lane, x, y);
-    const bool have = x < S.width && y < S.height;
-    const uint32_t p = have ? y * S.width + x : 0u;
-    const bool noise = S.consts.noise != 0;
-    const float irr_max = S.consts.irr_max;
-    PixelRegs s;
-    PixelMapRegs m;
-    float carried = 0.0f;
-    if (have) {
-      load_state(S.in, p, noise, s);
-      load_map(S.map, p, m);
-      carried = S.carried_in[p];
-    }
-    PixelCounters c;
-    const FieldDev& f = S.field;
-    const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, my_list);
-    auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
-    // The walk, its first kSplitStage samples after slot 0 staged.
-    uint32_t n = 0;
-    int level = 0;
-    if (have) {
-      level = field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
-      uint32_t k = 0;
-      n = sample_pixel_window(a.r, level, carried, false, render, [&](uint32_t dt, float v) {
-        if (k < static_cast<uint32_t>(kSplitStage)) {
-          st_dt[warp][k][lane] = dt;
-          st_v[warp][k][lane] = v;
-        }
-        ++k;
-      });
-    }
-    __syncwarp();
-    const bool staged = have && n - 1 <= static_cast<uint32_t>(kSplitStage);
-    // The window's noise candidates of all lanes together; the rejected ones leave the pixel model.
-    if (noise) {
-      const StagedRun run{t_w, &st_dt[warp][0][lane], &st_v[warp][0][lane], static_cast<int>(n) - 1};
-      noise_ahead(s, m, S.consts, p, staged, t_w, clamp_irr(carried, irr_max), t_w + kWindowNs, run, c);
-    }
-    // The clean segments in place; the first other one stops the pixel there (a window that overflowed the stage
-    // stops at its start).
-    bool post = have && !staged;
-    uint32_t j = 0;
-    int64_t prev_t = t_w;
-    float prev_v = 0.0f, last_raw = carried, x_prev = 0.0f;
-    if (staged) {
-      prev_v = clamp_irr(carried, irr_max);
-      x_prev = x_sample(s, m, prev_v);
-      for (; j + 1 < n; ++j) {
-        const float v = st_v[warp][j][lane];
-        const int64_t t = t_w + st_dt[warp][j][lane];
-        const float vc = clamp_irr(v, irr_max);
-        const float x1 = x_sample(s, m, vc);
-        if (!clean_segment(s, m, S.consts, prev_t, t, prev_v, vc, x_prev, x1) &&
-            !(kFirst && clean_after_start(s, m, S.consts, prev_t, t, prev_v, vc, x_prev, x1))) {
-          break;
-        }
-        ++c.pieces;
-        if (t - prev_t > 2) ++c.leaves;
-        s.t_search = maxi(s.t_search, t);
-        last_raw = v;
-        prev_t = t;
-        prev_v = vc;
-        x_prev = x1;
-      }
-      post = j + 1 < n;
-      if (!post) {
-        s.held = prev_v;
-        store_state(S.out, p, noise, s);
-        S.carried_out[p] = last_raw;
-      }
-    }
-    // One record per stopped pixel, the warp's records reserved together.
-    __syncwarp();
-    const unsigned posting = __ballot_sync(0xffffffffu, post);
-    if (posting != 0u) {
-      const int leader = __ffs(posting) - 1;
-      unsigned int base = 0;
-      if (static_cast<int>(lane) == leader) base = atomicAdd(rl.count, static_cast<unsigned int>(__popc(posting)));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (post) {
-        const unsigned int i = base + static_cast<unsigned int>(__popc(posting & ((1u << lane) - 1u)));
-        if (i >= rl.capacity) {
-          atomicOr(&S.counters[kCntErrors], kErrRestList);
-        } else {
-          rl.put_state(i, s);
-          rl.p64(kR64PrevT)[i] = prev_t;
-          rl.p32(kR32PrevV)[i] = __float_as_uint(prev_v);
-          rl.p32(kR32XPrev)[i] = __float_as_uint(x_prev);
-          rl.p32(kR32LastRaw)[i] = __float_as_uint(last_raw);
-          rl.p32(kR32Pixel)[i] = p;
-          const uint32_t left = staged ? n - 1 - j : kRestWhole;
-          rl.p32(kR32Tag)[i] = static_cast<uint32_t>(si) | left << 16 | static_cast<uint32_t>(level) << 24;
-          if (staged) {  // by plane, so that the posting lanes write each plane together
-            for (uint32_t u = 0; u < left; ++u) {
-              rl.p32(kR32Dt + static_cast<int>(u))[i] = st_dt[warp][j + u][lane];
-              rl.p32(kR32V + static_cast<int>(u))[i] = __float_as_uint(st_v[warp][j + u][lane]);
-            }
-          }
-        }
-      }
-    }
-    __syncwarp();
-    warp_add(&S.counters[kCntPieces], c.pieces);
-    warp_add(&S.counters[kCntLeaves], c.leaves);
-    warp_add(&S.counters[kCntSamples], have ? n : 0u);
-    warp_add(&S.counters[kCntNoise], c.noise_candidates);
-  }
-}
-
-// The posted pixels of window a.w0, one thread each: the rest of the window through the full pixel model (a window
-// posted whole is walked again from its start, every blob of the field evaluated: the same values as the warp's
-// culled list gives), then the state and the carried sample stored. Capped for 5 blocks per SM (at most 102
-// registers): more spills, but 20 warps per SM; on the six sensors 68.5 ms per step against 70.1 at 4 blocks (128
-// registers) and 69.0 at 6 (4 blocks had measured 0.5 % faster than 3, uncapped).
-__global__ void __launch_bounds__(128, 5) engine_rest_kernel(EngineArgs a, RestList rl) {
-  const int64_t t_w = *a.t0 + static_cast<int64_t>(a.w0) * kWindowNs;
-  const unsigned int count = min(*rl.count, rl.capacity);
-  for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    const uint32_t tag = rl.p32(kR32Tag)[i], pixel = rl.p32(kR32Pixel)[i];
-    const uint32_t left = tag >> 16 & 0xFFu;
-    const float raw0 = __uint_as_float(rl.p32(kR32LastRaw)[i]);
-    const EngineSensor& S = a.sensors[tag & 0xFFFFu];
-    PixelRegs s = rl.state(i);
-    PixelMapRegs m;
-    load_map(S.map, pixel, m);
-    PixelCounters c;
-    const ThreadSink sink{S.ev, &S.counters[kCntEvents]};
-    float held, last_raw;
-    if (left == kRestWhole) {
-      const FieldDev& f = S.field;
-      const BlobList all{nullptr, f.n_blobs};
-      const uint32_t x = pixel % S.width, y = pixel / S.width;
-      auto render = [&](uint32_t dt) { return field_eval(f, all, x, y, t_w + dt); };
-      RegFeed<true, ThreadSink> feed{s, m, c, S.consts, &S.consts, pixel, sink, t_w, t_w, s.held, raw0, 0.0f};
-      feed.start(raw0);
-      sample_pixel_window(a.r, static_cast<int>(tag >> 24), raw0, false, render, feed);
-      held = feed.prev_v;
-      last_raw = feed.last_raw;
-    } else {
-      RegFeed<true, ThreadSink> feed{s, m, c, S.consts, &S.consts, pixel, sink, t_w, rl.p64(kR64PrevT)[i],
-                                     __uint_as_float(rl.p32(kR32PrevV)[i]), raw0,
-                                     __uint_as_float(rl.p32(kR32XPrev)[i])};
-      for (uint32_t q = 0; q < left; ++q) {
-        feed(rl.p32(kR32Dt + static_cast<int>(q))[i], __uint_as_float(rl.p32(kR32V + static_cast<int>(q))[i]));
-      }
-      held = feed.prev_v;
-      last_raw = feed.last_raw;
-    }
-    s.held = held;
-    store_state(S.out, pixel, S.consts.noise != 0, s);
-    S.carried_out[pixel] = last_raw;
-    if (c.pieces) atomicAdd(&S.counters[kCntPieces], static_cast<unsigned long long>(c.pieces));
-    if (c.leaves) atomicAdd(&S.counters[kCntLeaves], static_cast<unsigned long long>(c.leaves));
-    if (c.noise_candidates) atomicAdd(&S.counters[kCntNoise], static_cast<unsigned long long>(c.noise_candidates));
   }
 }
 
@@ -2913,18 +2258,6 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
   else engine_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
 }
 
-void launch_engine_split(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
-                         int32_t w, const SamplerRules& r, unsigned int* tile_counter, void* rest, unsigned int* rest_count,
-                         unsigned int rest_capacity, int blocks, int warps_per_block, int tile_lw, int rest_blocks,
-                         cudaStream_t stream) {
-  const EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w, w + 1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
-  const RestList rl{static_cast<unsigned char*>(rest), rest_count, rest_capacity};
-  if (w == 0) engine_window_kernel<true><<<blocks, warps_per_block * 32, 0, stream>>>(a, rl);
-  else engine_window_kernel<false><<<blocks, warps_per_block * 32, 0, stream>>>(a, rl);
-  engine_rest_kernel<<<rest_blocks, 128, 0, stream>>>(a, rl);
-}
-
-size_t rest_record_bytes() { return kRestRecordBytes; }
 size_t row_rest_bytes() { return sizeof(RowRest); }
 int rows_rest_blocks_per_sm() {
   int n = 0;
@@ -2932,18 +2265,8 @@ int rows_rest_blocks_per_sm() {
   return n;
 }
 
-int engine_rest_blocks_per_sm() {
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_rest_kernel, 128, 0);
-  return n;
-}
-
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade) {
   int n = 0;
-  if (stage == kStageSplit) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_window_kernel<false>, warps_per_block * 32, 0);
-    return n;
-  }
   if (cascade == 2 && stage != 0) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel_staged, warps_per_block * 32, 0);
   } else if (cascade == 2) {

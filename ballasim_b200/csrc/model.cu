@@ -1121,6 +1121,7 @@ struct FieldHolder {
                     cudaMemcpyHostToDevice));
       f.blobs = blobs.p;
     }
+    field_bounds(f, h.blobs);
   }
 };
 
@@ -1576,16 +1577,13 @@ struct Engine {
   DevBuf<unsigned long long> rec_count;
   size_t rec_cap = 0;
   unsigned long long rec_n[2] = {0, 0};
-  // The split engine (stage kStageSplit): two scratch states and carried frames per sensor that the windows between
-  // a call's first and last pass the state through, the per-window descriptors, the posted-pixel list (room for every
-  // pixel), and per window a tile counter and a list count.
-  std::vector<std::unique_ptr<StateBufs>> split_state;
-  std::vector<std::unique_ptr<DevBuf<float>>> split_carried;
-  DevBuf<EngineSensor> split_desc;
-  PinBuf<EngineSensor> split_desc_pin;
+  // The split engine (stage kStageSplit): its scratch (the quick records and blob boxes), the posted-pixel list (room
+  // for every pixel), and a list count per window.
+  DevBuf<float4> split_scratch;
   DevBuf<unsigned char> rest;
   DevBuf<unsigned int> split_counts;
   unsigned int rest_capacity = 0;
+  uint32_t total_blobs = 0;
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
   // 0 the instantaneous response, 1 the cascade, 2 the cascade with its noise lattice (every sensor alike).
@@ -1624,6 +1622,8 @@ struct Engine {
       e.tiles_x = (m->width + 7) / 8;
       e.tiles_y = (m->height + 3) / 4;
       e.tile0 = tile0;
+      e.blob0 = total_blobs;
+      total_blobs += static_cast<uint32_t>(fields.back()->f.n_blobs);
       tile0 += e.tiles_x * e.tiles_y;
       host.push_back(e);
     }
@@ -1734,6 +1734,8 @@ struct Engine {
     const int wpb = block_warps();
     const int per_sm = blocks_per_sm > 0 ? blocks_per_sm
                                          : std::max(1, mlp ? learned_engine_max_blocks_per_sm(wpb)
+                                                       : stage == kStageSplit
+                                                           ? split_window_blocks_per_sm(wpb)
                                                            : engine_max_blocks_per_sm(wpb, stage, cascade()));
     return static_cast<int>(
         std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, (total_tiles + wpb - 1) / wpb));
@@ -1765,45 +1767,15 @@ struct Engine {
     t0_pin.p[0] = t0;
   }
 
-  // The split engine's descriptors, window-major: window w reads what w - 1 wrote (the call's input state for the
-  // first window), and writes a scratch state (the call's output state for the last one).
-  void describe_split(int32_t windows) {
-    const size_t ns = models.size();
-    if (split_state.size() < 2 * ns) {
-      split_state.clear();
-      split_carried.clear();
-      for (size_t i = 0; i < 2 * ns; ++i) {
-        split_state.push_back(std::make_unique<StateBufs>());
-        split_carried.push_back(std::make_unique<DevBuf<float>>());
-      }
-    }
+  void ensure_split(int32_t windows) {
     unsigned int pixels = 0;
     for (Model* m : models) pixels += m->n;
     if (rest_capacity < pixels) {
-      rest.ensure(static_cast<size_t>(pixels) * rest_record_bytes());
+      rest.ensure(static_cast<size_t>(pixels) * split_record_bytes());
       rest_capacity = pixels;
     }
-    const size_t nw = static_cast<size_t>(std::max(windows, 1));
-    split_desc_pin.ensure(nw * ns);
-    split_desc.ensure(nw * ns);
-    split_counts.ensure(2 * nw);
-    for (size_t i = 0; i < ns; ++i) {
-      Model* m = models[i];
-      const StateSoA tmp[2] = {split_state[2 * i]->soa(m->n, m->mode()), split_state[2 * i + 1]->soa(m->n, m->mode())};
-      float* tmp_c[2] = {split_carried[2 * i]->ensure(m->n), split_carried[2 * i + 1]->ensure(m->n)};
-      for (size_t w = 0; w < nw; ++w) {
-        EngineSensor e = host_pin.p[i];
-        if (w > 0) {
-          e.in = tmp[(w - 1) % 2];
-          e.carried_in = tmp_c[(w - 1) % 2];
-        }
-        if (w + 1 < nw) {
-          e.out = tmp[w % 2];
-          e.carried_out = tmp_c[w % 2];
-        }
-        split_desc_pin.p[w * ns + i] = e;
-      }
-    }
+    split_scratch.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4));
+    split_counts.ensure(static_cast<size_t>(std::max(windows, 1)));
   }
 
   // One step's device work, in stream order (what the CUDA graph holds): counters cleared, descriptors and the
@@ -1826,16 +1798,13 @@ struct Engine {
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
                               rules, l, tile_counter.p, blocks, block_warps(), tile_lw, st);
       } else if (stage == kStageSplit) {
-        const size_t ns = host.size();
-        CK(cudaMemcpyAsync(split_desc.p, split_desc_pin.p, static_cast<size_t>(windows) * ns * sizeof(EngineSensor),
-                           cudaMemcpyHostToDevice, st));
-        CK(cudaMemsetAsync(split_counts.p, 0, 2 * static_cast<size_t>(windows) * sizeof(unsigned int), st));
-        const int rest_blocks = sm_count() * std::max(1, engine_rest_blocks_per_sm());
-        for (int32_t w = 0; w < windows; ++w) {
-          launch_engine_split(split_desc.p + static_cast<size_t>(w) * ns, static_cast<int>(ns), total_tiles, t0_dev.p,
-                              w, rules, split_counts.p + 2 * w, rest.p, split_counts.p + 2 * w + 1, rest_capacity,
-                              blocks, warps_per_block, tile_lw, rest_blocks, st);
-        }
+        CK(cudaMemsetAsync(split_counts.p, 0, static_cast<size_t>(windows) * sizeof(unsigned int), st));
+        const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());
+        std::vector<uint32_t> tile0;
+        for (const EngineSensor& e : host) tile0.push_back(e.tile0);
+        launch_engine_split(sensors_dev.p, tile0.data(), static_cast<int>(host.size()), total_tiles, total_blobs,
+                            t0_dev.p, windows, rules, split_scratch.p, rest.p, split_counts.p, rest_capacity, blocks,
+                            warps_per_block, tile_lw, rest_blocks, st);
       } else {
         launch_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows, rules,
                       tile_counter.p, blocks, warps_per_block, stage, tile_lw, cascade(), st);
@@ -1873,7 +1842,7 @@ struct Engine {
     rec_n_pin.ensure(2);
     for (;;) {
       describe(t0);
-      if (stage == kStageSplit) describe_split(windows);
+      if (stage == kStageSplit) ensure_split(windows);
       if (use_graph && rec_cap == 0) {
         const uint64_t key[8] = {static_cast<uint64_t>(windows), static_cast<uint64_t>(blocks),
                                  static_cast<uint64_t>(block_warps()), static_cast<uint64_t>(stage),

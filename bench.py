@@ -75,12 +75,6 @@ NCU = {
     # traffic: one pass on the full 60-window launch; instructions and issue-active: the full set on its first 4
     # windows (74,251,870 pixel-samples).
     "six_sensors_4.6Mpx": [
-        # The split engine: one pass over all 120 launches of a step (traffic, instructions: the step's sums);
-        # issue-active: the two kernels' full-set figures on one window, weighted by their time (that full set was
-        # taken while the posted records were one struct per pixel rather than planes).
-        {"kernel": "engine_window_kernel+engine_rest_kernel", "stage": 1, "tile_width": 8,
-         "traffic": (32.41e9 + 0.5452e9 + 6.498e9) + (19.34e9 + 0.3281e9 + 3.512e9),
-         "inst_per_sample": (3.488e10 + 6.022e8 + 1.819e9) / 1103436116, "issue_active": 0.471},
         {"kernel": "engine_kernel_staged<16>", "stage": 16, "tile_width": 8, "traffic": 690.74e6 + 3.59e9,
          "inst_per_sample": 3.329e9 / 74251870, "issue_active": 0.209},
         {"kernel": "engine_kernel_staged<16>", "stage": 16, "tile_width": 4, "traffic": 694.48e6 + 3.67e9,
@@ -195,12 +189,13 @@ def engine_kernel_name(eng, cascade: bool, lattice: bool) -> str:
     if cascade:
         return "engine_lattice_kernel" if lattice else "engine_cascade_kernel"
     return {64: "engine_kernel_coop", 16: "engine_kernel_staged<16>", 32: "engine_kernel_staged<32>",
-            1: "engine_window_kernel+engine_rest_kernel"}.get(eng.launch["stage"], "engine_kernel")
+            1: "split_window_kernel+split_rest_kernel"}.get(eng.launch["stage"], "engine_kernel")
 
 
 def engine_launches(eng, windows: int) -> int:
-    """The engine's kernel launches in one step: one persistent launch, or two per window for the split engine."""
-    return 2 * windows if eng.launch["stage"] == 1 else 1
+    """The engine's kernel launches in one step: one persistent launch, or for the split engine two per window and its
+    begin and end kernels."""
+    return 2 * windows + 2 if eng.launch["stage"] == 1 else 1
 
 
 def run_ours(args, rank: int, world: int) -> dict | None:

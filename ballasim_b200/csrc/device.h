@@ -202,10 +202,6 @@ int learned_engine_max_blocks_per_sm(int warps_per_block);
 void launch_learned_reset(LearnedSoA st, uint32_t n, const float* irr0, cudaStream_t stream);
 
 // ---- event output order (events.cu) ----
-// Sorts n device events by (t_cross, pixel) into out (device), using sort_events_scratch_bytes(n) bytes of scratch.
-size_t sort_events_scratch_bytes(uint32_t n);
-cudaError_t sort_events(const RawEvent* ev, uint32_t n, RawEvent* out, void* scratch, cudaStream_t stream);
-
 // The readout of a crossing (Readout, src/sensor/readout.h:14-27): delayed, floored to the counter quantum from its
 // phase, then on the sensor clock (offset, drift).
 struct ReadoutDev {
@@ -230,7 +226,6 @@ BS_HD int64_t output_cut(const ReadoutDev& r, int64_t t_end) {
   return reported_time(clock, t_end);
 }
 
-// One output event (OutEvent, src/engine/output.h:25-32, without the ground-truth fields): 24 bytes.
 // Device event columns (any pointer null: that column is skipped).
 struct EventColumnsDev {
   uint32_t* pixel;
@@ -241,9 +236,25 @@ struct EventColumnsDev {
   uint16_t* flags;
   float *ds, *dn, *dl, *l_first;
 };
-cudaError_t event_columns(const RawEvent* ev, uint32_t n, uint32_t width, const ReadoutDev& rd,
-                          const EventColumnsDev& cols, cudaStream_t stream);
+// Where sorted events go: to records (not null), or split into columns (x, y by the frame's width, the reported time).
+struct EventsOut {
+  RawEvent* records;
+  EventColumnsDev cols;
+  uint32_t width;
+  ReadoutDev readout;
+};
+// What is known of a list of events: their times lie in [lo, hi] (hi < lo: nothing is known) and their pixels below
+// `pixels`.
+struct EventSpan {
+  int64_t lo, hi;
+  uint64_t pixels;
+};
+// Sorts n device events by (t_cross, pixel) into out, using sort_events_scratch_bytes(n) bytes of device scratch.
+size_t sort_events_scratch_bytes(uint32_t n);
+cudaError_t sort_events(const RawEvent* ev, uint32_t n, const EventSpan& span, const EventsOut& out, void* scratch,
+                        cudaStream_t stream);
 
+// One output event (OutEvent, src/engine/output.h:25-32, without the ground-truth fields): 24 bytes.
 struct OutRecord {
   int64_t t_reported, t_cross;
   uint16_t x, y, flags;

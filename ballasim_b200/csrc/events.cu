@@ -1,13 +1,14 @@
 // Event order on the device.
 //
 // sort_events: SensorModel::finish_events sorts a call's events by (t_cross, pixel) on the host
-// (src/sensor/sensor_model.cpp:996-1029); here two stable radix passes over an index permutation (pixel first, then
-// t_cross) and one gather put the RawEvent records in that order in device memory, so that the host only copies
-// them out. (t_cross, pixel) is unique per event (a pixel fires at most once per ns), so the order is the host
-// sort's exactly.
-//
-// event_columns: the sorted records split into event columns (x, y from the pixel index, the readout's reported time)
-// on the device, so that the host copies each column out whole.
+// (src/sensor/sensor_model.cpp:996-1029); here they are sorted on the device and written out either as records or split
+// into event columns (x, y from the pixel index, the readout's reported time), so that the host only copies them out.
+// (t_cross, pixel) is unique per event (a pixel fires at most once per ns), so the order is the host sort's exactly.
+// Three forms, by size and by what is known of the events:
+//  - up to kSmallSort events: one block sorts them in shared memory and writes the output, one launch;
+//  - where the events' time span and the pixels fit 64 bits together (a call's own events): one radix sort of that key
+//    over its used bits, then the output;
+//  - else two stable radix sorts (pixel, then t_cross).
 //
 // output_stage: the engine's output stage (Camera::output, src/engine/engine_impl.h:1761-1847): records with the
 // readout's reported time, three stable radix passes (t_cross, (x, y), t_reported) that order them by
@@ -34,18 +35,89 @@ __global__ void time_keys_kernel(const RawEvent* ev, const uint32_t* idx, uint32
   key[i] = static_cast<uint64_t>(ev[idx[i]].t_cross) ^ (uint64_t{1} << 63);
 }
 
-__global__ void gather_events_kernel(const RawEvent* ev, const uint32_t* idx, uint32_t n, RawEvent* out) {
+// The event's row of the output: the record itself, or its columns.
+__device__ __forceinline__ void put_event(const RawEvent& e, uint32_t i, const EventsOut& o) {
+  if (o.records) {
+    o.records[i] = e;
+    return;
+  }
+  const EventColumnsDev& c = o.cols;
+  if (c.pixel) c.pixel[i] = e.pixel;
+  if (c.x) c.x[i] = static_cast<uint16_t>(e.pixel % o.width);
+  if (c.y) c.y[i] = static_cast<uint16_t>(e.pixel / o.width);
+  if (c.p) c.p[i] = e.polarity;
+  if (c.t_cross) c.t_cross[i] = e.t_cross;
+  if (c.t_reported) c.t_reported[i] = reported_time(o.readout, e.t_cross);
+  if (c.label) c.label[i] = e.label;
+  if (c.flags) c.flags[i] = e.flags;
+  if (c.ds) c.ds[i] = e.ds;
+  if (c.dn) c.dn[i] = e.dn;
+  if (c.dl) c.dl[i] = e.dl;
+  if (c.l_first) c.l_first[i] = e.l_first;
+}
+
+__global__ void put_events_kernel(const RawEvent* ev, const uint32_t* idx, uint32_t n, EventsOut o) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) put_event(ev[idx[i]], i, o);
+}
+
+// (t - lo) in the high bits, the pixel in the low ones: the whole order in one key.
+__global__ void span_keys_kernel(const RawEvent* ev, uint32_t n, int64_t lo, int pixel_bits, uint64_t* key,
+                                 uint32_t* idx) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const uint4* src = reinterpret_cast<const uint4*>(ev + idx[i]);
-  uint4* dst = reinterpret_cast<uint4*>(out + i);
-  dst[0] = src[0];
-  dst[1] = src[1];
+  key[i] = static_cast<uint64_t>(ev[i].t_cross - lo) << pixel_bits | ev[i].pixel;
+  idx[i] = i;
+}
+
+// A short list, in one block: a bitonic sort of (t, pixel, index) in shared memory over the next power of two (the
+// rows past n sort last), then the output. Its few hundred dependent steps take 4 to 9 us, where the radix sorts are
+// seven launches and their two single-tile sorts alone 27 us (160 events).
+constexpr uint32_t kSmallSort = 2048;
+__global__ void __launch_bounds__(1024) small_sort_kernel(const RawEvent* ev, uint32_t n, uint32_t size, EventsOut o) {
+  __shared__ int64_t t[kSmallSort];
+  __shared__ uint32_t px[kSmallSort];
+  __shared__ uint16_t at[kSmallSort];
+  for (uint32_t i = threadIdx.x; i < size; i += blockDim.x) {
+    t[i] = i < n ? ev[i].t_cross : INT64_MAX;
+    px[i] = i < n ? ev[i].pixel : 0xFFFFFFFFu;
+    at[i] = static_cast<uint16_t>(i);
+  }
+  __syncthreads();
+  for (uint32_t k = 2; k <= size; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      for (uint32_t q = threadIdx.x; q < size / 2u; q += blockDim.x) {
+        const uint32_t a = 2u * q - (q & (j - 1u)), b = a + j;
+        const bool rising = (a & k) == 0u;
+        // Rows of equal time and pixel are the padding's only; the index keeps those behind any event like them.
+        const bool after = t[a] > t[b] || (t[a] == t[b] && (px[a] > px[b] || (px[a] == px[b] && at[a] > at[b])));
+        if (after == rising) {
+          const int64_t tt = t[a];
+          t[a] = t[b];
+          t[b] = tt;
+          const uint32_t pp = px[a];
+          px[a] = px[b];
+          px[b] = pp;
+          const uint16_t aa = at[a];
+          at[a] = at[b];
+          at[b] = aa;
+        }
+      }
+      __syncthreads();
+    }
+  }
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) put_event(ev[at[i]], i, o);
 }
 
 struct SortLayout {
   size_t k32_in, k32_out, idx_a, idx_b, k64_in, k64_out, temp, temp_bytes, total;
 };
+
+int bits_of(uint64_t v) {  // the bits that hold 0 .. v (at least 1)
+  int b = 1;
+  while (b < 64 && (v >> b) != 0) ++b;
+  return b;
+}
 
 size_t align256(size_t v) { return (v + 255) & ~size_t{255}; }
 
@@ -190,42 +262,19 @@ cudaError_t output_stage(const OutRecord* held, uint32_t n_held, const RawEvent*
   return cudaGetLastError();
 }
 
-// ---- event columns: the sorted records split into the caller's columns on the device ----
-namespace {
-__global__ void columns_kernel(const RawEvent* ev, uint32_t n, uint32_t width, ReadoutDev rd, EventColumnsDev c) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const RawEvent e = ev[i];
-  if (c.pixel) c.pixel[i] = e.pixel;
-  if (c.x) c.x[i] = static_cast<uint16_t>(e.pixel % width);
-  if (c.y) c.y[i] = static_cast<uint16_t>(e.pixel / width);
-  if (c.p) c.p[i] = e.polarity;
-  if (c.t_cross) c.t_cross[i] = e.t_cross;
-  if (c.t_reported) c.t_reported[i] = reported_time(rd, e.t_cross);
-  if (c.label) c.label[i] = e.label;
-  if (c.flags) c.flags[i] = e.flags;
-  if (c.ds) c.ds[i] = e.ds;
-  if (c.dn) c.dn[i] = e.dn;
-  if (c.dl) c.dl[i] = e.dl;
-  if (c.l_first) c.l_first[i] = e.l_first;
-}
-}  // namespace
+size_t sort_events_scratch_bytes(uint32_t n) { return n <= kSmallSort ? 0 : layout(n).total; }
 
-cudaError_t event_columns(const RawEvent* ev, uint32_t n, uint32_t width, const ReadoutDev& rd,
-                          const EventColumnsDev& cols, cudaStream_t stream) {
+cudaError_t sort_events(const RawEvent* ev, uint32_t n, const EventSpan& span, const EventsOut& out, void* scratch,
+                        cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
-  columns_kernel<<<(n + 255) / 256, 256, 0, stream>>>(ev, n, width, rd, cols);
-  return cudaGetLastError();
-}
-
-size_t sort_events_scratch_bytes(uint32_t n) { return n == 0 ? 0 : layout(n).total; }
-
-cudaError_t sort_events(const RawEvent* ev, uint32_t n, RawEvent* out, void* scratch, cudaStream_t stream) {
-  if (n == 0) return cudaSuccess;
+  if (n <= kSmallSort) {
+    uint32_t size = 2;
+    while (size < n) size <<= 1;
+    small_sort_kernel<<<1, size / 2u < 32u ? 32u : size / 2u, 0, stream>>>(ev, n, size, out);
+    return cudaGetLastError();
+  }
   const SortLayout l = layout(n);
   unsigned char* base = static_cast<unsigned char*>(scratch);
-  uint32_t* k32_in = reinterpret_cast<uint32_t*>(base + l.k32_in);
-  uint32_t* k32_out = reinterpret_cast<uint32_t*>(base + l.k32_out);
   uint32_t* idx_a = reinterpret_cast<uint32_t*>(base + l.idx_a);
   uint32_t* idx_b = reinterpret_cast<uint32_t*>(base + l.idx_b);
   uint64_t* k64_in = reinterpret_cast<uint64_t*>(base + l.k64_in);
@@ -233,16 +282,30 @@ cudaError_t sort_events(const RawEvent* ev, uint32_t n, RawEvent* out, void* scr
   void* temp = base + l.temp;
   size_t temp_bytes = l.temp_bytes;
   const unsigned grid = (n + 255) / 256;
-  pixel_keys_kernel<<<grid, 256, 0, stream>>>(ev, n, k32_in, idx_a);
-  cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k32_in, k32_out, idx_a, idx_b,
-                                                  static_cast<int>(n), 0, 32, stream);
-  if (e != cudaSuccess) return e;
-  time_keys_kernel<<<grid, 256, 0, stream>>>(ev, idx_b, n, k64_in);
-  temp_bytes = l.temp_bytes;
-  e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k64_in, k64_out, idx_b, idx_a, static_cast<int>(n), 0, 64,
-                                      stream);
-  if (e != cudaSuccess) return e;
-  gather_events_kernel<<<grid, 256, 0, stream>>>(ev, idx_a, n, out);
+  const uint32_t* order = nullptr;
+  const int pixel_bits = bits_of(span.pixels == 0 ? 0 : span.pixels - 1u);
+  const int time_bits = span.hi >= span.lo ? bits_of(static_cast<uint64_t>(span.hi) - static_cast<uint64_t>(span.lo)) : 64;
+  if (time_bits + pixel_bits <= 64) {
+    span_keys_kernel<<<grid, 256, 0, stream>>>(ev, n, span.lo, pixel_bits, k64_in, idx_a);
+    const cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k64_in, k64_out, idx_a, idx_b,
+                                                          static_cast<int>(n), 0, time_bits + pixel_bits, stream);
+    if (e != cudaSuccess) return e;
+    order = idx_b;
+  } else {
+    uint32_t* k32_in = reinterpret_cast<uint32_t*>(base + l.k32_in);
+    uint32_t* k32_out = reinterpret_cast<uint32_t*>(base + l.k32_out);
+    pixel_keys_kernel<<<grid, 256, 0, stream>>>(ev, n, k32_in, idx_a);
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k32_in, k32_out, idx_a, idx_b,
+                                                    static_cast<int>(n), 0, 32, stream);
+    if (e != cudaSuccess) return e;
+    time_keys_kernel<<<grid, 256, 0, stream>>>(ev, idx_b, n, k64_in);
+    temp_bytes = l.temp_bytes;
+    e = cub::DeviceRadixSort::SortPairs(temp, temp_bytes, k64_in, k64_out, idx_b, idx_a, static_cast<int>(n), 0, 64,
+                                        stream);
+    if (e != cudaSuccess) return e;
+    order = idx_a;
+  }
+  put_events_kernel<<<grid, 256, 0, stream>>>(ev, order, n, out);
   return cudaGetLastError();
 }
 

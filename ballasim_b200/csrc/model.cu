@@ -270,6 +270,7 @@ struct Model {
   DevBuf<RawEvent> events;
   size_t event_cap = 0;
   size_t last_events = 0;      // events of the last device call (on the device)
+  int64_t events_lo = 0, events_hi = -1;  // the times `events` holds (of the last call that wrote it)
   std::vector<RawEvent> kept;  // host-kept events (advance_runs, engine runs)
   // staging for host runs
   DevBuf<uint32_t> s_pixel;
@@ -664,6 +665,8 @@ struct Model {
       stat_samples += c[kCntSamples];
       stat_noise += c[kCntNoise];
       last_events = static_cast<size_t>(c[kCntEvents]);
+      events_lo = t_state;
+      events_hi = t_end;
       cur = 1 - cur;
       t_state = t_end;
       fresh = false;
@@ -695,6 +698,11 @@ struct Model {
     kept = download(events.p, last_events, own);
   }
 
+  // The model's own events lie in the call's times; nothing is known of another array's.
+  EventSpan span_of(const RawEvent* dev) const {
+    return dev == events.p ? EventSpan{events_lo, events_hi, n} : EventSpan{0, -1, uint64_t{1} << 32};
+  }
+
   // The events of a call, sorted by (t_cross, pixel) on the device (finish_events' order) and copied into pinned
   // host memory; the pointer stays valid until the next download.
   const RawEvent* download_pinned(const RawEvent* dev, size_t count, cudaStream_t s) const {
@@ -704,7 +712,7 @@ struct Model {
       const uint32_t n = static_cast<uint32_t>(count);
       sorted.ensure(count);
       sort_scratch.ensure(sort_events_scratch_bytes(n));
-      CK(sort_events(dev, n, sorted.p, sort_scratch.p, s));
+      CK(sort_events(dev, n, span_of(dev), EventsOut{sorted.p, {}, width, readout()}, sort_scratch.p, s));
       CK(cudaMemcpyAsync(staged.p, sorted.p, count * sizeof(RawEvent), cudaMemcpyDeviceToHost, s));
       CK(cudaStreamSynchronize(s));
     }
@@ -747,10 +755,7 @@ struct Model {
     if (count == 0) return false;
     if (count > 0x7fffffffull) throw std::invalid_argument("too many events in one call");
     const uint32_t n = static_cast<uint32_t>(count);
-    sorted.ensure(count);
     sort_scratch.ensure(sort_events_scratch_bytes(n));
-    CK(cudaEventRecord(take_timer.a, s));
-    CK(sort_events(dev, n, sorted.p, sort_scratch.p, s));
     Col cols[12] = {{o->pixel, 4, 0},      {o->x, 2, 0},     {o->y, 2, 0},  {o->p, 1, 0},
                     {o->t_cross_ns, 8, 0}, {o->t_reported_ns, 8, 0},        {o->label, 1, 0},
                     {o->flags, 2, 0},      {o->ds, 4, 0},    {o->dn, 4, 0}, {o->dl, 4, 0},
@@ -772,7 +777,8 @@ struct Model {
                             static_cast<uint8_t*>(at(6)), static_cast<uint16_t*>(at(7)),
                             static_cast<float*>(at(8)),   static_cast<float*>(at(9)),
                             static_cast<float*>(at(10)),  static_cast<float*>(at(11))};
-    CK(event_columns(sorted.p, n, width, readout(), d, s));
+    CK(cudaEventRecord(take_timer.a, s));
+    CK(sort_events(dev, n, span_of(dev), EventsOut{nullptr, d, width, readout()}, sort_scratch.p, s));
     CK(cudaEventRecord(take_timer.b, s));
     CK(cudaMemcpyAsync(col_pin.p, col_dev.p, total, cudaMemcpyDeviceToHost, s));
     CK(cudaEventRecord(take_timer_copy.b, s));
@@ -1915,6 +1921,8 @@ struct Engine {
         m->launch_ms_max = std::max(m->launch_ms_max, static_cast<double>(ms));
         m->last_events = static_cast<size_t>(c[kCntEvents]);
         m->kept.clear();
+        m->events_lo = t0;
+        m->events_hi = t0 + static_cast<int64_t>(windows) * kWindowNs;
         m->cur = 1 - m->cur;
         m->t_state = t0 + static_cast<int64_t>(windows) * kWindowNs;
         m->fresh = false;

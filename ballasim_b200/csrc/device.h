@@ -169,7 +169,8 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
                    int32_t w0, int32_t w1, const SamplerRules& r, unsigned int* tile_counter, int blocks,
                    int warps_per_block, int stage, int tile_lw, int cascade, cudaStream_t stream);
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
-// The split engine (stage kStageSplit): split_begin_kernel, then per window split_window_kernel (blocks x
+// The split engine (stage kStageSplit). solo: the whole call in split_solo_kernel, up to `blocks` blocks. Else
+// split_begin_kernel, then per window split_window_kernel (blocks x
 // warps_per_block warps over the tiles) and split_rest_kernel (rest_blocks x 128 threads) over the pixels that the first
 // posted to `rest` (rest_capacity records of split_record_bytes(); rest_counts: a word per window, zero before the
 // launch), and split_end_kernel. The state passes from S.in to S.out (carried_in to carried_out). tile0: the sensors'
@@ -180,7 +181,8 @@ size_t split_record_bytes();
 void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,
                          uint32_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
                          void* rest, unsigned int* rest_counts, unsigned int rest_capacity, int blocks,
-                         int warps_per_block, int tile_lw, int rest_blocks, cudaStream_t stream);
+                         int warps_per_block, int tile_lw, int rest_blocks, bool solo, cudaStream_t stream);
+int split_solo_blocks_per_sm(int warps_per_block);
 int split_window_blocks_per_sm(int warps_per_block);
 int split_rest_blocks_per_sm();
 // The fused engine with the learned step proposal (BF16 MLP operands and FP32 parameters in device memory):

@@ -86,11 +86,26 @@ struct SplitArgs {
   SamplerRules r;
   uint32_t tile_lw;
   uint32_t total_blobs;
+  uint32_t block_tiles;  // split_solo_kernel: the tiles of a block
   QuickPlanes q;
   SplitPixel* px;
   float4* boxes;  // this window's blob boxes (total_blobs), and the next one's (written by the rest kernel)
   float4* boxes_next;
   uint32_t tile0[kTile0Args];
+};
+
+// Window w of the call: its start, and its start and end since the call's start in seconds.
+struct WindowTimes {
+  int32_t w;
+  int64_t T0, T_end, t_w;
+  float tau_a, tau_b;
+  __device__ __forceinline__ WindowTimes(const SplitArgs& a, int32_t w_) : w(w_) {
+    T0 = *a.t0;
+    T_end = T0 + static_cast<int64_t>(a.windows) * kWindowNs;
+    t_w = T0 + static_cast<int64_t>(w) * kWindowNs;
+    tau_a = static_cast<float>(static_cast<double>(t_w - T0) * 1e-9);
+    tau_b = static_cast<float>(static_cast<double>(t_w - T0 + kWindowNs) * 1e-9);
+  }
 };
 
 __device__ __forceinline__ int sensor_of(const SplitArgs& a, uint32_t tile) {
@@ -109,21 +124,23 @@ __device__ __forceinline__ int sensor_of(const SplitArgs& a, uint32_t tile) {
   return si;
 }
 
-// Every blob's box for the window at t_w: where its 6 r disc, swept over the window, can be (a 1 px margin covers the
-// fp32 rounding of the per-sample test). The blobs of the whole call, over the launch's threads.
+// A blob's box for the window at t_w: where its 6 r disc, swept over the window, can be (a 1 px margin covers the fp32
+// rounding of the per-sample test): x from .x to .y, y from .z to .w.
+__device__ __forceinline__ float4 blob_box(const FieldDev& f, uint32_t k, float ta, float tb) {
+  const float* b = f.blobs + static_cast<size_t>(k) * kBlobWords;
+  const float cxa = b[1] + b[3] * ta, cxb = b[1] + b[3] * tb;
+  const float cya = b[2] + b[4] * ta, cyb = b[2] + b[4] * tb;
+  const float reach = sqrtf(b[6]) + 1.0f;
+  return make_float4(fminf(cxa, cxb) - reach, fmaxf(cxa, cxb) + reach, fminf(cya, cyb) - reach, fmaxf(cya, cyb) + reach);
+}
+// All sensors' boxes, over the launch's threads.
 __device__ __forceinline__ void write_boxes(const SplitArgs& a, int64_t t_w, float4* boxes) {
   const float ta = t_seconds(t_w), tb = t_seconds(t_w + kWindowNs);
   for (int si = 0; si < a.n_sensors; ++si) {
     const EngineSensor& S = a.sensors[si];
-    const FieldDev& f = S.field;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < static_cast<uint32_t>(f.n_blobs);
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < static_cast<uint32_t>(S.field.n_blobs);
          k += gridDim.x * blockDim.x) {
-      const float* b = f.blobs + static_cast<size_t>(k) * kBlobWords;
-      const float cxa = b[1] + b[3] * ta, cxb = b[1] + b[3] * tb;
-      const float cya = b[2] + b[4] * ta, cyb = b[2] + b[4] * tb;
-      const float reach = sqrtf(b[6]) + 1.0f;
-      boxes[S.blob0 + k] = make_float4(fminf(cxa, cxb) - reach, fmaxf(cxa, cxb) + reach, fminf(cya, cyb) - reach,
-                                       fmaxf(cya, cyb) + reach);
+      boxes[S.blob0 + k] = blob_box(S.field, k, ta, tb);
     }
   }
 }
@@ -181,12 +198,9 @@ __device__ __forceinline__ void skip_rejected(const SensorConsts& k, uint32_t pi
   }
 }
 
-__global__ void __launch_bounds__(128) split_begin_kernel(const __grid_constant__ SplitArgs a) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// The records of one tile.
+__device__ __forceinline__ void begin_tile(const SplitArgs& a, uint32_t tile, uint32_t lane) {
   const int64_t T0 = *a.t0, T_end = T0 + static_cast<int64_t>(a.windows) * kWindowNs;
-  write_boxes(a, T0, a.boxes);
-  if (tile >= a.total_tiles) return;
   const EngineSensor& S = a.sensors[sensor_of(a, tile)];
   uint32_t x, y;
   tile_xy(tile - S.tile0, S.tiles_x, a.tile_lw, lane, x, y);
@@ -249,12 +263,9 @@ __global__ void __launch_bounds__(128) split_begin_kernel(const __grid_constant_
   if (lane == 0u && sum != 0u) atomicAdd(&S.counters[kCntNoise], static_cast<unsigned long long>(sum));
 }
 
-// The call's output: every pixel's state, its search at least at the call's end (a quiet window moves it to its own),
-// the held and the carried sample.
-__global__ void __launch_bounds__(128) split_end_kernel(const __grid_constant__ SplitArgs a) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (tile >= a.total_tiles) return;
+// The output of one tile: every pixel's state, its search at least at the call's end (a quiet window moves it to its
+// own), the held and the carried sample.
+__device__ __forceinline__ void end_tile(const SplitArgs& a, uint32_t tile, uint32_t lane) {
   const EngineSensor& S = a.sensors[sensor_of(a, tile)];
   uint32_t x, y;
   tile_xy(tile - S.tile0, S.tiles_x, a.tile_lw, lane, x, y);
@@ -278,6 +289,16 @@ __global__ void __launch_bounds__(128) split_end_kernel(const __grid_constant__ 
   s.n_ba = r.n_ba;
   store_state(S.out, p, S.consts.noise != 0, s);
   S.carried_out[p] = carried;
+}
+
+__global__ void __launch_bounds__(128) split_begin_kernel(const __grid_constant__ SplitArgs a) {
+  const uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  write_boxes(a, *a.t0, a.boxes);
+  if (tile < a.total_tiles) begin_tile(a, tile, threadIdx.x & 31u);
+}
+__global__ void __launch_bounds__(128) split_end_kernel(const __grid_constant__ SplitArgs a) {
+  const uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (tile < a.total_tiles) end_tile(a, tile, threadIdx.x & 31u);
 }
 
 // exp_f for x in [-80, 0] (no range test, one exact scaling step): the same operations, so the same bits. The rounding
@@ -343,202 +364,179 @@ __device__ __noinline__ uint32_t walk_refined(const SamplerRules* r, const Field
                              });
 }
 
-// Window a.w of every tile.
-__global__ void __launch_bounds__(128, 8) split_window_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
+// One window of one tile, by a warp: the quiet pixels' carried samples, the others' records in rl. n_samples, n_clean:
+// the lane's samples staged and its clean segments. kBoxes: the blobs' boxes of the window are in a.boxes; else they are
+// formed here.
+template <bool kBoxes>
+__device__ __forceinline__ void window_tile(const SplitArgs& a, const RestList& rl, const WindowTimes& wt, WarpShared& w,
+                                            const EngineSensor& S, int si, uint32_t tile, uint32_t lane,
+                                            unsigned long long& n_samples, unsigned long long& n_clean) {
   const unsigned full = 0xffffffffu;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  __shared__ WarpShared sh[4];
-  WarpShared& w = sh[warp];
-  const int64_t t_w = *a.t0 + static_cast<int64_t>(a.w) * kWindowNs;
-  const float tau_a = static_cast<float>(static_cast<double>(static_cast<int64_t>(a.w) * kWindowNs) * 1e-9);
-  const float tau_b = static_cast<float>(static_cast<double>((static_cast<int64_t>(a.w) + 1) * kWindowNs) * 1e-9);
+  const int64_t t_w = wt.t_w;
   const float tol_lo = a.r.tol - 0x1p-20f * fabs_f(a.r.tol);
-  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
-  // The block's samples and clean segments per sensor, added to the sensors' counters once at the end (one atomic per
-  // warp and sensor would take longer than the kernel: atomics on one address pass one at a time).
-  __shared__ unsigned long long sums[kTile0Args][2];
-  for (int q = static_cast<int>(threadIdx.x); q < 2 * kTile0Args; q += static_cast<int>(blockDim.x)) {
-    sums[q / 2][q % 2] = 0ull;
-  }
-  __syncthreads();
-  int counted = -1;  // the sensor whose samples and clean segments n_samples and n_clean count
-  unsigned long long n_samples = 0, n_clean = 0;
-  const auto flush = [&]() {
-    if (counted >= 0) {
-      if (a.n_sensors <= kTile0Args) {
-        warp_add(&sums[counted][0], n_samples);
-        warp_add(&sums[counted][1], n_clean);
-      } else {
-        unsigned long long* cnt = a.sensors[counted].counters;
-        warp_add(&cnt[kCntSamples], n_samples);
-        warp_add(&cnt[kCntPieces], n_clean);
-        warp_add(&cnt[kCntLeaves], n_clean);
+  uint32_t x, y;
+  tile_xy(tile - S.tile0, S.tiles_x, a.tile_lw, lane, x, y);
+  const bool have = x < S.width && y < S.height;
+  const uint32_t slot = tile * 32u + lane;
+  const float4 qa = a.q.a[slot];
+  const float2 qb = a.q.b[slot];
+  const float carried = a.q.c[slot];
+  const FieldDev& f = S.field;
+  const float xc = static_cast<float>(x) + 0.5f, yc = static_cast<float>(y) + 0.5f;
+  // The blobs in reach of the tile during the window, in blob order; n_list < 0: no list (a tanh edge, more than
+  // kMaxListed, or a table whose 1 / (2 r^2) and (6 r)^2 leave exp_neg's range).
+  int n_list = f.kind == kFieldBlobs && f.listable ? 0 : -1;
+  if (n_list == 0) {
+    const uint32_t tx = __shfl_sync(full, x, 0), ty = __shfl_sync(full, y, 0);
+    const float bx0 = static_cast<float>(tx) + 0.5f, bx1 = static_cast<float>(tx + (1u << a.tile_lw)) - 0.5f;
+    const float by0 = static_cast<float>(ty) + 0.5f, by1 = static_cast<float>(ty + (32u >> a.tile_lw)) - 0.5f;
+    const float ta = t_seconds(t_w), tb = t_seconds(t_w + kWindowNs);
+    for (int32_t base = 0; base < f.n_blobs; base += 32) {
+      const int32_t k = base + static_cast<int32_t>(lane);
+      bool keep = false;
+      if (k < f.n_blobs) {
+        const float4 b = kBoxes ? a.boxes[S.blob0 + k] : blob_box(f, static_cast<uint32_t>(k), ta, tb);
+        keep = !(b.y < bx0 || b.x > bx1 || b.w < by0 || b.z > by1);
       }
-    }
-    n_samples = n_clean = 0;
-  };
-  for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + warp; tile < a.total_tiles; tile += warps) {
-    const int si = sensor_of(a, tile);
-    const EngineSensor& S = a.sensors[si];
-    if (si != counted) {
-      flush();
-      counted = si;
-    }
-    uint32_t x, y;
-    tile_xy(tile - S.tile0, S.tiles_x, a.tile_lw, lane, x, y);
-    const bool have = x < S.width && y < S.height;
-    const uint32_t slot = tile * 32u + lane;
-    const float4 qa = a.q.a[slot];
-    const float2 qb = a.q.b[slot];
-    const float carried = a.q.c[slot];
-    const FieldDev& f = S.field;
-    const float xc = static_cast<float>(x) + 0.5f, yc = static_cast<float>(y) + 0.5f;
-    // The blobs in reach of the tile during the window, in blob order; n_list < 0: no list (a tanh edge, more than
-    // kMaxListed, or a table whose 1 / (2 r^2) and (6 r)^2 leave exp_neg's range).
-    int n_list = f.kind == kFieldBlobs && f.listable ? 0 : -1;
-    if (n_list == 0) {
-      const uint32_t tx = __shfl_sync(full, x, 0), ty = __shfl_sync(full, y, 0);
-      const float bx0 = static_cast<float>(tx) + 0.5f, bx1 = static_cast<float>(tx + (1u << a.tile_lw)) - 0.5f;
-      const float by0 = static_cast<float>(ty) + 0.5f, by1 = static_cast<float>(ty + (32u >> a.tile_lw)) - 0.5f;
-      for (int32_t base = 0; base < f.n_blobs; base += 32) {
-        const int32_t k = base + static_cast<int32_t>(lane);
-        bool keep = false;
-        if (k < f.n_blobs) {
-          const float4 b = a.boxes[S.blob0 + k];
-          keep = !(b.y < bx0 || b.x > bx1 || b.w < by0 || b.z > by1);
-        }
-        const uint32_t bits = __ballot_sync(full, keep);
-        if (n_list + __popc(bits) > kMaxListed) {
-          n_list = -1;
-          break;
-        }
-        if (keep) w.list[n_list + __popc(bits & ((1u << lane) - 1u))] = static_cast<uint16_t>(k);
-        n_list += __popc(bits);
+      const uint32_t bits = __ballot_sync(full, keep);
+      if (n_list + __popc(bits) > kMaxListed) {
+        n_list = -1;
+        break;
       }
-      __syncwarp();
-    }
-    const bool listed = n_list >= 0 && n_list <= kCentres;  // else each lane evaluates its own samples
-    // The level rule (field_level), the centres at the window's start shared by the warp.
-    int level = a.r.l_min;
-    if (n_list != 0 && f.kind == kFieldBlobs) {
-      level = field_level(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t_w,
-                          a.r.l_min, a.r.l_max);
-    }
-    // The lattice: slot j of the tile's finest level, at every lane whose own level has it. A lane whose level holds
-    // more than kSplitStage samples is posted whole.
-    const bool fits = have && (1 << level) <= kSplitStage;
-    const int fine = static_cast<int>(__reduce_max_sync(full, static_cast<unsigned>(fits ? level : 0)));
-    const int slots = 1 << fine;
-    const int skip = fits ? (1 << (fine - level)) - 1 : -1;  // a slot is the lane's own where (j & skip) == 0
-    float p2 = carried, p1 = carried, v_lo = carried, v_hi = carried;
-    bool flagged = false;
-    uint32_t n = 1;
-    const int group = listed && n_list > 0 ? kCentres / n_list : slots;
-    for (int j0 = 1; j0 <= slots; j0 += group) {
-      const int j1 = j0 + group <= slots + 1 ? j0 + group : slots + 1;
-      if (listed && n_list > 0) {
-        __syncwarp();
-        const int entries = (j1 - j0) * n_list;
-        for (int q = static_cast<int>(lane); q < entries; q += 32) {
-          const int i = q % n_list, j = j0 + q / n_list;
-          const float* b = f.blobs + static_cast<size_t>(w.list[i]) * kBlobWords;
-          const float ts = t_seconds(t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine)));
-          w.centre[q] = make_float4(b[1] + b[3] * ts, b[2] + b[4] * ts, b[5], b[6]);
-          w.amp[q] = b[0];
-        }
-        __syncwarp();
-      }
-      for (int j = j0; j < j1; ++j) {
-        const bool mine = fits && (j & skip) == 0;
-        float e = f.base;
-        if (listed) {
-          const int c0 = (j - j0) * n_list;
-          for (int i = 0; i < n_list; ++i) {
-            const float4 c = w.centre[c0 + i];
-            const float dx = xc - c.x, dy = yc - c.y;
-            const float d2 = dx * dx + dy * dy;
-            const bool in = d2 < c.w;
-            const float term = w.amp[c0 + i] * exp_neg(in ? -(d2 * c.z) : 0.0f);
-            e = e + (in ? term : 0.0f);
-          }
-        } else if (mine) {
-          const int64_t t = t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine));
-          e = field_eval(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t);
-        }
-        if (mine) {
-          if (n >= 2u) flagged = flagged || (a.r.midpoint != 0 && exceeds_fast(a.r, tol_lo, p2, p1, e));
-          w.v[n - 1u][lane] = e;
-          ++n;
-          p2 = p1;
-          p1 = e;
-          v_lo = min_nan(v_lo, e);
-          v_hi = max_nan(v_hi, e);
-        }
-      }
-    }
-    float last = p1;
-    // A flagged interval refines where it can still be split: such lanes walk the window in the general form.
-    const bool refine = fits && flagged && (static_cast<uint32_t>(kWindowNs) >> level) >= a.r.min_split &&
-                        a.r.max_refine_levels > 0;
-    bool staged = fits;
-    if (refine) {
-      n = walk_refined(&a.r, &f, w.list, n_list, x, y, t_w, level, carried, &w.v[0][lane], &w.dt[0][lane]);
-      staged = n - 1u <= static_cast<uint32_t>(kSplitStage);
-      if (staged) {
-        for (uint32_t q = 0; q + 1u < n; ++q) {
-          const float e = w.v[q][lane];
-          v_lo = min_nan(v_lo, e);
-          v_hi = max_nan(v_hi, e);
-          last = e;
-        }
-      }
-    }
-    if (staged) n_samples += n;
-    // Quiet: the whole window clean by the bounds (NaN answers no); segments of one or two ns count no node in the
-    // model, so a refined window that can hold them is posted.
-    const float I_hi = qb.x + qb.y * v_hi, I_lo = qb.x + qb.y * v_lo;
-    const float pad = 0x1p-21f * I_hi;
-    const bool quiet = staged && a.w < __float_as_int(qa.w) && v_lo >= 0.0f && v_hi <= S.consts.irr_max &&
-                       __log2f(I_hi + pad) < qa.x - qa.z * tau_b && __log2f(I_lo - pad) > qa.y - qa.z * tau_a &&
-                       !(refine && a.r.min_split <= 4u);
-    if (quiet) {
-      n_clean += n - 1u;
-      a.q.c[slot] = last;
-    }
-    // One record per posted pixel, the warp's records reserved together.
-    const bool post = have && !quiet;
-    const unsigned posting = __ballot_sync(full, post);
-    if (posting != 0u) {
-      const int leader = __ffs(posting) - 1;
-      unsigned int base = 0;
-      if (static_cast<int>(lane) == leader) base = atomicAdd(rl.count, static_cast<unsigned int>(__popc(posting)));
-      base = __shfl_sync(full, base, leader);
-      if (post) {
-        const unsigned int i = base + static_cast<unsigned int>(__popc(posting & ((1u << lane) - 1u)));
-        if (i >= rl.capacity) {
-          atomicOr(&S.counters[kCntErrors], kErrRestList);
-        } else {
-          const uint32_t left = staged ? n - 1u : kRestWhole;
-          RestRecord& rec = rl.rec[i];
-          rec.slot = slot;
-          rec.pixel = y * S.width + x;
-          rec.tag = static_cast<uint32_t>(si) | left << 16 | static_cast<uint32_t>(level) << 24 |
-                    (refine ? 0x80000000u : 0u);
-          if (staged) {
-            for (uint32_t u = 0; u < left; ++u) {
-              rec.v[u] = w.v[u][lane];
-              if (refine) rl.times[i].dt[u] = w.dt[u][lane];
-            }
-          }
-        }
-      }
+      if (keep) w.list[n_list + __popc(bits & ((1u << lane) - 1u))] = static_cast<uint16_t>(k);
+      n_list += __popc(bits);
     }
     __syncwarp();
   }
-  flush();
-  __syncthreads();
-  if (static_cast<int>(threadIdx.x) < a.n_sensors && a.n_sensors <= kTile0Args) {
-    const unsigned long long n = sums[threadIdx.x][0], clean = sums[threadIdx.x][1];
+  const bool listed = n_list >= 0 && n_list <= kCentres;  // else each lane evaluates its own samples
+  // The level rule (field_level), the centres at the window's start shared by the warp.
+  int level = a.r.l_min;
+  if (n_list != 0 && f.kind == kFieldBlobs) {
+    level = field_level(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t_w,
+                        a.r.l_min, a.r.l_max);
+  }
+  // The lattice: slot j of the tile's finest level, at every lane whose own level has it. A lane whose level holds
+  // more than kSplitStage samples is posted whole.
+  const bool fits = have && (1 << level) <= kSplitStage;
+  const int fine = static_cast<int>(__reduce_max_sync(full, static_cast<unsigned>(fits ? level : 0)));
+  const int slots = 1 << fine;
+  const int skip = fits ? (1 << (fine - level)) - 1 : -1;  // a slot is the lane's own where (j & skip) == 0
+  float p2 = carried, p1 = carried, v_lo = carried, v_hi = carried;
+  bool flagged = false;
+  uint32_t n = 1;
+  const int group = listed && n_list > 0 ? kCentres / n_list : slots;
+  for (int j0 = 1; j0 <= slots; j0 += group) {
+    const int j1 = j0 + group <= slots + 1 ? j0 + group : slots + 1;
+    if (listed && n_list > 0) {
+      __syncwarp();
+      const int entries = (j1 - j0) * n_list;
+      for (int q = static_cast<int>(lane); q < entries; q += 32) {
+        const int i = q % n_list, j = j0 + q / n_list;
+        const float* b = f.blobs + static_cast<size_t>(w.list[i]) * kBlobWords;
+        const float ts = t_seconds(t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine)));
+        w.centre[q] = make_float4(b[1] + b[3] * ts, b[2] + b[4] * ts, b[5], b[6]);
+        w.amp[q] = b[0];
+      }
+      __syncwarp();
+    }
+    for (int j = j0; j < j1; ++j) {
+      const bool mine = fits && (j & skip) == 0;
+      float e = f.base;
+      if (listed) {
+        const int c0 = (j - j0) * n_list;
+        for (int i = 0; i < n_list; ++i) {
+          const float4 c = w.centre[c0 + i];
+          const float dx = xc - c.x, dy = yc - c.y;
+          const float d2 = dx * dx + dy * dy;
+          const bool in = d2 < c.w;
+          const float term = w.amp[c0 + i] * exp_neg(in ? -(d2 * c.z) : 0.0f);
+          e = e + (in ? term : 0.0f);
+        }
+      } else if (mine) {
+        const int64_t t = t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine));
+        e = field_eval(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t);
+      }
+      if (mine) {
+        if (n >= 2u) flagged = flagged || (a.r.midpoint != 0 && exceeds_fast(a.r, tol_lo, p2, p1, e));
+        w.v[n - 1u][lane] = e;
+        ++n;
+        p2 = p1;
+        p1 = e;
+        v_lo = min_nan(v_lo, e);
+        v_hi = max_nan(v_hi, e);
+      }
+    }
+  }
+  float last = p1;
+  // A flagged interval refines where it can still be split: such lanes walk the window in the general form.
+  const bool refine = fits && flagged && (static_cast<uint32_t>(kWindowNs) >> level) >= a.r.min_split &&
+                      a.r.max_refine_levels > 0;
+  bool staged = fits;
+  if (refine) {
+    n = walk_refined(&a.r, &f, w.list, n_list, x, y, t_w, level, carried, &w.v[0][lane], &w.dt[0][lane]);
+    staged = n - 1u <= static_cast<uint32_t>(kSplitStage);
+    if (staged) {
+      for (uint32_t q = 0; q + 1u < n; ++q) {
+        const float e = w.v[q][lane];
+        v_lo = min_nan(v_lo, e);
+        v_hi = max_nan(v_hi, e);
+        last = e;
+      }
+    }
+  }
+  if (staged) n_samples += n;
+  // Quiet: the whole window clean by the bounds (NaN answers no); segments of one or two ns count no node in the
+  // model, so a refined window that can hold them is posted.
+  const float I_hi = qb.x + qb.y * v_hi, I_lo = qb.x + qb.y * v_lo;
+  const float pad = 0x1p-21f * I_hi;
+  const bool quiet = staged && wt.w < __float_as_int(qa.w) && v_lo >= 0.0f && v_hi <= S.consts.irr_max &&
+                     __log2f(I_hi + pad) < qa.x - qa.z * wt.tau_b && __log2f(I_lo - pad) > qa.y - qa.z * wt.tau_a &&
+                     !(refine && a.r.min_split <= 4u);
+  if (quiet) {
+    n_clean += n - 1u;
+    a.q.c[slot] = last;
+  }
+  // One record per posted pixel, the warp's records reserved together.
+  const bool post = have && !quiet;
+  const unsigned posting = __ballot_sync(full, post);
+  if (posting != 0u) {
+    const int leader = __ffs(posting) - 1;
+    unsigned int base = 0;
+    if (static_cast<int>(lane) == leader) base = atomicAdd(rl.count, static_cast<unsigned int>(__popc(posting)));
+    base = __shfl_sync(full, base, leader);
+    if (post) {
+      const unsigned int i = base + static_cast<unsigned int>(__popc(posting & ((1u << lane) - 1u)));
+      if (i >= rl.capacity) {
+        atomicOr(&S.counters[kCntErrors], kErrRestList);
+      } else {
+        const uint32_t left = staged ? n - 1u : kRestWhole;
+        RestRecord& rec = rl.rec[i];
+        rec.slot = slot;
+        rec.pixel = y * S.width + x;
+        rec.tag = static_cast<uint32_t>(si) | left << 16 | static_cast<uint32_t>(level) << 24 |
+                  (refine ? 0x80000000u : 0u);
+        if (staged) {
+          for (uint32_t u = 0; u < left; ++u) {
+            rec.v[u] = w.v[u][lane];
+            if (refine) rl.times[i].dt[u] = w.dt[u][lane];
+          }
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// A block's samples and clean segments per sensor, added to the sensors' counters once at the end (one atomic per warp
+// and sensor would take longer than the kernel: atomics on one address pass one at a time).
+struct SplitSums {
+  unsigned long long v[kTile0Args][2];
+  __device__ __forceinline__ void clear() {
+    for (int q = static_cast<int>(threadIdx.x); q < 2 * kTile0Args; q += static_cast<int>(blockDim.x)) v[q / 2][q % 2] = 0ull;
+  }
+  __device__ __forceinline__ void add(const SplitArgs& a) const {
+    if (static_cast<int>(threadIdx.x) >= a.n_sensors || a.n_sensors > kTile0Args) return;
+    const unsigned long long n = v[threadIdx.x][0], clean = v[threadIdx.x][1];
     unsigned long long* cnt = a.sensors[threadIdx.x].counters;
     if (n) atomicAdd(&cnt[kCntSamples], n);
     if (clean) {
@@ -546,6 +544,50 @@ __global__ void __launch_bounds__(128, 8) split_window_kernel(const __grid_const
       atomicAdd(&cnt[kCntLeaves], clean);
     }
   }
+};
+// A warp's share of them, for the sensor it is at.
+struct WarpSums {
+  int counted = -1;
+  unsigned long long samples = 0, clean = 0;
+  __device__ __forceinline__ void flush(const SplitArgs& a, SplitSums& sums) {
+    if (counted >= 0) {
+      if (a.n_sensors <= kTile0Args) {
+        warp_add(&sums.v[counted][0], samples);
+        warp_add(&sums.v[counted][1], clean);
+      } else {
+        unsigned long long* cnt = a.sensors[counted].counters;
+        warp_add(&cnt[kCntSamples], samples);
+        warp_add(&cnt[kCntPieces], clean);
+        warp_add(&cnt[kCntLeaves], clean);
+      }
+    }
+    samples = clean = 0;
+  }
+  __device__ __forceinline__ void of(const SplitArgs& a, SplitSums& sums, int si) {
+    if (si == counted) return;
+    flush(a, sums);
+    counted = si;
+  }
+};
+
+// Window a.w of every tile.
+__global__ void __launch_bounds__(128, 8) split_window_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  __shared__ WarpShared sh[4];
+  __shared__ SplitSums sums;
+  sums.clear();
+  __syncthreads();
+  const WindowTimes wt(a, a.w);
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  WarpSums mine;
+  for (uint32_t tile = blockIdx.x * (blockDim.x >> 5) + warp; tile < a.total_tiles; tile += warps) {
+    const int si = sensor_of(a, tile);
+    mine.of(a, sums, si);
+    window_tile<true>(a, rl, wt, sh[warp], a.sensors[si], si, tile, lane, mine.samples, mine.clean);
+  }
+  mine.flush(a, sums);
+  __syncthreads();
+  sums.add(a);
 }
 
 // A window posted whole (more samples than the stage holds), out of line: walked from its start with every blob of the
@@ -745,294 +787,337 @@ struct RestPixel {
   }
 };
 
-// The posted pixels of window a.w, one thread each. A lane steps through its window (quiet segments by the quick
+// Record i of the posted pixels of a window, by one thread. A lane steps through its window (quiet segments by the quick
 // bounds, the refractory release, noise candidates) until it needs a crossing search or is done; the warp's lanes then
 // search together (a loop that searched inside the step, at each lane's own segment, took 15.1 ms of rest kernels on
-// 346x260, 239 windows, against 4.1). Where the list is shorter than the launch, each warp takes fewer records (a power
-// of two of its lanes), since what one pixel does hardly ever falls together with what its neighbour does. 128
-// registers (4 blocks per SM): 5.90 ms of engine time there, 6.17 at 5 blocks, 6.58 at 6.
+// 346x260, 239 windows, against 4.1).
+__device__ __forceinline__ void rest_pixel(const SplitArgs& a, const RestList& rl, const WindowTimes& wt, unsigned int i,
+                                           unsigned int lane) {
+  const int64_t T0 = wt.T0, T_end = wt.T_end, t_w = wt.t_w;
+  const float tau_a = wt.tau_a, tau_b = wt.tau_b;
+  const RestRecord& rec = rl.rec[i];
+  const uint32_t tag = rec.tag, pixel = rec.pixel, slot = rec.slot;
+  const uint32_t left = tag >> 16 & 0xFFu;
+  const int level = static_cast<int>(tag >> 24 & 0x7Fu);
+  const bool timed = (tag & 0x80000000u) != 0u;
+  const EngineSensor& S = a.sensors[tag & 0xFFFFu];
+  const SensorConsts& k = S.consts;
+  const bool noise = k.noise != 0;
+  float raw = a.q.c[slot];
+  const SplitPixel px = a.px[slot];
+  // Quiet windows moved the search to their ends; the held sample is the carried one.
+  PixelRegs s{px.t_ref, maxi(px.t_search, t_w), px.blind_until, px.s3_ref, px.n3_ref, px.dr_ref, px.i_scale,
+              clamp_irr(raw, k.irr_max), px.flags, px.t_shot, px.t_ba, px.n_shot, px.n_ba};
+  const PixelMapRegs m{px.theta_on, px.theta_off, px.leak, px.dark, px.scale, px.ba_rate_hz, px.shot_max_hz};
+  int64_t later_t0 = px.later_t[0], later_t1 = px.later_t[1];
+  uint32_t later_n0 = px.later_n[0], later_n1 = px.later_n[1];
+  PixelCounters c;
+  if (left == kRestWhole) {
+    PixelRegs st = s;  // copies, so that the state itself stays in registers
+    PixelMapRegs mt = m;
+    PixelCounters ct = c;
+    float rt = raw;
+    const uint32_t n = rest_whole(&a, &S, pixel, level, t_w, &st, &mt, &ct, &rt);
+    s = st;
+    c = ct;
+    raw = rt;
+    if (s.n_shot != px.n_shot) later_t0 = later_t1 = -1;
+    atomicAdd(&S.counters[kCntSamples], static_cast<unsigned long long>(n));
+  } else {
+    ThreadSink sink{S.ev, &S.counters[kCntEvents]};
+    RestPixel r{m, s.s3_ref, 0.0f - s.n3_ref, s.dr_ref, s.i_scale, t_w - s.t_ref, 0u, 0u, 0.0f, 0.0f, 0.0f};
+    r.v1 = clamp_irr(raw, k.irr_max);
+    float4 bounds = a.q.a[slot];
+    float x0 = 0.0f, x1 = 0.0f;  // x at the segment's ends, where have_x
+    bool have_x = false;
+    uint32_t q = 0;
+    bool next = true, done = false;
+    for (;;) {
+      // Steps until a search is needed: from `da` (Delta there does not fire) to before `stop`.
+      bool need = false, found = false, on = false;
+      uint32_t da = 0, hit = 0;
+      float xa = 0.0f, x_hit = 0.0f;
+      int64_t stop = 0;
+      int label = -1;
+      while (!done && !need && !found) {
+        if (next) {  // the next sample's segment
+          if (q == left) {
+            done = true;
+            break;
+          }
+          raw = rec.v[q];
+          r.d0 = r.d1;
+          r.v0 = r.v1;
+          r.d1 = timed ? rl.times[i].dt[q]
+                       : (q + 1u) << (static_cast<uint32_t>(kWindowLog2) - static_cast<uint32_t>(level));
+          r.v1 = clamp_irr(raw, k.irr_max);
+          r.inv = __uint_as_float((127u - (31u - static_cast<uint32_t>(__clz(static_cast<int>(r.d1 - r.d0))))) << 23);
+          ++q;
+          ++c.pieces;
+          next = false;
+          have_x = false;
+        }
+        const int64_t t0 = t_w + r.d0, e = t_w + r.d1;
+        const int64_t tn = noise ? mini(s.t_shot, s.t_ba) : kForever;
+        bool cand = false, drop = false;
+        if (s.blind_until != kNotBlind) {
+          cand = drop = s.blind_until >= e ? tn < e : tn <= s.blind_until;
+          if (!cand) {
+            if (s.blind_until >= e) {
+              next = true;
+            } else {  // the release: a new reference at x(t_rel) - eps_ci
+              const uint32_t db = static_cast<uint32_t>(s.blind_until - t_w);
+              r.s3 = r.x_of(r.current(db));
+              r.dn = 0.0f;
+              r.dr = -k.eps_ci;
+              r.since = t_w - s.blind_until;
+              s.t_ref = s.blind_until;
+              s.blind_until = kNotBlind;
+              s.s3_ref = r.s3;
+              s.n3_ref = 0.0f;
+              s.dr_ref = r.dr;
+              bounds = quick_record(s, m, false, T0, T_end);
+            }
+          }
+        } else {
+          const int64_t lo = maxi(s.t_search, t0);
+          stop = mini(e, tn);
+          if (lo < stop) {
+            // Quiet by the bounds (split_window_kernel's test on this segment alone), or by Delta at lo and the
+            // segment's ends (PixelProc::segment_fast's).
+            const float Ia = m.dark + m.scale * r.v0, Ib = m.dark + m.scale * r.v1;
+            const float I_hi = fmaxf(Ia, Ib), I_lo = fminf(Ia, Ib);
+            const float pad = 0x1p-21f * I_hi;
+            bool quiet = __log2f(I_hi + pad) < bounds.x - bounds.z * tau_b &&
+                         __log2f(I_lo - pad) > bounds.y - bounds.z * tau_a;
+            ++c.leaves;
+            if (!quiet) {
+              if (!have_x) {
+                x0 = r.x_of(Ia);
+                x1 = r.x_of(Ib);
+                have_x = true;
+              }
+              da = static_cast<uint32_t>(lo - t_w);
+              xa = lo == t0 ? x0 : r.x_of(r.current(da));
+              const float la = r.dl(da), D = r.delta(xa, la);
+              if (D >= m.theta_on || D <= -m.theta_off) {
+                found = true;
+                hit = da;
+                x_hit = xa;
+                on = D >= m.theta_on;
+              } else if (stop - lo == 1) {
+                quiet = true;
+              } else {
+                if (r.v0 + (r.v1 - r.v0) == r.v1) {
+                  const float top = r.delta(maxr(xa, x1), r.dl(r.d1)), low = r.delta(minr(xa, x1), la);
+                  quiet = top < m.theta_on && low > -m.theta_off;
+                }
+                need = !quiet;
+              }
+            }
+            if (quiet) s.t_search = maxi(s.t_search, stop);
+          } else if (tn >= e) {
+            next = true;
+          } else {
+            cand = true;
+            drop = tn < s.t_search;
+          }
+        }
+        if (cand) {
+          const bool shot = s.t_shot <= s.t_ba;
+          const uint32_t dc = static_cast<uint32_t>(tn - t_w);
+          const float I = drop ? 0.0f : r.current(dc);
+          CandidateOut o;
+          candidate_step(&k, pixel, shot, shot ? s.n_shot : s.n_ba, tn, shot ? m.shot_max_hz : m.ba_rate_hz, drop,
+                         !shot || later_t0 < 0, m.dark, I, &o);
+          ++c.noise_candidates;
+          if (shot && later_t0 >= 0) {  // the chain's next stop
+            s.t_shot = later_t0;
+            s.n_shot = later_n0;
+            later_t0 = later_t1;
+            later_n0 = later_n1;
+            later_t1 = -1;
+          } else if (shot) {  // more stops than the record holds: one candidate on
+            ++s.n_shot;
+            s.t_shot = o.next;
+          } else {
+            ++s.n_ba;
+            s.t_ba = o.next;
+          }
+          if (o.accepted) {
+            found = true;
+            hit = dc;
+            x_hit = r.x_of(I);
+            on = o.on;
+            label = kLabelNoise;
+          }
+        }
+      }
+      if (done) break;
+      if (need) {
+        bool hard = false;
+        const uint32_t end = static_cast<uint32_t>(stop - t_w);
+        found = r.search(da, xa, end, x0, x1, end == r.d1 && r.v0 + (r.v1 - r.v0) == r.v1, hit, x_hit, on, hard,
+                         c.leaves);
+        if (hard) {
+          PixelRegs st = s;
+          st.s3_ref = r.s3;
+          st.n3_ref = 0.0f - r.dn;
+          st.dr_ref = r.dr;
+          NullSink none;
+          PixelMapRegs mt = m;
+          PixelCounters ct;
+          PixelProc<NullSink> proc{st, mt, k, pixel, none, ct};
+          int64_t th = t_w;
+          bool up = false;
+          float xt = 0.0f;
+          found = proc.search(Segment{t_w + r.d0, t_w + r.d1, r.v0, r.v1}, t_w + da, stop, th, up, xt);
+          hit = static_cast<uint32_t>(th - t_w);
+          on = up;
+          x_hit = xt;
+          c.leaves += ct.leaves;
+        }
+        if (!found) s.t_search = maxi(s.t_search, stop);
+      }
+      if (found) {  // the event and the reset (PixelProc::fire)
+        const int64_t t = t_w + hit;
+        const float ds = x_hit - r.s3;
+        const float l = m.leak * static_cast<float>(static_cast<double>(t - s.t_ref) * 1e-9);
+        const float dl = l + r.dr;
+        const float D = ds + r.dn + dl;
+        const bool first = (s.flags & kFlagFirstAfterInit) != 0u;
+        RawEvent ev;
+        ev.pixel = pixel;
+        ev.polarity = on ? 1 : 0;
+        ev.label = label >= 0 ? static_cast<uint8_t>(label)
+                   : first    ? first_label(on, ds, r.dn, l, k.label_cut)
+                              : split_label(ds, dl, D, k.label_cut);
+        ev.flags = static_cast<uint16_t>(s.flags);
+        ev.t_cross = t;
+        ev.ds = ds;
+        ev.dn = r.dn;
+        ev.dl = dl;
+        ev.l_first = first ? l : 0.0f;
+        sink.push(ev);
+        s.flags = 0;
+        if (k.ideal_reset || k.refractory_ns == 0) {
+          s.t_ref = t;
+          r.since = t_w - t;
+          r.s3 = x_hit;
+          r.dn = 0.0f;
+          r.dr = k.ideal_reset ? D - (on ? m.theta_on : -m.theta_off) : -k.eps_ci;
+          s.t_search = t + 1 + (k.ideal_reset ? k.refractory_ns : 0);
+          s.s3_ref = r.s3;
+          s.n3_ref = 0.0f;
+          s.dr_ref = r.dr;
+          bounds = quick_record(s, m, false, T0, T_end);
+        } else {
+          s.blind_until = t + k.refractory_ns;
+          s.t_search = s.blind_until + 1;
+        }
+      }
+    }
+  }
+  if (s.n_shot != px.n_shot && later_t0 < 0 && s.t_shot < T_end) {  // no stop noted: on to the next one
+    const uint32_t from = s.n_shot;
+    U4 w = draw(k.seed, kPurposeShot, k.camera, pixel, s.n_shot);
+    skip_rejected(k, pixel, accept_limit(m, k, S.field, raw), m.shot_max_hz, T_end, w, s.t_shot, s.n_shot);
+    c.noise_candidates += s.n_shot - from;
+  }
+  SplitPixel& out = a.px[slot];
+  out.t_ref = s.t_ref;
+  out.t_search = s.t_search;
+  out.blind_until = s.blind_until;
+  out.t_shot = s.t_shot;
+  out.t_ba = s.t_ba;
+  out.s3_ref = s.s3_ref;
+  out.n3_ref = s.n3_ref;
+  out.dr_ref = s.dr_ref;
+  out.flags = s.flags;
+  out.n_shot = s.n_shot;
+  out.n_ba = s.n_ba;
+  if (s.n_shot != px.n_shot) {
+    out.later_t[0] = later_t0;
+    out.later_t[1] = later_t1;
+    out.later_n[0] = later_n0;
+  }
+  a.q.a[slot] = quick_record(s, m, noise, T0, T_end);
+  a.q.c[slot] = raw;
+  // The counters, one atomic per sensor among the lanes that are here (an atomic per pixel on the few counters would
+  // bound the kernel).
+  for (unsigned todo = __activemask();;) {
+    const int lead = __ffs(static_cast<int>(todo)) - 1;
+    const uint32_t si = __shfl_sync(todo, tag & 0xFFFFu, lead);
+    const bool same = (tag & 0xFFFFu) == si;
+    const unsigned group = __ballot_sync(todo, same);
+    if (same) {
+      const uint32_t pieces = __reduce_add_sync(group, c.pieces), leaves = __reduce_add_sync(group, c.leaves);
+      const uint32_t cands = __reduce_add_sync(group, c.noise_candidates);
+      if (static_cast<int>(lane) == lead) {
+        atomicAdd(&S.counters[kCntPieces], static_cast<unsigned long long>(pieces));
+        atomicAdd(&S.counters[kCntLeaves], static_cast<unsigned long long>(leaves));
+        if (cands) atomicAdd(&S.counters[kCntNoise], static_cast<unsigned long long>(cands));
+      }
+      break;
+    }
+    todo &= ~group;
+  }
+}
+
+// The posted pixels of window a.w. Where the list is shorter than the launch, each warp takes fewer records (a power of
+// two of its lanes), since what one pixel does hardly ever falls together with what its neighbour does. 128 registers (4
+// blocks per SM): 5.90 ms of engine time on 346x260, 239 windows; 6.17 at 5 blocks, 6.58 at 6.
 __global__ void __launch_bounds__(128, 4) split_rest_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
-  const int64_t T0 = *a.t0, T_end = T0 + static_cast<int64_t>(a.windows) * kWindowNs;
-  const int64_t t_w = T0 + static_cast<int64_t>(a.w) * kWindowNs;
-  const float tau_a = static_cast<float>(static_cast<double>(static_cast<int64_t>(a.w) * kWindowNs) * 1e-9);
-  const float tau_b = static_cast<float>(static_cast<double>((static_cast<int64_t>(a.w) + 1) * kWindowNs) * 1e-9);
-  const bool last_window = a.w + 1 == a.windows;
-  if (!last_window) write_boxes(a, t_w + kWindowNs, a.boxes_next);
+  const WindowTimes wt(a, a.w);
+  if (a.w + 1 < a.windows) write_boxes(a, wt.t_w + kWindowNs, a.boxes_next);
   const unsigned int count = min(*rl.count, rl.capacity);
   const unsigned int warps = gridDim.x * (blockDim.x >> 5);
   const unsigned int warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
   unsigned int share = 32u;
   while (share > 1u && static_cast<uint64_t>(share / 2u) * warps >= count) share /= 2u;
   if (lane >= share) return;
-  for (unsigned int i = warp * share + lane; i < count; i += warps * share) {
-    const RestRecord& rec = rl.rec[i];
-    const uint32_t tag = rec.tag, pixel = rec.pixel, slot = rec.slot;
-    const uint32_t left = tag >> 16 & 0xFFu;
-    const int level = static_cast<int>(tag >> 24 & 0x7Fu);
-    const bool timed = (tag & 0x80000000u) != 0u;
-    const EngineSensor& S = a.sensors[tag & 0xFFFFu];
-    const SensorConsts& k = S.consts;
-    const bool noise = k.noise != 0;
-    float raw = a.q.c[slot];
-    const SplitPixel px = a.px[slot];
-    // Quiet windows moved the search to their ends; the held sample is the carried one.
-    PixelRegs s{px.t_ref, maxi(px.t_search, t_w), px.blind_until, px.s3_ref, px.n3_ref, px.dr_ref, px.i_scale,
-                clamp_irr(raw, k.irr_max), px.flags, px.t_shot, px.t_ba, px.n_shot, px.n_ba};
-    const PixelMapRegs m{px.theta_on, px.theta_off, px.leak, px.dark, px.scale, px.ba_rate_hz, px.shot_max_hz};
-    int64_t later_t0 = px.later_t[0], later_t1 = px.later_t[1];
-    uint32_t later_n0 = px.later_n[0], later_n1 = px.later_n[1];
-    PixelCounters c;
-    if (left == kRestWhole) {
-      PixelRegs st = s;  // copies, so that the state itself stays in registers
-      PixelMapRegs mt = m;
-      PixelCounters ct = c;
-      float rt = raw;
-      const uint32_t n = rest_whole(&a, &S, pixel, level, t_w, &st, &mt, &ct, &rt);
-      s = st;
-      c = ct;
-      raw = rt;
-      if (s.n_shot != px.n_shot) later_t0 = later_t1 = -1;
-      atomicAdd(&S.counters[kCntSamples], static_cast<unsigned long long>(n));
-    } else {
-      ThreadSink sink{S.ev, &S.counters[kCntEvents]};
-      RestPixel r{m, s.s3_ref, 0.0f - s.n3_ref, s.dr_ref, s.i_scale, t_w - s.t_ref, 0u, 0u, 0.0f, 0.0f, 0.0f};
-      r.v1 = clamp_irr(raw, k.irr_max);
-      float4 bounds = a.q.a[slot];
-      float x0 = 0.0f, x1 = 0.0f;  // x at the segment's ends, where have_x
-      bool have_x = false;
-      uint32_t q = 0;
-      bool next = true, done = false;
-      for (;;) {
-        // Steps until a search is needed: from `da` (Delta there does not fire) to before `stop`.
-        bool need = false, found = false, on = false;
-        uint32_t da = 0, hit = 0;
-        float xa = 0.0f, x_hit = 0.0f;
-        int64_t stop = 0;
-        int label = -1;
-        while (!done && !need && !found) {
-          if (next) {  // the next sample's segment
-            if (q == left) {
-              done = true;
-              break;
-            }
-            raw = rec.v[q];
-            r.d0 = r.d1;
-            r.v0 = r.v1;
-            r.d1 = timed ? rl.times[i].dt[q]
-                         : (q + 1u) << (static_cast<uint32_t>(kWindowLog2) - static_cast<uint32_t>(level));
-            r.v1 = clamp_irr(raw, k.irr_max);
-            r.inv = __uint_as_float((127u - (31u - static_cast<uint32_t>(__clz(static_cast<int>(r.d1 - r.d0))))) << 23);
-            ++q;
-            ++c.pieces;
-            next = false;
-            have_x = false;
-          }
-          const int64_t t0 = t_w + r.d0, e = t_w + r.d1;
-          const int64_t tn = noise ? mini(s.t_shot, s.t_ba) : kForever;
-          bool cand = false, drop = false;
-          if (s.blind_until != kNotBlind) {
-            cand = drop = s.blind_until >= e ? tn < e : tn <= s.blind_until;
-            if (!cand) {
-              if (s.blind_until >= e) {
-                next = true;
-              } else {  // the release: a new reference at x(t_rel) - eps_ci
-                const uint32_t db = static_cast<uint32_t>(s.blind_until - t_w);
-                r.s3 = r.x_of(r.current(db));
-                r.dn = 0.0f;
-                r.dr = -k.eps_ci;
-                r.since = t_w - s.blind_until;
-                s.t_ref = s.blind_until;
-                s.blind_until = kNotBlind;
-                s.s3_ref = r.s3;
-                s.n3_ref = 0.0f;
-                s.dr_ref = r.dr;
-                bounds = quick_record(s, m, false, T0, T_end);
-              }
-            }
-          } else {
-            const int64_t lo = maxi(s.t_search, t0);
-            stop = mini(e, tn);
-            if (lo < stop) {
-              // Quiet by the bounds (split_window_kernel's test on this segment alone), or by Delta at lo and the
-              // segment's ends (PixelProc::segment_fast's).
-              const float Ia = m.dark + m.scale * r.v0, Ib = m.dark + m.scale * r.v1;
-              const float I_hi = fmaxf(Ia, Ib), I_lo = fminf(Ia, Ib);
-              const float pad = 0x1p-21f * I_hi;
-              bool quiet = __log2f(I_hi + pad) < bounds.x - bounds.z * tau_b &&
-                           __log2f(I_lo - pad) > bounds.y - bounds.z * tau_a;
-              ++c.leaves;
-              if (!quiet) {
-                if (!have_x) {
-                  x0 = r.x_of(Ia);
-                  x1 = r.x_of(Ib);
-                  have_x = true;
-                }
-                da = static_cast<uint32_t>(lo - t_w);
-                xa = lo == t0 ? x0 : r.x_of(r.current(da));
-                const float la = r.dl(da), D = r.delta(xa, la);
-                if (D >= m.theta_on || D <= -m.theta_off) {
-                  found = true;
-                  hit = da;
-                  x_hit = xa;
-                  on = D >= m.theta_on;
-                } else if (stop - lo == 1) {
-                  quiet = true;
-                } else {
-                  if (r.v0 + (r.v1 - r.v0) == r.v1) {
-                    const float top = r.delta(maxr(xa, x1), r.dl(r.d1)), low = r.delta(minr(xa, x1), la);
-                    quiet = top < m.theta_on && low > -m.theta_off;
-                  }
-                  need = !quiet;
-                }
-              }
-              if (quiet) s.t_search = maxi(s.t_search, stop);
-            } else if (tn >= e) {
-              next = true;
-            } else {
-              cand = true;
-              drop = tn < s.t_search;
-            }
-          }
-          if (cand) {
-            const bool shot = s.t_shot <= s.t_ba;
-            const uint32_t dc = static_cast<uint32_t>(tn - t_w);
-            const float I = drop ? 0.0f : r.current(dc);
-            CandidateOut o;
-            candidate_step(&k, pixel, shot, shot ? s.n_shot : s.n_ba, tn, shot ? m.shot_max_hz : m.ba_rate_hz, drop,
-                           !shot || later_t0 < 0, m.dark, I, &o);
-            ++c.noise_candidates;
-            if (shot && later_t0 >= 0) {  // the chain's next stop
-              s.t_shot = later_t0;
-              s.n_shot = later_n0;
-              later_t0 = later_t1;
-              later_n0 = later_n1;
-              later_t1 = -1;
-            } else if (shot) {  // more stops than the record holds: one candidate on
-              ++s.n_shot;
-              s.t_shot = o.next;
-            } else {
-              ++s.n_ba;
-              s.t_ba = o.next;
-            }
-            if (o.accepted) {
-              found = true;
-              hit = dc;
-              x_hit = r.x_of(I);
-              on = o.on;
-              label = kLabelNoise;
-            }
-          }
-        }
-        if (done) break;
-        if (need) {
-          bool hard = false;
-          const uint32_t end = static_cast<uint32_t>(stop - t_w);
-          found = r.search(da, xa, end, x0, x1, end == r.d1 && r.v0 + (r.v1 - r.v0) == r.v1, hit, x_hit, on, hard,
-                           c.leaves);
-          if (hard) {
-            PixelRegs st = s;
-            st.s3_ref = r.s3;
-            st.n3_ref = 0.0f - r.dn;
-            st.dr_ref = r.dr;
-            NullSink none;
-            PixelMapRegs mt = m;
-            PixelCounters ct;
-            PixelProc<NullSink> proc{st, mt, k, pixel, none, ct};
-            int64_t th = t_w;
-            bool up = false;
-            float xt = 0.0f;
-            found = proc.search(Segment{t_w + r.d0, t_w + r.d1, r.v0, r.v1}, t_w + da, stop, th, up, xt);
-            hit = static_cast<uint32_t>(th - t_w);
-            on = up;
-            x_hit = xt;
-            c.leaves += ct.leaves;
-          }
-          if (!found) s.t_search = maxi(s.t_search, stop);
-        }
-        if (found) {  // the event and the reset (PixelProc::fire)
-          const int64_t t = t_w + hit;
-          const float ds = x_hit - r.s3;
-          const float l = m.leak * static_cast<float>(static_cast<double>(t - s.t_ref) * 1e-9);
-          const float dl = l + r.dr;
-          const float D = ds + r.dn + dl;
-          const bool first = (s.flags & kFlagFirstAfterInit) != 0u;
-          RawEvent ev;
-          ev.pixel = pixel;
-          ev.polarity = on ? 1 : 0;
-          ev.label = label >= 0 ? static_cast<uint8_t>(label)
-                     : first    ? first_label(on, ds, r.dn, l, k.label_cut)
-                                : split_label(ds, dl, D, k.label_cut);
-          ev.flags = static_cast<uint16_t>(s.flags);
-          ev.t_cross = t;
-          ev.ds = ds;
-          ev.dn = r.dn;
-          ev.dl = dl;
-          ev.l_first = first ? l : 0.0f;
-          sink.push(ev);
-          s.flags = 0;
-          if (k.ideal_reset || k.refractory_ns == 0) {
-            s.t_ref = t;
-            r.since = t_w - t;
-            r.s3 = x_hit;
-            r.dn = 0.0f;
-            r.dr = k.ideal_reset ? D - (on ? m.theta_on : -m.theta_off) : -k.eps_ci;
-            s.t_search = t + 1 + (k.ideal_reset ? k.refractory_ns : 0);
-            s.s3_ref = r.s3;
-            s.n3_ref = 0.0f;
-            s.dr_ref = r.dr;
-            bounds = quick_record(s, m, false, T0, T_end);
-          } else {
-            s.blind_until = t + k.refractory_ns;
-            s.t_search = s.blind_until + 1;
-          }
-        }
-      }
+  for (unsigned int i = warp * share + lane; i < count; i += warps * share) rest_pixel(a, rl, wt, i, lane);
+}
+
+// The whole call in one launch, for few tiles: a block keeps its tiles through all windows, and each window's posted
+// pixels stay in the block, spread over its warps. Nothing passes between blocks, so no window waits for the slowest
+// pixel of another block's, and none of the two launches per window is paid.
+__global__ void __launch_bounds__(128, 4) split_solo_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
+  const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  __shared__ WarpShared sh[4];
+  __shared__ SplitSums sums;
+  __shared__ unsigned int posted;
+  sums.clear();
+  // This block's tiles, and its part of the list.
+  const uint32_t first = blockIdx.x * a.block_tiles;
+  const uint32_t end = first + a.block_tiles < a.total_tiles ? first + a.block_tiles : a.total_tiles;
+  RestList mine_list = rl;
+  mine_list.rec += static_cast<size_t>(first) * 32u;
+  mine_list.times += static_cast<size_t>(first) * 32u;
+  mine_list.count = &posted;
+  mine_list.capacity = a.block_tiles * 32u;
+  for (uint32_t tile = first + warp; tile < end; tile += warps) begin_tile(a, tile, lane);
+  if (threadIdx.x == 0) posted = 0;
+  __syncthreads();
+  WarpSums mine;
+  for (int32_t w = 0; w < a.windows; ++w) {
+    const WindowTimes wt(a, w);
+    for (uint32_t tile = first + warp; tile < end; tile += warps) {
+      const int si = sensor_of(a, tile);
+      mine.of(a, sums, si);
+      window_tile<false>(a, mine_list, wt, sh[warp], a.sensors[si], si, tile, lane, mine.samples, mine.clean);
     }
-    if (s.n_shot != px.n_shot && later_t0 < 0 && s.t_shot < T_end) {  // no stop noted: on to the next one
-      const uint32_t from = s.n_shot;
-      U4 w = draw(k.seed, kPurposeShot, k.camera, pixel, s.n_shot);
-      skip_rejected(k, pixel, accept_limit(m, k, S.field, raw), m.shot_max_hz, T_end, w, s.t_shot, s.n_shot);
-      c.noise_candidates += s.n_shot - from;
-    }
-    SplitPixel& out = a.px[slot];
-    out.t_ref = s.t_ref;
-    out.t_search = s.t_search;
-    out.blind_until = s.blind_until;
-    out.t_shot = s.t_shot;
-    out.t_ba = s.t_ba;
-    out.s3_ref = s.s3_ref;
-    out.n3_ref = s.n3_ref;
-    out.dr_ref = s.dr_ref;
-    out.flags = s.flags;
-    out.n_shot = s.n_shot;
-    out.n_ba = s.n_ba;
-    if (s.n_shot != px.n_shot) {
-      out.later_t[0] = later_t0;
-      out.later_t[1] = later_t1;
-      out.later_n[0] = later_n0;
-    }
-    a.q.a[slot] = quick_record(s, m, noise, T0, T_end);
-    a.q.c[slot] = raw;
-    // The counters, one atomic per sensor among the lanes that are here (an atomic per pixel on the few counters would
-    // bound the kernel).
-    for (unsigned todo = __activemask();;) {
-      const int lead = __ffs(static_cast<int>(todo)) - 1;
-      const uint32_t si = __shfl_sync(todo, tag & 0xFFFFu, lead);
-      const bool same = (tag & 0xFFFFu) == si;
-      const unsigned group = __ballot_sync(todo, same);
-      if (same) {
-        const uint32_t pieces = __reduce_add_sync(group, c.pieces), leaves = __reduce_add_sync(group, c.leaves);
-        const uint32_t cands = __reduce_add_sync(group, c.noise_candidates);
-        if (static_cast<int>(lane) == lead) {
-          atomicAdd(&S.counters[kCntPieces], static_cast<unsigned long long>(pieces));
-          atomicAdd(&S.counters[kCntLeaves], static_cast<unsigned long long>(leaves));
-          if (cands) atomicAdd(&S.counters[kCntNoise], static_cast<unsigned long long>(cands));
-        }
-        break;
-      }
-      todo &= ~group;
-    }
+    __syncthreads();
+    const unsigned int count = posted;
+    __syncthreads();
+    if (threadIdx.x == 0) posted = 0;
+    for (unsigned int i = warp + warps * lane; i < count; i += warps * 32u) rest_pixel(a, mine_list, wt, i, lane);
+    __syncthreads();
   }
+  for (uint32_t tile = first + warp; tile < end; tile += warps) end_tile(a, tile, lane);
+  mine.flush(a, sums);
+  __syncthreads();
+  sums.add(a);
 }
 
 }  // namespace
@@ -1047,7 +1132,7 @@ size_t split_record_bytes() { return sizeof(RestRecord) + sizeof(RestTimes); }
 void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,
                          uint32_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
                          void* rest, unsigned int* rest_counts, unsigned int rest_capacity, int blocks,
-                         int warps_per_block, int tile_lw, int rest_blocks, cudaStream_t stream) {
+                         int warps_per_block, int tile_lw, int rest_blocks, bool solo, cudaStream_t stream) {
   const size_t slots = static_cast<size_t>(total_tiles) * 32u;
   SplitArgs a{};
   a.sensors = sensors_dev;
@@ -1067,6 +1152,13 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   RestTimes* times = reinterpret_cast<RestTimes*>(records + rest_capacity);
   for (int i = 0; i < n_sensors && i < kTile0Args; ++i) a.tile0[i] = tile0[i];
   a.boxes = boxes;
+  if (solo) {
+    const uint32_t most = static_cast<uint32_t>(blocks);
+    a.block_tiles = (total_tiles + most - 1) / most;
+    const RestList rl{records, times, nullptr, rest_capacity};
+    split_solo_kernel<<<(total_tiles + a.block_tiles - 1) / a.block_tiles, warps_per_block * 32, 0, stream>>>(a, rl);
+    return;
+  }
   split_begin_kernel<<<(total_tiles + 3) / 4, 128, 0, stream>>>(a);
   for (int32_t w = 0; w < windows; ++w) {
     a.w = w;
@@ -1082,6 +1174,11 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
 int split_rest_blocks_per_sm() {
   int n = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, split_rest_kernel, 128, 0);
+  return n;
+}
+int split_solo_blocks_per_sm(int warps_per_block) {
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, split_solo_kernel, warps_per_block * 32, 0);
   return n;
 }
 int split_window_blocks_per_sm(int warps_per_block) {

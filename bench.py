@@ -195,7 +195,9 @@ def engine_kernel_name(eng, cascade: bool, lattice: bool) -> str:
 def engine_launches(eng, windows: int) -> int:
     """The engine's kernel launches in one step: one persistent launch, or for the split engine two per window and its
     begin and end kernels."""
-    return 2 * windows + 2 if eng.launch["stage"] == 1 else 1
+    tile_w = eng.launch["tile_width"]
+    tiles = sum(-(-m.width // tile_w) * -(-m.height // (32 // tile_w)) for m, _ in eng.sensors)
+    return 2 * windows + 2 if eng.launch["stage"] == 1 and tiles > 2 * 16 * N_SMS else 1
 
 
 def run_ours(args, rank: int, world: int) -> dict | None:

@@ -56,11 +56,14 @@ struct DevBuf {
   ~DevBuf() {
     if (p) cudaFree(p);
   }
-  T* ensure(size_t n) {
-    if (n <= cap && p) return p;
+  void release() {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
+  }
+  T* ensure(size_t n) {
+    if (n <= cap && p) return p;
+    release();
     const size_t want = n == 0 ? 1 : n;
     CK(cudaMalloc(&p, want * sizeof(T)));
     cap = want;
@@ -1557,6 +1560,7 @@ struct Engine {
   std::vector<EngineSensor> host;
   uint32_t total_tiles = 0;
   int warps_per_block = 4, blocks_per_sm = 0, stage = 0, tile_lw = 3;
+  bool stage_chosen = true;  // by set_launch or the autotuner, not the constructor's
   double last_ms = 0;
   Timer timer;
   mutable Timer take_timer;           // the last download's device part: sort + column split
@@ -1634,6 +1638,13 @@ struct Engine {
       host.push_back(e);
     }
     total_tiles = tile0;
+    // The launch shape until set_launch or the autotuner: the split engine for the instantaneous response. From the
+    // first frame on (64x48 to 640x480, 1 to 160 windows, with and without noise) it takes 0.24 to 0.93 of the streaming
+    // engine's time, and 0.37 of it on 1280x720.
+    if (cascade() == 0) {
+      stage = kStageSplit;
+      stage_chosen = false;
+    }
     retile();
     sensors_dev.ensure(host.size());
     tile_counter.ensure(1);
@@ -1780,6 +1791,7 @@ struct Engine {
   // (1,974 tiles, 37 windows) 1.25 against 1.60, 640x480 (9,600 tiles) 3.33 against 3.37, 1280x720 12.5 against 11.8.
   bool split_solo() const { return total_tiles <= 2u * 16u * static_cast<uint32_t>(sm_count()); }
   void ensure_split(int32_t windows) {
+    if (total_tiles > (1u << 26)) throw BudgetError("the split engine: too many pixels for its records");
     const unsigned int slots = total_tiles * 32u;
     if (rest_capacity < slots) {
       rest.ensure(static_cast<size_t>(slots) * split_record_bytes());
@@ -1848,12 +1860,22 @@ struct Engine {
       if ((t0 & (kWindowNs - 1)) != 0) throw std::invalid_argument("engine: the model time must be a window start");
     }
     if (mlp && lcur.size() != models.size()) throw std::logic_error("engine: call start() after set_proposal()");
+    if (stage == kStageSplit && !mlp && !stage_chosen) {
+      try {
+        ensure_split(windows);
+      } catch (const BudgetError&) {  // its records (about 300 bytes a pixel) do not fit: the streaming engine's need none
+        split_scratch.release();
+        rest.release();
+        rest_capacity = 0;
+        stage = 0;
+      }
+    }
     const int blocks = grid_blocks();
     t0_pin.ensure(1);
     rec_n_pin.ensure(2);
     for (;;) {
       describe(t0);
-      if (stage == kStageSplit) ensure_split(windows);
+      if (stage == kStageSplit && !mlp) ensure_split(windows);
       if (use_graph && rec_cap == 0) {
         const uint64_t key[8] = {static_cast<uint64_t>(windows), static_cast<uint64_t>(blocks),
                                  static_cast<uint64_t>(block_warps()), static_cast<uint64_t>(stage),
@@ -1987,6 +2009,7 @@ struct Engine {
     warps_per_block = warps ? warps : 4;
     blocks_per_sm = per_sm;
     stage = stg;
+    stage_chosen = true;
     tile_lw = lw ? lw : 3;
     retile();
   }

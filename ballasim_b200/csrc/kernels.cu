@@ -6,6 +6,8 @@
 //
 // Events leave through warp-aggregated atomics: the lanes that emit together take one slot range with one atomic
 // (coalesced group rank), and a call whose events exceed the buffer is re-run from its unchanged input state.
+#include <algorithm>
+
 #include "engine_dev.cuh"
 
 namespace bs {
@@ -1191,23 +1193,38 @@ struct CascadeFeed {
   }
 };
 
-// At most 128 registers (168 uncapped): on the 346x260 cascade workload 36.6 against 38.2 ms per step, spills
-// included (the lattice engine, capped alike, ran 1,936 against 1,870 ms and stays uncapped).
-__global__ void __launch_bounds__(128, 4) engine_cascade_kernel(EngineArgs a) {
-  const uint32_t lane = threadIdx.x & 31u;
+// The block's warps take one sub-step a turn together, a barrier between turns. A sub-step is some thousands of
+// instructions that run once (two stage-1 solves, logarithms, residual exponentials, the crossing search), more than the
+// instruction caches next to the schedulers hold: warps that drift apart each fetch it for themselves (10.7 of the 16
+// cycles between a warp's issues waited for instructions; 0.7 in step). So the samples of a window are staged first (as
+// engine_kernel_staged does), and every turn each lane runs its next sub-step, whichever segment it stands in. One block
+// per multiprocessor with as many warps as the registers allow (at most 102 each). What is left is the wait at the
+// barrier for the turn's longest sub-step. 346x260, 60 windows: 12.0 ms against 16.4 free-running, 640x480 17.3 against
+// 23.5; 2 or 4 turns between barriers 13.4 and 14.9, a barrier before the comparator too 12.9, two blocks of 10 warps
+// 11.4 and 19.4, warps free to go on to their next window 14.1.
+constexpr int kCascadeStage = 16;
+constexpr int kCascadeWarps = 20;
+
+struct CascadeWarpShared {
+  uint16_t list[kMaxListed];
+  uint32_t dt[kCascadeStage][32];
+  float v[kCascadeStage][32];
+};
+
+__global__ void __launch_bounds__(32 * kCascadeWarps, 1) engine_cascade_kernel(EngineArgs a) {
+  extern __shared__ CascadeWarpShared cascade_shared[];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  CascadeWarpShared& sh = cascade_shared[warp];
   const int64_t t0 = *a.t0;
-  for (;;) {
-    uint32_t tile = 0;
-    if (lane == 0) tile = atomicAdd(a.tile_counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if (tile >= a.total_tiles) break;
+  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first += gridDim.x * warps) {
+    const uint32_t tile = first + warp < a.total_tiles ? first + warp : a.total_tiles - 1u;
+    const bool real = first + warp < a.total_tiles;  // a warp past the last tile only keeps the barriers
     int si = 0;
     while (si + 1 < a.n_sensors && a.sensors[si + 1].tile0 <= tile) ++si;
     const EngineSensor& S = a.sensors[si];
-    const uint32_t local = tile - S.tile0;
     uint32_t x, y;
-    tile_xy(local, S.tiles_x, a.tile_lw, lane, x, y);
-    const bool have = x < S.width && y < S.height;
+    tile_xy(tile - S.tile0, S.tiles_x, a.tile_lw, lane, x, y);
+    const bool have = real && x < S.width && y < S.height;
     const uint32_t p = have ? y * S.width + x : 0u;
     PixelRegs s;
     CascadeRegs q;
@@ -1225,17 +1242,62 @@ __global__ void __launch_bounds__(128, 4) engine_cascade_kernel(EngineArgs a) {
     GlobalSink sink{S.ev, &S.counters[kCntEvents]};
     CascadeProc<GlobalSink> proc{s, q, m, S.consts, S.cc, p, sink, c, cn};
     const FieldDev& f = S.field;
-    __shared__ uint16_t lists[4][kMaxListed];
-    uint16_t* my_list = lists[threadIdx.x >> 5];
+    const float irr_max = S.consts.irr_max;
     for (int32_t w = a.w0; w < a.w1; ++w) {
       const int64_t t_w = t0 + static_cast<int64_t>(w) * kWindowNs;
-      const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, my_list);
+      const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, sh.list);
+      auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
+      // The walk, its first kCascadeStage samples after slot 0 staged.
+      uint32_t n = 0;
+      int level = 0;
       if (have) {
-        const int level = field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
-        CascadeFeed feed{&proc, t_w, S.consts.irr_max, t_w, s.held, carried};
+        level = field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
+        uint32_t k = 0;
+        n = sample_pixel_window(a.r, level, carried, false, render, [&](uint32_t dt, float v) {
+          if (k < static_cast<uint32_t>(kCascadeStage)) {
+            sh.dt[k][lane] = dt;
+            sh.v[k][lane] = v;
+          }
+          ++k;
+        });
+        samples += n;
+      }
+      const bool staged = have && n - 1u <= static_cast<uint32_t>(kCascadeStage);
+      // One sub-step a turn (CascadeProc::segment and run_piece; a segment never crosses the window: one piece).
+      uint32_t next = 0;
+      bool inside = false;
+      LinearPiece pc{};
+      int64_t ta = 0, h_hint = 0, prev_t = t_w;
+      float prev_v = clamp_irr(carried, irr_max), last_raw = carried;
+      while (__syncthreads_or(staged && (inside || next + 1u < n))) {
+        if (staged && (inside || next + 1u < n)) {
+          if (!inside) {
+            last_raw = sh.v[next][lane];
+            const float vc = clamp_irr(last_raw, irr_max);
+            const int64_t t = t_w + sh.dt[next][lane];
+            const Segment g{prev_t, t, prev_v, vc};
+            pc = LinearPiece{prev_t, t, proc.current(g, prev_t), proc.current(g, t)};
+            ++c.pieces;
+            ta = prev_t;
+            h_hint = 0;
+            prev_t = t;
+            prev_v = vc;
+            ++next;
+            inside = true;
+          }
+          SubStep sub;
+          ta = proc.make_substep(pc, ta, h_hint, sub);
+          proc.comparator(sub);
+          inside = ta < pc.t_b;
+        }
+      }
+      if (staged) {
+        s.held = prev_v;
+        carried = last_raw;
+      } else if (have) {  // the window overflowed the stage: the walk again with the model fed inline
+        CascadeFeed feed{&proc, t_w, irr_max, t_w, s.held, carried};
         feed.start(carried);
-        auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
-        samples += sample_pixel_window(a.r, level, carried, false, render, feed);
+        sample_pixel_window(a.r, level, carried, false, render, feed);
         s.held = feed.prev_v;
         carried = feed.last_raw;
       }
@@ -1251,6 +1313,20 @@ __global__ void __launch_bounds__(128, 4) engine_cascade_kernel(EngineArgs a) {
     warp_add(&S.counters[kCntSamples], samples);
     warp_add(&S.counters[kCntSubsteps], cn.substeps);
   }
+}
+
+// The launch of a kernel of one block per multiprocessor and at most `most_warps` warps a block for a number of tiles:
+// whole rounds of blocks, the tiles spread evenly over them.
+struct StepShape {
+  int blocks, warps;
+};
+StepShape step_shape(uint32_t total_tiles, int sms, int most_warps) {
+  const uint32_t most = static_cast<uint32_t>(sms) * static_cast<uint32_t>(most_warps);
+  const uint32_t rounds = (total_tiles + most - 1) / most;
+  const uint32_t groups = rounds * static_cast<uint32_t>(sms);
+  const uint32_t warps = (total_tiles + groups - 1) / groups;
+  return {static_cast<int>(std::min<uint32_t>(static_cast<uint32_t>(sms), (total_tiles + warps - 1) / warps)),
+          static_cast<int>(warps)};
 }
 
 // The fused engine with the cascade's noise lattice. A cell's look-ahead needs the cell's input up to its end, so
@@ -1479,7 +1555,10 @@ struct LatticeStageFeed {
   }
 };
 
-__global__ void __launch_bounds__(128) engine_lattice_kernel_staged(EngineArgs a) {
+// At most 102 registers (168 uncapped), 5 blocks per SM: 87.6 against 92.6 ms on 346x260, 8 windows (a form that kept the
+// block's warps in step, as engine_cascade_kernel does, with the tree walks put off until an eighth of the lanes wait for
+// one, took 133: some pixels need a walk in nearly every cell).
+__global__ void __launch_bounds__(128, 5) engine_lattice_kernel_staged(EngineArgs a) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t t0 = *a.t0;
   __shared__ uint16_t lists[4][kMaxListed];
@@ -2249,9 +2328,16 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
                    int32_t w0, int32_t w1, const SamplerRules& r, unsigned int* tile_counter, int blocks,
                    int warps_per_block, int stage, int tile_lw, int cascade, cudaStream_t stream) {
   EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w0, w1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
-  if (cascade == 2 && stage != 0) engine_lattice_kernel_staged<<<blocks, warps_per_block * 32, 0, stream>>>(a);
+  if (cascade == 1) {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const StepShape c = step_shape(total_tiles, sms, kCascadeWarps);
+    const int bytes = c.warps * static_cast<int>(sizeof(CascadeWarpShared));
+    cudaFuncSetAttribute(engine_cascade_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    engine_cascade_kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a);
+  } else if (cascade == 2 && stage != 0) engine_lattice_kernel_staged<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (cascade == 2) engine_lattice_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
-  else if (cascade == 1) engine_cascade_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 64) engine_kernel_coop<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 16) engine_kernel_staged<16><<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 32) engine_kernel_staged<32><<<blocks, warps_per_block * 32, 0, stream>>>(a);
@@ -2267,12 +2353,12 @@ int rows_rest_blocks_per_sm() {
 
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade) {
   int n = 0;
-  if (cascade == 2 && stage != 0) {
+  if (cascade == 1) {
+    n = 1;  // launch_engine takes a shape of its own (step_shape)
+  } else if (cascade == 2 && stage != 0) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel_staged, warps_per_block * 32, 0);
   } else if (cascade == 2) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel, warps_per_block * 32, 0);
-  } else if (cascade == 1) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_cascade_kernel, warps_per_block * 32, 0);
   } else if (stage == 64) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_kernel_coop, warps_per_block * 32, 0);
   } else if (stage == 16) {

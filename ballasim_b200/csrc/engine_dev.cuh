@@ -408,4 +408,60 @@ struct RegFeed {
   }
 };
 
+// ---------------------------------------------------------------------------------------------
+// Quiet windows and noise stops (the split engine's header comment says what they are for)
+// ---------------------------------------------------------------------------------------------
+// The quick record's bounds from the state. Delta = ln(I / i_scale) - s3 - n3 + (leak (t - t_ref) 1e-9 + dr), so it
+// stays below theta_on while log2 I < upper - leak log2(e) (t - T0), and above -theta_off alike. The slack, 2e-5 of the
+// sum of the terms' magnitudes, is over 20 times what the roundings of Delta (four fp32 operations, log_f, the
+// division) and of this evaluation (lg2.approx: 2^-22) add up to.
+__device__ __forceinline__ float4 quick_record(const PixelRegs& s, const PixelMapRegs& m, bool noise, int64_t T0,
+                                               int64_t T_end) {
+  const float log2e = 1.4426950408889634f;
+  const float drift = m.leak * since_ref(T0, s.t_ref);
+  const float span = m.leak * static_cast<float>(static_cast<double>(T_end - T0) * 1e-9);
+  const float c = ((s.s3_ref + s.n3_ref) - s.dr_ref) - drift;
+  const float mag = 4.0f + fabs_f(s.s3_ref) + fabs_f(s.n3_ref) + fabs_f(s.dr_ref) + fabs_f(drift) + fabs_f(span) +
+                    m.theta_on + m.theta_off;
+  const float slack = 2.0e-5f * mag;
+  const float li = __log2f(s.i_scale);
+  float4 q;
+  q.x = (c + m.theta_on - slack) * log2e + li - 1.0e-6f * fabs_f(li);
+  q.y = (c - m.theta_off + slack) * log2e + li + 1.0e-6f * fabs_f(li);
+  q.z = m.leak * log2e;
+  int32_t gate = INT32_MAX;
+  if (noise) {
+    const int64_t tn = mini(s.t_shot, s.t_ba);
+    if (tn < T_end) gate = static_cast<int32_t>((tn - T0) >> kWindowLog2);
+  }
+  if (s.blind_until != kNotBlind || !(mag < 1.0e3f)) gate = INT32_MIN;
+  q.w = __int_as_float(gate);
+  return q;
+}
+
+// Shot candidate n is accepted when its u1 < sqrt(I_dk / I) (PixelProc::candidate_accepted). Every photocurrent of the
+// pixel in the call is at least that of the least sample (the field's lower bound or the carried sample; the
+// interpolation's rounding, relative to the largest sample, taken off), so a candidate whose u1 is at or above the root
+// there is rejected whenever it comes, and changes nothing but its chain. The largest word of u1 that may be accepted:
+__device__ __forceinline__ uint32_t accept_limit(const PixelMapRegs& m, const SensorConsts& k, const FieldDev& f,
+                                                 float carried) {
+  const float v0 = clamp_irr(carried, k.irr_max);
+  const float lo = minr(v0, clamp_irr(f.lo, k.irr_max)), hi = maxr(v0, clamp_irr(f.hi, k.irr_max));
+  const float v = maxr(0.0f, lo - 0x1p-21f * hi);
+  const float I = m.dark + m.scale * v;
+  const double root = sqrt(static_cast<double>(m.dark) / static_cast<double>(I));
+  const double bound = root * 0x1p32 + 2.0;  // u1 = (word + 1/2) 2^-32 < root only where word < bound
+  return bound < 0x1p32 - 1.0 ? static_cast<uint32_t>(bound) : 0xFFFFFFFFu;
+}
+// From the chain's candidate n at t (w its draw) to its next stop: the first candidate that may be accepted, or the
+// first at or after t_end.
+__device__ __forceinline__ void skip_rejected(const SensorConsts& k, uint32_t pixel, uint32_t limit, double rate_hz,
+                                              int64_t t_end, U4& w, int64_t& t, uint32_t& n) {
+  while (t < t_end && w.v[1] > limit) {
+    ++n;
+    w = draw(k.seed, kPurposeShot, k.camera, pixel, n);
+    t = noise_after(w, t, rate_hz);
+  }
+}
+
 }  // namespace bs

@@ -33,7 +33,7 @@ namespace {
 
 constexpr int kSplitStage = 16;       // samples after slot 0 that a posted pixel takes along (lattice level 4)
 constexpr uint32_t kRestWhole = 0xFF;  // the samples of a window that has more: walked again by the rest kernel
-constexpr int kCentres = 64;          // blob centres (one blob at one lattice slot) a warp holds at a time
+constexpr int kCentres = 64;          // blobs a warp holds, and centres (one blob at two lattice slots) at a time
 constexpr int kTile0Args = 16;        // sensors whose first tiles travel as kernel arguments
 
 // The quick record of lane l of tile t, entry 32 t + l of each plane (tile order: a warp's loads are whole lines).
@@ -86,6 +86,7 @@ struct SplitArgs {
   SamplerRules r;
   uint32_t tile_lw;
   uint32_t total_blobs;
+  unsigned long long minus_zero2;  // two fp32 -0 (mul2)
   uint32_t block_tiles;  // split_solo_kernel: the tiles of a block
   QuickPlanes q;
   SplitPixel* px;
@@ -142,59 +143,6 @@ __device__ __forceinline__ void write_boxes(const SplitArgs& a, int64_t t_w, flo
          k += gridDim.x * blockDim.x) {
       boxes[S.blob0 + k] = blob_box(S.field, k, ta, tb);
     }
-  }
-}
-
-// The quick record's bounds from the state. Delta = ln(I / i_scale) - s3 - n3 + (leak (t - t_ref) 1e-9 + dr), so it
-// stays below theta_on while log2 I < upper - leak log2(e) (t - T0), and above -theta_off alike. The slack, 2e-5 of the
-// sum of the terms' magnitudes, is over 20 times what the roundings of Delta (four fp32 operations, log_f, the
-// division) and of this evaluation (lg2.approx: 2^-22) add up to.
-__device__ __forceinline__ float4 quick_record(const PixelRegs& s, const PixelMapRegs& m, bool noise, int64_t T0,
-                                               int64_t T_end) {
-  const float log2e = 1.4426950408889634f;
-  const float drift = m.leak * since_ref(T0, s.t_ref);
-  const float span = m.leak * static_cast<float>(static_cast<double>(T_end - T0) * 1e-9);
-  const float c = ((s.s3_ref + s.n3_ref) - s.dr_ref) - drift;
-  const float mag = 4.0f + fabs_f(s.s3_ref) + fabs_f(s.n3_ref) + fabs_f(s.dr_ref) + fabs_f(drift) + fabs_f(span) +
-                    m.theta_on + m.theta_off;
-  const float slack = 2.0e-5f * mag;
-  const float li = __log2f(s.i_scale);
-  float4 q;
-  q.x = (c + m.theta_on - slack) * log2e + li - 1.0e-6f * fabs_f(li);
-  q.y = (c - m.theta_off + slack) * log2e + li + 1.0e-6f * fabs_f(li);
-  q.z = m.leak * log2e;
-  int32_t gate = INT32_MAX;
-  if (noise) {
-    const int64_t tn = mini(s.t_shot, s.t_ba);
-    if (tn < T_end) gate = static_cast<int32_t>((tn - T0) >> kWindowLog2);
-  }
-  if (s.blind_until != kNotBlind || !(mag < 1.0e3f)) gate = INT32_MIN;
-  q.w = __int_as_float(gate);
-  return q;
-}
-
-// Shot candidate n is accepted when its u1 < sqrt(I_dk / I) (PixelProc::candidate_accepted). Every photocurrent of the
-// pixel in the call is at least that of the least sample (the field's lower bound or the carried sample; the
-// interpolation's rounding, relative to the largest sample, taken off), so a candidate whose u1 is at or above the root
-// there is rejected whenever it comes, and changes nothing but its chain. The largest word of u1 that may be accepted:
-__device__ __forceinline__ uint32_t accept_limit(const PixelMapRegs& m, const SensorConsts& k, const FieldDev& f,
-                                                 float carried) {
-  const float v0 = clamp_irr(carried, k.irr_max);
-  const float lo = minr(v0, clamp_irr(f.lo, k.irr_max)), hi = maxr(v0, clamp_irr(f.hi, k.irr_max));
-  const float v = maxr(0.0f, lo - 0x1p-21f * hi);
-  const float I = m.dark + m.scale * v;
-  const double root = sqrt(static_cast<double>(m.dark) / static_cast<double>(I));
-  const double bound = root * 0x1p32 + 2.0;  // u1 = (word + 1/2) 2^-32 < root only where word < bound
-  return bound < 0x1p32 - 1.0 ? static_cast<uint32_t>(bound) : 0xFFFFFFFFu;
-}
-// From the chain's candidate n at t (w its draw) to its next stop: the first candidate that may be accepted, or the
-// first at or after t_end.
-__device__ __forceinline__ void skip_rejected(const SensorConsts& k, uint32_t pixel, uint32_t limit, double rate_hz,
-                                              int64_t t_end, U4& w, int64_t& t, uint32_t& n) {
-  while (t < t_end && w.v[1] > limit) {
-    ++n;
-    w = draw(k.seed, kPurposeShot, k.camera, pixel, n);
-    t = noise_after(w, t, rate_hz);
   }
 }
 
@@ -301,22 +249,50 @@ __global__ void __launch_bounds__(128) split_end_kernel(const __grid_constant__ 
   if (tile < a.total_tiles) end_tile(a, tile, threadIdx.x & 31u);
 }
 
-// exp_f for x in [-80, 0] (no range test, one exact scaling step): the same operations, so the same bits. The rounding
-// to an integer adds and takes off 1.5 2^23, whose sum also holds the integer in its low bits.
-__device__ __forceinline__ float exp_neg(float x) {
-  const float magic = 12582912.0f;
-  const float t = x * 0x1.715476p+0f + magic;
-  const float k = t - magic;
-  const float r = (x - k * 0x1.62e400p-1f) - k * 0x1.7f7d1cp-20f;
-  float p = 1.0f / 5040.0f;
-  p = p * r + 1.0f / 720.0f;
-  p = p * r + 1.0f / 120.0f;
-  p = p * r + 1.0f / 24.0f;
-  p = p * r + 1.0f / 6.0f;
-  p = p * r + 0.5f;
-  p = p * r + 1.0f;
-  p = p * r + 1.0f;
-  return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
+// Two fp32 values in one register pair, added and multiplied by one instruction each (the same roundings; 73.7 against
+// 36.1 T operations a second in a loop of both). The assembler contracts a packed product and sum into one rounding even
+// where both ask for theirs, so a product is formed as a fused one plus -0 (which changes nothing), with the -0s (z) read
+// from the launch's arguments, where it cannot see them.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b, F2 z) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(z.v));
+  return r;
+}
+__device__ __forceinline__ F2 both(float a) { return pack2(a, a); }
+
+// exp_f of two values in [-80, 0] (no range test, one exact scaling step): the same operations, so the same bits (x - y
+// is x + -y). The rounding to an integer adds and takes off 1.5 2^23, whose sum also holds the integer in its low bits.
+__device__ __forceinline__ F2 exp_neg2(F2 x, F2 z) {
+  const F2 t = add2(mul2(x, both(0x1.715476p+0f), z), both(12582912.0f));
+  const F2 k = add2(t, both(-12582912.0f));
+  const F2 r = add2(add2(x, mul2(k, both(-0x1.62e400p-1f), z)), mul2(k, both(-0x1.7f7d1cp-20f), z));
+  F2 p = both(1.0f / 5040.0f);
+  p = add2(mul2(p, r, z), both(1.0f / 720.0f));
+  p = add2(mul2(p, r, z), both(1.0f / 120.0f));
+  p = add2(mul2(p, r, z), both(1.0f / 24.0f));
+  p = add2(mul2(p, r, z), both(1.0f / 6.0f));
+  p = add2(mul2(p, r, z), both(0.5f));
+  p = add2(mul2(p, r, z), both(1.0f));
+  p = add2(mul2(p, r, z), both(1.0f));
+  float p0, p1, t0, t1;
+  unpack2(p, p0, p1);
+  unpack2(t, t0, t1);
+  return pack2(__uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23)),
+               __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23)));
 }
 
 __device__ __forceinline__ float min_nan(float a, float b) {
@@ -341,8 +317,8 @@ __device__ __forceinline__ bool exceeds_fast(const SamplerRules& r, float tol_lo
 }
 
 struct WarpShared {
-  float4 centre[kCentres];  // cx, cy, 1 / (2 r^2), (6 r)^2
-  float amp[kCentres];
+  float4 centre[kCentres];  // a blob at two lattice slots: -cx, -cx', -cy, -cy'; first, at the window's start: cx, cy, (3 r)^2
+  float4 blob[kCentres];    // -1 / (2 r^2), (6 r)^2, the amplitude; the speed
   uint16_t list[kMaxListed];
   float v[kSplitStage][32];
   uint32_t dt[kSplitStage][32];
@@ -409,9 +385,27 @@ __device__ __forceinline__ void window_tile(const SplitArgs& a, const RestList& 
     __syncwarp();
   }
   const bool listed = n_list >= 0 && n_list <= kCentres;  // else each lane evaluates its own samples
-  // The level rule (field_level), the centres at the window's start shared by the warp.
+  // The listed blobs, one a lane; and the level rule (field_level) from their centres at the window's start.
+  if (listed) {
+    const float ts = t_seconds(t_w);
+    for (int i = static_cast<int>(lane); i < n_list; i += 32) {
+      const float* b = f.blobs + static_cast<size_t>(w.list[i]) * kBlobWords;
+      w.blob[i] = make_float4(-b[5], b[6], b[0], b[8]);
+      w.centre[i] = make_float4(b[1] + b[3] * ts, b[2] + b[4] * ts, b[7], 0.0f);
+    }
+    __syncwarp();
+  }
   int level = a.r.l_min;
-  if (n_list != 0 && f.kind == kFieldBlobs) {
+  if (listed) {
+    float v = 0.0f;
+    for (int i = 0; i < n_list; ++i) {
+      const float4 c = w.centre[i];
+      const float dx = xc - c.x, dy = yc - c.y;
+      const float d2 = dx * dx + dy * dy, speed = w.blob[i].w;
+      v = (d2 <= c.z && speed > v) ? speed : v;
+    }
+    level = level_of_speed(v, a.r.l_min, a.r.l_max);
+  } else if (f.kind == kFieldBlobs) {
     level = field_level(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t_w,
                         a.r.l_min, a.r.l_max);
   }
@@ -424,47 +418,63 @@ __device__ __forceinline__ void window_tile(const SplitArgs& a, const RestList& 
   float p2 = carried, p1 = carried, v_lo = carried, v_hi = carried;
   bool flagged = false;
   uint32_t n = 1;
-  const int group = listed && n_list > 0 ? kCentres / n_list : slots;
-  for (int j0 = 1; j0 <= slots; j0 += group) {
-    const int j1 = j0 + group <= slots + 1 ? j0 + group : slots + 1;
-    if (listed && n_list > 0) {
+  const auto take = [&](int j, float e) {  // the field at slot j, where the lane has it
+    if (!fits || (j & skip) != 0) return;
+    if (n >= 2u) flagged = flagged || (a.r.midpoint != 0 && exceeds_fast(a.r, tol_lo, p2, p1, e));
+    w.v[n - 1u][lane] = e;
+    ++n;
+    p2 = p1;
+    p1 = e;
+    v_lo = min_nan(v_lo, e);
+    v_hi = max_nan(v_hi, e);
+  };
+  if (listed) {
+    // Slots in pairs (1, 2), (3, 4), ..., each blob's term at both in one run of packed operations.
+    const int shift = n_list > 1 ? 32 - __clz(n_list - 1) : 0;  // lanes per pair: the next power of two
+    const int pairs = (slots + 1) / 2, group = n_list > 0 ? kCentres / n_list : pairs;
+    const F2 xc2 = both(xc), yc2 = both(yc), z{a.minus_zero2};
+    for (int g0 = 0; g0 < pairs; g0 += group) {
+      const int g1 = g0 + group < pairs ? g0 + group : pairs;
       __syncwarp();
-      const int entries = (j1 - j0) * n_list;
-      for (int q = static_cast<int>(lane); q < entries; q += 32) {
-        const int i = q % n_list, j = j0 + q / n_list;
-        const float* b = f.blobs + static_cast<size_t>(w.list[i]) * kBlobWords;
-        const float ts = t_seconds(t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine)));
-        w.centre[q] = make_float4(b[1] + b[3] * ts, b[2] + b[4] * ts, b[5], b[6]);
-        w.amp[q] = b[0];
-      }
-      __syncwarp();
-    }
-    for (int j = j0; j < j1; ++j) {
-      const bool mine = fits && (j & skip) == 0;
-      float e = f.base;
-      if (listed) {
-        const int c0 = (j - j0) * n_list;
-        for (int i = 0; i < n_list; ++i) {
-          const float4 c = w.centre[c0 + i];
-          const float dx = xc - c.x, dy = yc - c.y;
-          const float d2 = dx * dx + dy * dy;
-          const bool in = d2 < c.w;
-          const float term = w.amp[c0 + i] * exp_neg(in ? -(d2 * c.z) : 0.0f);
-          e = e + (in ? term : 0.0f);
+      for (int q = static_cast<int>(lane); q < (g1 - g0) << shift; q += 32) {
+        const int i = q & ((1 << shift) - 1), g = g0 + (q >> shift);
+        if (i < n_list) {
+          const float* b = f.blobs + static_cast<size_t>(w.list[i]) * kBlobWords;
+          const float ta = t_seconds(t_w + (static_cast<int64_t>(2 * g + 1) << (kWindowLog2 - fine)));
+          const float tb = t_seconds(t_w + (static_cast<int64_t>(2 * g + 2) << (kWindowLog2 - fine)));
+          w.centre[(g - g0) * n_list + i] = make_float4(-(b[1] + b[3] * ta), -(b[1] + b[3] * tb), -(b[2] + b[4] * ta),
+                                                        -(b[2] + b[4] * tb));
         }
-      } else if (mine) {
-        const int64_t t = t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine));
-        e = field_eval(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y, t);
       }
-      if (mine) {
-        if (n >= 2u) flagged = flagged || (a.r.midpoint != 0 && exceeds_fast(a.r, tol_lo, p2, p1, e));
-        w.v[n - 1u][lane] = e;
-        ++n;
-        p2 = p1;
-        p1 = e;
-        v_lo = min_nan(v_lo, e);
-        v_hi = max_nan(v_hi, e);
+      __syncwarp();
+      for (int g = g0; g < g1; ++g) {
+        F2 e = both(f.base);
+        const float4* centre = w.centre + (g - g0) * n_list;
+        for (int i = 0; i < n_list; ++i) {
+          const float4 c = centre[i], b = w.blob[i];
+          const F2 dx = add2(xc2, pack2(c.x, c.y)), dy = add2(yc2, pack2(c.z, c.w));
+          const F2 d2 = add2(mul2(dx, dx, z), mul2(dy, dy, z));
+          float da, db, xa, xb, ta, tb;
+          unpack2(d2, da, db);
+          unpack2(mul2(d2, both(b.x), z), xa, xb);
+          const bool ina = da < b.y, inb = db < b.y;
+          unpack2(mul2(both(b.z), exp_neg2(pack2(ina ? xa : 0.0f, inb ? xb : 0.0f), z), z), ta, tb);
+          e = add2(e, pack2(ina ? ta : 0.0f, inb ? tb : 0.0f));
+        }
+        float ea, eb;
+        unpack2(e, ea, eb);
+        take(2 * g + 1, ea);
+        if (2 * g + 2 <= slots) take(2 * g + 2, eb);
       }
+    }
+  } else {
+    for (int j = 1; j <= slots; ++j) {
+      float e = 0.0f;
+      if (fits && (j & skip) == 0) {
+        e = field_eval(f, BlobList{n_list > 0 ? w.list : nullptr, n_list > 0 ? n_list : f.n_blobs}, x, y,
+                       t_w + (static_cast<int64_t>(j) << (kWindowLog2 - fine)));
+      }
+      take(j, e);
     }
   }
   float last = p1;
@@ -570,8 +580,9 @@ struct WarpSums {
   }
 };
 
-// Window a.w of every tile.
-__global__ void __launch_bounds__(128, 8) split_window_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
+// Window a.w of every tile. 6 blocks per SM (80 registers): 11.1 ms of engine time on 1280x720 with noise, 23.9 on the
+// five sensors; 11.3 and 24.3 at 7, 11.5 and 24.7 at 8 (11.8 and 24.9 with the field's terms one slot at a time).
+__global__ void __launch_bounds__(128, 6) split_window_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   __shared__ WarpShared sh[4];
   __shared__ SplitSums sums;
@@ -1143,6 +1154,7 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   a.r = r;
   a.tile_lw = static_cast<uint32_t>(tile_lw);
   a.total_blobs = total_blobs;
+  a.minus_zero2 = 0x8000000080000000ull;
   a.px = static_cast<SplitPixel*>(scratch);
   float4* boxes = reinterpret_cast<float4*>(a.px + slots);
   a.q.a = boxes + 2u * total_blobs;

@@ -128,6 +128,19 @@ static __host__ __device__ __noinline__ float field_eval(const FieldDev& f, cons
   return e;
 }
 
+// The lattice level of a pixel under a blob of speed v (0: none): clamp(ceil(log2(v W / 0.25 px)), l_min, l_max).
+BS_HD int32_t level_of_speed(float v, int32_t l_min, int32_t l_max) {
+  if (!(v > 0.0f)) return l_min;
+  const float q = v * 0.033554432f;  // v W / 0.25 px with W = 2^23 ns
+  const uint32_t bq = f2u(q);
+  const int e = static_cast<int>((bq >> 23) & 0xffu) - 126;  // q = m 2^e, m in [0.5, 1) (q is normal)
+  const bool half = (bq & 0x7fffffu) == 0u;                    // m == 0.5: log2 q = e - 1 exactly
+  int32_t level = half ? e - 1 : e;
+  if (level < l_min) level = l_min;
+  if (level > l_max) level = l_max;
+  return level;
+}
+
 // The level rule at the window start: clamp(ceil(log2(v W / 0.25 px)), l_min, l_max), v the speed of the fastest
 // blob whose 3 r support covers the pixel (none, or the tanh edge: l_min).
 BS_HD int32_t field_level(const FieldDev& f, const BlobList& l, uint32_t x, uint32_t y, int64_t t_w, int32_t l_min,
@@ -145,15 +158,7 @@ BS_HD int32_t field_level(const FieldDev& f, const BlobList& l, uint32_t x, uint
     const float d2 = dx * dx + dy * dy;
     v = (d2 <= b[7] && b[8] > v) ? b[8] : v;
   }
-  if (!(v > 0.0f)) return l_min;
-  const float q = v * 0.033554432f;  // v W / 0.25 px with W = 2^23 ns
-  const uint32_t bq = f2u(q);
-  const int e = static_cast<int>((bq >> 23) & 0xffu) - 126;  // q = m 2^e, m in [0.5, 1) (q is normal)
-  const bool half = (bq & 0x7fffffu) == 0u;                    // m == 0.5: log2 q = e - 1 exactly
-  int32_t level = half ? e - 1 : e;
-  if (level < l_min) level = l_min;
-  if (level > l_max) level = l_max;
-  return level;
+  return level_of_speed(v, l_min, l_max);
 }
 
 #if defined(__CUDACC__)

@@ -2064,35 +2064,67 @@ __global__ void learned_reset_kernel(LearnedSoA st, uint32_t n, const float* irr
   store_learned(st, p, n, L);
 }
 
+// Samples of a window not yet taken by the pixel model (entry i at dt[32 i], v[32 i]), fed to it out of line, on copies:
+// few windows come here. pos: where the feed stands.
+constexpr uint32_t kLearnedStage = 8;
+struct FeedPos {
+  int64_t prev_t;
+  float prev_v, x_prev;
+};
+__device__ __noinline__ void feed_samples(PixelRegs* s, const PixelMapRegs* m, const SensorConsts* k, uint32_t pixel,
+                                          GlobalSink sink, PixelCounters* c, int64_t t_w, FeedPos* pos,
+                                          const uint32_t* dt, const float* v, uint32_t n) {
+  PixelRegs sl = *s;
+  PixelCounters cl = *c;
+  PixelProc<GlobalSink> proc{sl, *m, *k, pixel, sink, cl};
+  WindowFeed feed{&proc, t_w, k->irr_max, pos->prev_t, pos->prev_v, 0.0f, pos->x_prev};
+  if (pos->prev_t == t_w) feed.x_prev = proc.x_at_sample(pos->prev_v);
+  for (uint32_t i = 0; i < n; ++i) feed(dt[i * 32u], v[i * 32u]);
+  *pos = FeedPos{feed.prev_t, feed.prev_v, feed.x_prev};
+  *s = sl;
+  *c = cl;
+}
+
 // Per window and warp: every lane with its walk inside the window writes its 16 features, the warp runs the MLP on
-// the tensor cores (32 rows), and each lane takes its proposed step (judge, fallback and pixel model on its own);
-// the loop ends when every lane has reached the window's end.
-// At most 64 registers (8 blocks per SM; 128 uncapped held it to 4): on the 1280x720 held-out field 170.5 against
-// 198.7 ms (186.3 at 6 blocks, 177.2 at 7), the proposals and the events unchanged.
-__global__ void __launch_bounds__(128, 8) learned_engine_kernel(EngineArgs a, LearnedLaunch l) {
+// the tensor cores (32 rows), and each lane takes its proposed step (judge and fallback on its own); the loop ends when
+// every lane has reached the window's end. The samples are staged, and a window that the quick bounds show to be quiet
+// leaves the pixel model out (the split engine's test, engine_split.cu); the others, and a window past the stage, feed
+// it. The shot chain stands at its next candidate that may be accepted, as there.
+// The block's warps take their trips in step (engine_cascade_kernel says why: 19 of the 28 cycles between a warp's issues
+// waited for instructions). 640x360 with noise, 30 windows: 12.6 ms with blocks of 32 warps (64 registers), 13.5 with
+// two of 12, 15.7 with one of 16 (free-running 15.7, and 17.6 with every sample fed to the pixel model).
+constexpr int kLearnedWarps = 32;
+struct alignas(16) LearnedWarpShared {
+  uint16_t rows[32 * kSF];
+  float y[32];
+  uint32_t dt[kLearnedStage][32];
+  float v[kLearnedStage][32];
+  uint16_t list[kMaxListed];
+};
+constexpr size_t kMlpSharedBytes = (sizeof(MlpShared) + 15) / 16 * 16;
+
+__global__ void __launch_bounds__(32 * kLearnedWarps, 1) learned_engine_kernel(EngineArgs a, LearnedLaunch l) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t t0 = *a.t0;
-  __shared__ MlpShared W;
-  __shared__ __align__(16) uint16_t rows[4][32 * kSF];
-  __shared__ float ys[4][32];
-  __shared__ uint16_t lists[4][kMaxListed];
+  extern __shared__ __align__(16) unsigned char learned_shared[];
+  MlpShared& W = *reinterpret_cast<MlpShared*>(learned_shared);
+  LearnedWarpShared& sh = reinterpret_cast<LearnedWarpShared*>(learned_shared + kMlpSharedBytes)[warp];
   mlp_load_shared(W, l.ops, l.params);
-  uint16_t* my_list = lists[warp];
-  uint16_t* my_rows = rows[warp];
-  float* my_y = ys[warp];
+  uint16_t* my_list = sh.list;
+  uint16_t* my_rows = sh.rows;
+  float* my_y = sh.y;
   const bool rec_s = l.rec_samples.capacity > 0, rec_p = l.rec_steps.capacity > 0;
-  for (;;) {
-    uint32_t tile = 0;
-    if (lane == 0) tile = atomicAdd(a.tile_counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if (tile >= a.total_tiles) break;
+  const uint32_t warps = blockDim.x >> 5;
+  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first += gridDim.x * warps) {
+    const uint32_t tile = first + warp < a.total_tiles ? first + warp : a.total_tiles - 1u;
+    const bool real = first + warp < a.total_tiles;  // a warp past the last tile only keeps the barriers
     int si = 0;
     while (si + 1 < a.n_sensors && a.sensors[si + 1].tile0 <= tile) ++si;
     const EngineSensor& S = a.sensors[si];
     const uint32_t local = tile - S.tile0;
     uint32_t x, y;
     tile_xy(local, S.tiles_x, a.tile_lw, lane, x, y);
-    const bool have = x < S.width && y < S.height;
+    const bool have = real && x < S.width && y < S.height;
     const uint32_t np = S.width * S.height;
     const uint32_t p = have ? y * S.width + x : 0u;
     const uint32_t tag = (static_cast<uint32_t>(si) << 24) | p;
@@ -2109,29 +2141,72 @@ __global__ void __launch_bounds__(128, 8) learned_engine_kernel(EngineArgs a, Le
     }
     PixelCounters c;
     unsigned long long samples = 0;
-    GlobalSink sink{S.ev, &S.counters[kCntEvents]};
-    PixelProc<GlobalSink> proc{s, m, S.consts, p, sink, c};
+    const GlobalSink sink{S.ev, &S.counters[kCntEvents]};
     const FieldDev& f = S.field;
+    const int64_t T0 = t0 + static_cast<int64_t>(a.w0) * kWindowNs, T_end = t0 + static_cast<int64_t>(a.w1) * kWindowNs;
+    uint32_t limit = 0;
+    float4 bounds = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const auto next_stop = [&]() {  // the shot chain on to its next stop, and the bounds of the state as it is
+      if (noise && m.shot_max_hz > 0.0 && s.t_shot < T_end) {
+        const uint32_t from = s.n_shot;
+        U4 u = draw(S.consts.seed, kPurposeShot, S.consts.camera, p, s.n_shot);
+        skip_rejected(S.consts, p, limit, m.shot_max_hz, T_end, u, s.t_shot, s.n_shot);
+        c.noise_candidates += s.n_shot - from;
+      }
+      bounds = quick_record(s, m, noise, T0, T_end);
+    };
+    if (have) {
+      limit = accept_limit(m, S.consts, f, carried);
+      next_stop();
+    }
+    uint32_t* my_dt = &sh.dt[0][lane];
+    float* my_v = &sh.v[0][lane];
     for (int32_t w = a.w0; w < a.w1; ++w) {
       const int64_t t_w = t0 + static_cast<int64_t>(w) * kWindowNs;
+      const float tau_a = static_cast<float>(static_cast<double>(t_w - T0) * 1e-9);
+      const float tau_b = static_cast<float>(static_cast<double>(t_w - T0 + kWindowNs) * 1e-9);
       const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, my_list);
       auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
-      WindowFeed feed{&proc, t_w, S.consts.irr_max, t_w, s.held, carried, 0.0f};
       int s_floor = kWindowLog2;
       uint32_t cur = 0;
       float v_cur = carried, x_cur = 0.0f;
       if (have) {
         s_floor = kWindowLog2 - field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
-        feed.start(carried);
         x_cur = log_f(carried);
       }
+      uint32_t staged = 0, n_seg = 0;  // samples in the stage, segments of the window
+      bool fed = false;                // the pixel model has taken the window's first samples
+      FeedPos pos{t_w, clamp_irr(carried, S.consts.irr_max), 0.0f};
+      float v_lo = carried, v_hi = carried, last = carried;
+      const auto flush = [&]() {
+        PixelRegs ts = s;
+        PixelMapRegs tm = m;
+        PixelCounters tc = c;
+        FeedPos tp = pos;
+        feed_samples(&ts, &tm, &S.consts, p, sink, &tc, t_w, &tp, my_dt, my_v, staged);
+        s = ts;
+        c = tc;
+        pos = tp;
+        staged = 0;
+        fed = true;
+      };
       auto emit = [&](uint32_t dt, float v) {
-        feed(dt, v);
+        if (staged == kLearnedStage) flush();
+        my_dt[staged * 32u] = dt;
+        my_v[staged * 32u] = v;
+        ++staged;
+        ++n_seg;
+        v_lo = fminf(v_lo, v);
+        v_hi = fmaxf(v_hi, v);
+        // A NaN never reaches the extremes: it takes the window out of the quick test.
+        if (v != v) v_lo = -1.0f;
+        last = v;
         if (rec_s) rec_push(l.rec_samples, t_w + dt, tag, v);
       };
       for (;;) {
         const bool act = have && cur < static_cast<uint32_t>(kWindowNs);
-        if (!__any_sync(0xffffffffu, act)) break;
+        if (!__syncthreads_or(act)) break;
+        if (!__any_sync(0xffffffffu, act)) continue;
         float feat[16];
         if (act) {
           step_features(L.hx, L.gaps, x_cur, feat);
@@ -2160,8 +2235,22 @@ __global__ void __launch_bounds__(128, 8) learned_engine_kernel(EngineArgs a, Le
       }
       if (have) {
         ++samples;  // the carried slot, as in the plain engine's count
-        s.held = feed.prev_v;
-        carried = feed.last_raw;
+        const float I_hi = m.dark + m.scale * v_hi, I_lo = m.dark + m.scale * v_lo;
+        const float pad = 0x1p-21f * I_hi;
+        const bool quiet = !fed && w - a.w0 < __float_as_int(bounds.w) && v_lo >= 0.0f && v_hi <= S.consts.irr_max &&
+                           __log2f(I_hi + pad) < bounds.x - bounds.z * tau_b &&
+                           __log2f(I_lo - pad) > bounds.y - bounds.z * tau_a && a.r.min_split > 4u;
+        if (quiet) {
+          c.pieces += n_seg;
+          c.leaves += n_seg;
+          s.t_search = maxi(s.t_search, t_w + kWindowNs);
+          s.held = last;
+        } else {
+          flush();
+          s.held = pos.prev_v;
+          next_stop();
+        }
+        carried = last;
       }
       __syncwarp();
     }
@@ -2380,15 +2469,20 @@ void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint3
                            unsigned int* tile_counter, int blocks, int warps_per_block, int tile_lw,
                            cudaStream_t stream) {
   EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w0, w1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
-  (void)warps_per_block;  // 4 warps: the shared tiles are sized for them
-  learned_engine_kernel<<<blocks, 128, 0, stream>>>(a, l);
+  (void)warps_per_block;  // a shape of its own
+  (void)blocks;
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const StepShape c = step_shape(total_tiles, sms, kLearnedWarps);
+  const int bytes = static_cast<int>(kMlpSharedBytes) + c.warps * static_cast<int>(sizeof(LearnedWarpShared));
+  cudaFuncSetAttribute(learned_engine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  learned_engine_kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a, l);
 }
 
 int learned_engine_max_blocks_per_sm(int warps_per_block) {
   (void)warps_per_block;
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, learned_engine_kernel, 128, 0);
-  return n;
+  return 1;  // launch_learned_engine takes a shape of its own (step_shape)
 }
 
 void launch_learned_reset(LearnedSoA st, uint32_t n, const float* irr0, cudaStream_t stream) {

@@ -351,8 +351,8 @@ bs_status bs_engine_take_events(bs_engine* e, bs_event_columns* out);
  * finishing the posted pixels' windows one thread per pixel, or one launch per call for few pixels; the instantaneous
  * response only, and the stage an engine of such sensors starts with; an engine with the noise lattice starts with 32)
  * and the tile width in
- * pixels (4, 8, 16 or 32; the tile is 32 / width pixels high, one warp per tile; 0: 8). The learned engine runs 4 warps
- * per block, the cascade without the lattice one block per SM with as many warps as its tiles need. */
+ * pixels (4, 8, 16 or 32; the tile is 32 / width pixels high, one warp per tile; 0: 8). The learned engine and the
+ * cascade without the lattice run one block per SM with as many warps as their tiles need. */
 bs_status bs_engine_set_launch(bs_engine* e, int32_t warps_per_block, int32_t blocks_per_sm, int32_t stage,
                                int32_t tile_width);
 /* The current launch shape: warps per block, blocks per SM, staging depth, tile width. */

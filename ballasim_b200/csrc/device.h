@@ -302,7 +302,7 @@ struct TrainArgs {
   uint32_t rows;     // rows of this step
   int32_t sampled;   // 1: rows drawn with replacement from n (Philox, keyed by the step counter); 0: rows 0..n-1
   uint64_t seed;
-  const int64_t* step;
+  int64_t* step;  // [0] the completed steps; [1] takes them for launch_adam
   const uint16_t* ops;
   const float* params;
   float* partial;         // [grid][kMlpParamsPad]
@@ -319,7 +319,7 @@ void launch_train_partials(const TrainArgs& a, cudaStream_t stream);
 // step's loss (sum / (2 rows)) at losses[step] when step < loss_cap.
 void launch_adam(float* params, float* m, float* v, uint16_t* ops, const float* partial, const double* partial_loss,
                  int ctas, float lr, float inv_rows, int64_t* step, float* losses, int64_t loss_cap,
-                 unsigned int* done, cudaStream_t stream);
+                 cudaStream_t stream);
 // The summed gradient (FP64) and loss of the partials (the gradient check).
 void launch_reduce_partials(const float* partial, const double* partial_loss, int ctas, float inv_rows,
                             double* grad, double* loss, cudaStream_t stream);

@@ -261,6 +261,12 @@ __device__ __forceinline__ void warp_column_sums(float (&v)[64], int lane) {
   }
 }
 
+// Ordering within a run of steps (programmatic dependent launches: a kernel's head runs while the one before it
+// finishes). Each kernel lets its successor start once its own predecessor has completed, so what lies two kernels back
+// is complete when a kernel starts, and what the predecessor writes is read after this wait.
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __global__ void __launch_bounds__(128, 1) train_partials_kernel(TrainArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TrainTiles& S = *reinterpret_cast<TrainTiles*>(smem_raw);
@@ -275,6 +281,9 @@ __global__ void __launch_bounds__(128, 1) train_partials_kernel(TrainArgs a) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  wait_predecessor();
+  start_successor();
+  if (blockIdx.x == 0 && t == 0) a.step[1] = a.step[0];
   // The operands of the weights (BF16, row-major in ops) into their tiles.
   {
     const int h = t >> 1, j = t & 1;
@@ -504,40 +513,60 @@ __global__ void operands_kernel(const float* params, uint16_t* ops) {
   if (p < kMlpParams) write_operand(ops, p, params[p]);
 }
 
-__global__ void adam_kernel(float* params, float* m, float* v, uint16_t* ops, const float* partial,
-                            const double* partial_loss, int ctas, float lr, float inv_rows, int64_t* step,
-                            float* losses, int64_t loss_cap, unsigned int* done) {
+// step[0]: the completed steps, which the training kernel draws its batch by; step[1]: the same as that kernel saw it,
+// for this one (which moves step[0] on while its blocks still read step[1]). The partial rows are summed in order, 32
+// loads at a time in flight; small blocks spread them over the multiprocessors.
+constexpr int kAdamBlock = 64;
+__global__ void __launch_bounds__(kAdamBlock) adam_kernel(float* params, float* m, float* v, uint16_t* ops,
+                                                          const float* partial, const double* partial_loss, int ctas,
+                                                          float lr, float inv_rows, int64_t* step, float* losses,
+                                                          int64_t loss_cap) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t s = *step;  // completed steps before this one
-  if (p < kMlpParams) {
+  const bool mine = p < kMlpParams;
+  // From the step before (complete): the parameter and its moments.
+  const float p0 = mine ? params[p] : 0.0f, m0 = mine ? m[p] : 0.0f, v0 = mine ? v[p] : 0.0f;
+  wait_predecessor();
+  start_successor();
+  const int64_t s = step[1];
+  if (mine) {
     float gsum = 0.0f;
-    for (int c = 0; c < ctas; ++c) gsum += partial[static_cast<size_t>(c) * kMlpParamsPad + p];
+    int c = 0;
+    for (; c + 32 <= ctas; c += 32) {
+      float g[32];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) g[k] = partial[static_cast<size_t>(c + k) * kMlpParamsPad + p];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) gsum += g[k];
+    }
+    for (; c < ctas; ++c) gsum += partial[static_cast<size_t>(c) * kMlpParamsPad + p];
     const float b1 = 0.9f, b2 = 0.999f;
-    const float mm = b1 * m[p] + (1.0f - b1) * gsum;
-    const float vv = b2 * v[p] + (1.0f - b2) * gsum * gsum;
+    const float mm = b1 * m0 + (1.0f - b1) * gsum;
+    const float vv = b2 * v0 + (1.0f - b2) * gsum * gsum;
     m[p] = mm;
     v[p] = vv;
     const double t = static_cast<double>(s + 1);
     const float c1 = static_cast<float>(1.0 - pow(0.9, t)), c2 = static_cast<float>(1.0 - pow(0.999, t));
-    const float np = params[p] - lr * (mm / c1) / (sqrtf(vv / c2) + 1e-8f);
+    const float np = p0 - lr * (mm / c1) / (sqrtf(vv / c2) + 1e-8f);
     params[p] = np;
     write_operand(ops, p, np);
   }
-  // The last block to finish records the loss and advances the step counter (every block has read it).
-  __syncthreads();
-  __shared__ bool last;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(done, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
+  // The last block (its last threads have no parameter): the step's loss, summed in the CTAs' order, and the counter.
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ double part[kAdamBlock];
     double l = 0.0;
-    for (int c = 0; c < ctas; ++c) l += partial_loss[c];
-    if (losses && s < loss_cap) losses[s] = static_cast<float>(l * 0.5 * inv_rows);
-    *step = s + 1;
-    *done = 0u;
-    __threadfence();
+    for (int c0 = 0; c0 < ctas; c0 += kAdamBlock) {
+      const int n = ctas - c0 < kAdamBlock ? ctas - c0 : kAdamBlock;
+      if (static_cast<int>(threadIdx.x) < n) part[threadIdx.x] = partial_loss[c0 + threadIdx.x];
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        for (int k = 0; k < n; ++k) l += part[k];
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+      if (losses && s < loss_cap) losses[s] = static_cast<float>(l * 0.5 * inv_rows);
+      step[0] = s + 1;
+    }
   }
 }
 
@@ -586,6 +615,24 @@ void launch_walk_pairs(const WalkArgs& a, cudaStream_t stream) {
   walk_pairs_kernel<<<(walkers + 127) / 128, 128, 0, stream>>>(a);
 }
 
+namespace {
+// A launch whose head may overlap the end of the kernel before it in the stream (programmatic stream serialization).
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), int grid, int block, int bytes, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = static_cast<size_t>(bytes);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+}  // namespace
+
 int train_grid(uint32_t rows) { return static_cast<int>((rows + kRowsPerCta - 1) / kRowsPerCta); }
 
 void launch_train_partials(const TrainArgs& a, cudaStream_t stream) {
@@ -595,14 +642,14 @@ void launch_train_partials(const TrainArgs& a, cudaStream_t stream) {
     cudaFuncSetAttribute(train_partials_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     configured = true;
   }
-  train_partials_kernel<<<train_grid(a.rows), kRowsPerCta, bytes, stream>>>(a);
+  launch_after(train_partials_kernel, train_grid(a.rows), kRowsPerCta, bytes, stream, a);
 }
 
 void launch_adam(float* params, float* m, float* v, uint16_t* ops, const float* partial, const double* partial_loss,
                  int ctas, float lr, float inv_rows, int64_t* step, float* losses, int64_t loss_cap,
-                 unsigned int* done, cudaStream_t stream) {
-  adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, stream>>>(params, m, v, ops, partial, partial_loss, ctas, lr,
-                                                             inv_rows, step, losses, loss_cap, done);
+                 cudaStream_t stream) {
+  launch_after(adam_kernel, (kMlpParams + kAdamBlock - 1) / kAdamBlock, kAdamBlock, 0, stream, params, m, v, ops, partial,
+               partial_loss, ctas, lr, inv_rows, step, losses, loss_cap);
 }
 
 void launch_reduce_partials(const float* partial, const double* partial_loss, int ctas, float inv_rows,

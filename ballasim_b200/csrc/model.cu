@@ -1301,7 +1301,7 @@ struct Mlp {
   DevBuf<uint16_t> ops;
   DevBuf<double> partial_loss, grad, loss;
   DevBuf<int64_t> step;
-  DevBuf<unsigned int> done;  // [0]: Adam's block counter; [1]: the training kernel's error word
+  DevBuf<unsigned int> chain_err;  // the training kernel's error word
   cudaStream_t own = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1326,8 +1326,8 @@ struct Mlp {
     m.ensure(kMlpParams);
     v.ensure(kMlpParams);
     ops.ensure(kOpWords);
-    step.ensure(1);
-    done.ensure(2);
+    step.ensure(2);
+    chain_err.ensure(1);
     grad.ensure(kMlpParams);
     loss.ensure(1);
     losses.ensure(kLossCap);
@@ -1352,8 +1352,8 @@ struct Mlp {
     CK(cudaMemsetAsync(m.p, 0, kMlpParams * sizeof(float), own));
     CK(cudaMemsetAsync(v.p, 0, kMlpParams * sizeof(float), own));
     CK(cudaMemsetAsync(ops.p, 0, kOpWords * sizeof(uint16_t), own));
-    CK(cudaMemsetAsync(step.p, 0, sizeof(int64_t), own));
-    CK(cudaMemsetAsync(done.p, 0, 2 * sizeof(unsigned int), own));
+    CK(cudaMemsetAsync(step.p, 0, 2 * sizeof(int64_t), own));
+    CK(cudaMemsetAsync(chain_err.p, 0, sizeof(unsigned int), own));
     launch_operands(params.p, ops.p, own);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(own));
@@ -1381,7 +1381,7 @@ struct Mlp {
     partial.ensure(static_cast<size_t>(ctas) * kMlpParamsPad);
     partial_loss.ensure(ctas);
     TrainArgs a{x, y, n, static_cast<uint32_t>(n), 0, 0, step.p, ops.p, params.p, partial.p, partial_loss.p,
-                1.0f / static_cast<float>(n), 0.5f, done.p + 1};
+                1.0f / static_cast<float>(n), 0.5f, chain_err.p};
     launch_train_partials(a, s);
     launch_reduce_partials(partial.p, partial_loss.p, ctas, a.inv_rows, grad.p, loss.p, s);
     CK(cudaGetLastError());
@@ -1394,9 +1394,9 @@ struct Mlp {
   // The training kernel's error word: a tensor-core chain whose completion it did not see in time.
   void check_chains() {
     unsigned int e = 0;
-    CK(cudaMemcpy(&e, done.p + 1, sizeof(e), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&e, chain_err.p, sizeof(e), cudaMemcpyDeviceToHost));
     if (e != 0) {
-      CK(cudaMemset(done.p + 1, 0, sizeof(e)));
+      CK(cudaMemset(chain_err.p, 0, sizeof(e)));
       throw CudaError("mlp: a tensor-core chain of the training step did not complete within its wait bound");
     }
   }
@@ -1415,11 +1415,11 @@ struct Mlp {
     partial_loss.ensure(ctas);
     const int64_t s0 = steps_from_device(s);
     const TrainArgs a{x, y, n, static_cast<uint32_t>(batch), 1, seed, step.p, ops.p, params.p, partial.p,
-                      partial_loss.p, 1.0f / static_cast<float>(batch), tau, done.p + 1};
+                      partial_loss.p, 1.0f / static_cast<float>(batch), tau, chain_err.p};
     auto one = [&](cudaStream_t st) {
       launch_train_partials(a, st);
       launch_adam(params.p, m.p, v.p, ops.p, partial.p, partial_loss.p, ctas, lr, a.inv_rows, step.p, losses.p,
-                  static_cast<int64_t>(losses.cap), done.p, st);
+                  static_cast<int64_t>(losses.cap), st);
     };
     constexpr int kGraphSteps = 32;
     int32_t left = steps;

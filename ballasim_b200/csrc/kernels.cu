@@ -1211,7 +1211,8 @@ struct CascadeWarpShared {
   float v[kCascadeStage][32];
 };
 
-__global__ void __launch_bounds__(32 * kCascadeWarps, 1) engine_cascade_kernel(EngineArgs a) {
+template <int kWarps, int kBlocks>
+__global__ void __launch_bounds__(32 * kWarps, kBlocks) engine_cascade_kernel(EngineArgs a) {
   extern __shared__ CascadeWarpShared cascade_shared[];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   CascadeWarpShared& sh = cascade_shared[warp];
@@ -1320,6 +1321,16 @@ __global__ void __launch_bounds__(32 * kCascadeWarps, 1) engine_cascade_kernel(E
 struct StepShape {
   int blocks, warps;
 };
+// Up to so many tiles per multiprocessor the warps run apart instead, one to a block and without the register cap: few
+// warps share few fetches, and each would wait for the slowest. Cascade, in step / apart: 97x61 (1.4 tiles) 6.16 / 5.59
+// ms, 160x120 (4.1) 13.7 / 15.2. Learned: 160x120 14.2 / 6.1 ms, 200x150 (6.4) 8.7 / 6.0, 300x220 (14) 9.7 / 10.0.
+constexpr int kCascadeApart = 2, kLearnedApart = 8;
+// The staged lattice kernel's cap pays once the blocks it makes room for are there; uncapped / capped: 64x48 23.3 / 33.6
+// ms, 240x180 (9.1 tiles) 77.6 / 91.0, 300x220 (14) alike within 1 %, 346x260 (19) 95.2 / 89.9.
+constexpr int kLatticeFew = 16;
+bool at_most_per_sm(uint32_t total_tiles, int sms, int tiles) {
+  return total_tiles <= static_cast<uint32_t>(tiles) * static_cast<uint32_t>(sms);
+}
 StepShape step_shape(uint32_t total_tiles, int sms, int most_warps) {
   const uint32_t most = static_cast<uint32_t>(sms) * static_cast<uint32_t>(most_warps);
   const uint32_t rounds = (total_tiles + most - 1) / most;
@@ -1555,10 +1566,11 @@ struct LatticeStageFeed {
   }
 };
 
-// At most 102 registers (168 uncapped), 5 blocks per SM: 87.6 against 92.6 ms on 346x260, 8 windows (a form that kept the
+// kBlocks 5: at most 102 registers, 87.6 against 92.6 ms at 168 (kBlocks 3) on 346x260, 8 windows (a form that kept the
 // block's warps in step, as engine_cascade_kernel does, with the tree walks put off until an eighth of the lanes wait for
 // one, took 133: some pixels need a walk in nearly every cell).
-__global__ void __launch_bounds__(128, 5) engine_lattice_kernel_staged(EngineArgs a) {
+template <int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) engine_lattice_kernel_staged(EngineArgs a) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t t0 = *a.t0;
   __shared__ uint16_t lists[4][kMaxListed];
@@ -2103,7 +2115,8 @@ struct alignas(16) LearnedWarpShared {
 };
 constexpr size_t kMlpSharedBytes = (sizeof(MlpShared) + 15) / 16 * 16;
 
-__global__ void __launch_bounds__(32 * kLearnedWarps, 1) learned_engine_kernel(EngineArgs a, LearnedLaunch l) {
+template <int kWarps, int kBlocks>
+__global__ void __launch_bounds__(32 * kWarps, kBlocks) learned_engine_kernel(EngineArgs a, LearnedLaunch l) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t t0 = *a.t0;
   extern __shared__ __align__(16) unsigned char learned_shared[];
@@ -2421,12 +2434,21 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const StepShape c = step_shape(total_tiles, sms, kCascadeWarps);
+    const bool alone = at_most_per_sm(total_tiles, sms, kCascadeApart);
+    const StepShape c =
+        alone ? StepShape{static_cast<int>(total_tiles), 1} : step_shape(total_tiles, sms, kCascadeWarps);
     const int bytes = c.warps * static_cast<int>(sizeof(CascadeWarpShared));
-    cudaFuncSetAttribute(engine_cascade_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    engine_cascade_kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a);
-  } else if (cascade == 2 && stage != 0) engine_lattice_kernel_staged<<<blocks, warps_per_block * 32, 0, stream>>>(a);
-  else if (cascade == 2) engine_lattice_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
+    const auto kernel = alone ? engine_cascade_kernel<1, kCascadeApart> : engine_cascade_kernel<kCascadeWarps, 1>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a);
+  } else if (cascade == 2 && stage != 0) {
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const auto kernel = at_most_per_sm(total_tiles, sms, kLatticeFew) ? engine_lattice_kernel_staged<3>
+                                                                      : engine_lattice_kernel_staged<5>;
+    kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
+  } else if (cascade == 2) engine_lattice_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 64) engine_kernel_coop<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 16) engine_kernel_staged<16><<<blocks, warps_per_block * 32, 0, stream>>>(a);
   else if (stage == 32) engine_kernel_staged<32><<<blocks, warps_per_block * 32, 0, stream>>>(a);
@@ -2445,7 +2467,7 @@ int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade) {
   if (cascade == 1) {
     n = 1;  // launch_engine takes a shape of its own (step_shape)
   } else if (cascade == 2 && stage != 0) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel_staged, warps_per_block * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel_staged<5>, warps_per_block * 32, 0);
   } else if (cascade == 2) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel, warps_per_block * 32, 0);
   } else if (stage == 64) {
@@ -2474,10 +2496,13 @@ void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint3
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const StepShape c = step_shape(total_tiles, sms, kLearnedWarps);
+  const bool alone = at_most_per_sm(total_tiles, sms, kLearnedApart);
+  const StepShape c =
+      alone ? StepShape{static_cast<int>(total_tiles), 1} : step_shape(total_tiles, sms, kLearnedWarps);
   const int bytes = static_cast<int>(kMlpSharedBytes) + c.warps * static_cast<int>(sizeof(LearnedWarpShared));
-  cudaFuncSetAttribute(learned_engine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  learned_engine_kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a, l);
+  const auto kernel = alone ? learned_engine_kernel<1, kLearnedApart> : learned_engine_kernel<kLearnedWarps, 1>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a, l);
 }
 
 int learned_engine_max_blocks_per_sm(int warps_per_block) {

@@ -14,12 +14,14 @@ pytestmark = pytest.mark.gpu
 
 RULES = W.Rules()
 CASES = {
+    "one round in step": ([(200, 120)], False, RULES, 3),
     "two rounds": ([(400, 250)], False, RULES, 2),
     "one pixel": ([(1, 1)], False, RULES, 12),
     "ragged": ([(75, 43), (33, 9)], False, RULES, 6),
     "past the stage": ([(40, 22)], False, replace(RULES, l_min=5), 3),
     "some past the stage": ([(40, 22)], False, replace(RULES, tol=2e-4), 4),
     "lattice": ([(75, 43), (33, 9)], True, RULES, 3),
+    "lattice, capped": ([(332, 244)], True, RULES, 2),
     "lattice past the stage": ([(24, 16)], True, replace(RULES, l_min=6), 2),
 }
 
@@ -60,3 +62,26 @@ def test_against_the_runs_route(cuda_lib, name):
         total += len(g["p"])
         assert a[i][0].save_state() == b[i][0].save_state()
     assert total > 0 or name == "one pixel"
+
+
+@pytest.mark.parametrize("alone, beside", [((75, 43), (400, 250)), ((1, 1), (320, 160)), ((128, 74), (300, 130))])
+def test_learned_warps_apart_and_in_step(cuda_lib, alone, beside):
+    """A sensor on its own (few tiles: its warps run apart) and beside a larger one (the blocks' warps in step) gives the
+    same events and state."""
+    from ballasim_b200.engine import Engine
+    from ballasim_b200.learned import StepMLP
+    from ballasim_b200.sensor import SensorModel
+
+    net, r, got = StepMLP(seed=3), RULES, []
+    for sizes in ([alone], [alone, beside]):
+        sensors = [(SensorModel(resolve("ideal", W.NOISE), w, h, 60 + i, [{"type": "constant"}], i),
+                    F.blobs(w, h, 60 + i, max(3, w * h // 2000), v_sigma=120.0)) for i, (w, h) in enumerate(sizes)]
+        eng = Engine(sensors, tol=r.tol, dark=r.dark, min_dt_ns=r.min_dt_ns, max_refine_levels=r.max_refine_levels,
+                     l_min=r.l_min, l_max=r.l_max)
+        eng.set_proposal(net, margin=0.0)
+        eng.start(0)
+        eng.run(6)
+        got.append((eng.take_events(with_pixel=True)[0], sensors[0][0].save_state()))
+    for k in got[0][0]:
+        assert got[0][0][k].tobytes() == got[1][0][k].tobytes(), k
+    assert got[0][1] == got[1][1]

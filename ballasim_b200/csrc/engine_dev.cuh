@@ -31,7 +31,7 @@ struct GlobalSink {
 };
 
 // Appends each event with the pushing thread's own atomic: for a kernel whose lanes serve pixels of different
-// sensors (engine_rest_kernel).
+// sensors (split_rest_kernel).
 struct ThreadSink {
   EventBuf ev;
   unsigned long long* count;

@@ -21,10 +21,10 @@
 // would only move its search time to the window's end; where it does not, the model decides. So the events and the
 // state are those of the other engines, bit for bit.
 //
-// Measured on five sensors of 4.3 Mpx with noise, 60 windows: the window kernels 15.2 ms, the rest kernels 8.7, begin
+// Measured on five sensors of 4.3 Mpx with noise, 60 windows: the window kernels 14.1 ms, the rest kernels 8.8, begin
 // 1.5, end 0.16; a form whose window kernel ran the model's clean segments in registers (one logarithm a sample, the
 // noise chains met window by window, the full state through HBM) took 53.0 and 10.0 ms. Issue bounds the window kernel
-// (71 % of its slots), the length of one pixel's chain the rest kernel.
+// (61 % of its slots), the length of one pixel's chain the rest kernel.
 #include "engine_dev.cuh"
 
 namespace bs {

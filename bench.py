@@ -188,16 +188,23 @@ def compute_fraction(wl_name: str, kernel: str, launch: dict, samples: float, km
 def engine_kernel_name(eng, cascade: bool, lattice: bool) -> str:
     if cascade:
         return "engine_lattice_kernel" if lattice else "engine_cascade_kernel"
+    if split_per_window(eng):
+        return "split_window_kernel+split_rest_kernel"
     return {64: "engine_kernel_coop", 16: "engine_kernel_staged<16>", 32: "engine_kernel_staged<32>",
-            1: "split_window_kernel+split_rest_kernel"}.get(eng.launch["stage"], "engine_kernel")
+            1: "split_solo_kernel"}.get(eng.launch["stage"], "engine_kernel")
+
+
+def split_per_window(eng) -> bool:
+    """Whether the split engine launches per window (its whole call is one launch up to two tiles per resident warp)."""
+    tile_w = eng.launch["tile_width"]
+    tiles = sum(-(-m.width // tile_w) * -(-m.height // (32 // tile_w)) for m, _ in eng.sensors)
+    return eng.launch["stage"] == 1 and tiles > 2 * 16 * N_SMS
 
 
 def engine_launches(eng, windows: int) -> int:
     """The engine's kernel launches in one step: one persistent launch, or for the split engine two per window and its
     begin and end kernels."""
-    tile_w = eng.launch["tile_width"]
-    tiles = sum(-(-m.width // tile_w) * -(-m.height // (32 // tile_w)) for m, _ in eng.sensors)
-    return 2 * windows + 2 if eng.launch["stage"] == 1 and tiles > 2 * 16 * N_SMS else 1
+    return 2 * windows + 2 if split_per_window(eng) else 1
 
 
 def run_ours(args, rank: int, world: int) -> dict | None:
@@ -333,7 +340,7 @@ def run_ours(args, rank: int, world: int) -> dict | None:
                 "split_ms_per_step": {k: round(v, 3) for k, v in split.items()}},
         "roofline": {"kernel": kname + " (sampler + pixel model fused, runs kept on chip)"
                      + (" (per window: the common path, then the posted pixels' rare paths; avg_launch_ms is the "
-                        "step's engine time, all windows)" if eng.launch["stage"] == 1 else ""),
+                        "step's engine time, all windows)" if split_per_window(eng) else ""),
                      "bound": "issue",
                      "bound_note": "SIMT fp32 issue and latency (field exps, one log per sample, each crossing's "
                                    "search and fire), not HBM; achieved/peak/frac are the algorithmic bytes of the "

@@ -21,6 +21,7 @@
 
 #include "../../include/ballasim_b200.h"
 #include "device.h"
+#include "split_bufs.h"
 #include "stationary.h"
 
 namespace bs {
@@ -1587,12 +1588,7 @@ struct Engine {
   DevBuf<unsigned long long> rec_count;
   size_t rec_cap = 0;
   unsigned long long rec_n[2] = {0, 0};
-  // The split engine (stage kStageSplit): its scratch (the quick records and blob boxes), the posted-pixel list (room
-  // for every tile's pixels), and a list count per window.
-  DevBuf<float4> split_scratch;
-  DevBuf<unsigned char> rest;
-  DevBuf<unsigned int> split_counts;
-  unsigned int rest_capacity = 0;
+  SplitBufs<DevBuf<float4>, DevBuf<unsigned char>, DevBuf<unsigned int>> split;  // stage kStageSplit's
   uint32_t total_blobs = 0;
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
@@ -1794,13 +1790,8 @@ struct Engine {
   bool split_solo() const { return total_tiles <= 2u * 16u * static_cast<uint32_t>(sm_count()); }
   void ensure_split(int32_t windows) {
     if (total_tiles > (1u << 26)) throw BudgetError("the split engine: too many pixels for its records");
-    const unsigned int slots = total_tiles * 32u;
-    if (rest_capacity < slots) {
-      rest.ensure(static_cast<size_t>(slots) * split_record_bytes());
-      rest_capacity = slots;
-    }
-    split_scratch.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4));
-    split_counts.ensure(static_cast<size_t>(std::max(windows, 1)));
+    split.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4),
+                 total_tiles * 32u, split_record_bytes(), static_cast<size_t>(std::max(windows, 1)));
   }
 
   // One step's device work, in stream order (what the CUDA graph holds): counters cleared, descriptors and the
@@ -1823,12 +1814,12 @@ struct Engine {
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
                               rules, l, tile_counter.p, blocks, block_warps(), tile_lw, st);
       } else if (stage == kStageSplit) {
-        CK(cudaMemsetAsync(split_counts.p, 0, static_cast<size_t>(windows) * sizeof(unsigned int), st));
+        CK(cudaMemsetAsync(split.counts.p, 0, static_cast<size_t>(windows) * sizeof(unsigned int), st));
         const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());
         std::vector<uint32_t> tile0;
         for (const EngineSensor& e : host) tile0.push_back(e.tile0);
         launch_engine_split(sensors_dev.p, tile0.data(), static_cast<int>(host.size()), total_tiles, total_blobs,
-                            t0_dev.p, windows, rules, split_scratch.p, rest.p, split_counts.p, rest_capacity, blocks,
+                            t0_dev.p, windows, rules, split.scratch.p, split.rest.p, split.counts.p, split.capacity, blocks,
                             warps_per_block, tile_lw, rest_blocks, split_solo(), st);
       } else {
         launch_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows, rules,
@@ -1866,9 +1857,7 @@ struct Engine {
       try {
         ensure_split(windows);
       } catch (const BudgetError&) {  // its records (about 300 bytes a pixel) do not fit: the streaming engine's need none
-        split_scratch.release();
-        rest.release();
-        rest_capacity = 0;
+        split.release();
         stage = 0;
       }
     }

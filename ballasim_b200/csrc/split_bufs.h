@@ -1,0 +1,35 @@
+// The split engine's device buffers: its scratch (the pixel and quick records, the blob boxes), the posted-pixel list (a
+// record for every slot of the tiles) and a list count per window. Host code over any buffer type with a pointer p, a
+// capacity cap, ensure(n) (which frees the old allocation before it makes the new one, and throws where that fails) and
+// release(), so that the CPU tests run it over buffers that fail.
+#pragma once
+
+#include <cstddef>
+
+namespace bs {
+
+template <class Scratch, class Rest, class Counts>
+struct SplitBufs {
+  Scratch scratch;
+  Rest rest;
+  Counts counts;
+  unsigned int capacity = 0;  // the records `rest` has room for: 0 wherever it is not allocated
+
+  void ensure(size_t scratch_n, unsigned int slots, size_t record_bytes, size_t windows) {
+    if (capacity < slots || !rest.p) {
+      capacity = 0;
+      rest.ensure(static_cast<size_t>(slots) * record_bytes);
+      capacity = slots;
+    }
+    scratch.ensure(scratch_n);
+    counts.ensure(windows);
+  }
+  void release() {
+    capacity = 0;
+    rest.release();
+    scratch.release();
+    counts.release();
+  }
+};
+
+}  // namespace bs

@@ -1569,8 +1569,8 @@ struct Engine {
   mutable double take_ms[4] = {0, 0, 0, 0};  // sort + split, copy out, host column copies, whole call (ms)
   cudaStream_t own = nullptr;
   cudaEvent_t order = nullptr;
-  // The step as a CUDA graph (rebuilt when its launch shape, window count or proposal changes), fed from pinned
-  // descriptors and model time.
+  // The step as a CUDA graph (rebuilt when its launch shape, window count or proposal changes, dropped where a buffer
+  // that it holds by address moves), fed from pinned descriptors and model time.
   bool use_graph = true;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1791,7 +1791,8 @@ struct Engine {
   void ensure_split(int32_t windows) {
     if (total_tiles > (1u << 26)) throw BudgetError("the split engine: too many pixels for its records");
     split.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4),
-                 total_tiles * 32u, split_record_bytes(), static_cast<size_t>(std::max(windows, 1)));
+                 total_tiles * 32u, split_record_bytes(), static_cast<size_t>(std::max(windows, 1)),
+                 [&] { release_graph(); });
   }
 
   // One step's device work, in stream order (what the CUDA graph holds): counters cleared, descriptors and the
@@ -1857,6 +1858,7 @@ struct Engine {
       try {
         ensure_split(windows);
       } catch (const BudgetError&) {  // its records (about 300 bytes a pixel) do not fit: the streaming engine's need none
+        release_graph();
         split.release();
         stage = 0;
       }

@@ -15,14 +15,21 @@ struct SplitBufs {
   Counts counts;
   unsigned int capacity = 0;  // the records `rest` has room for: 0 wherever it is not allocated
 
-  void ensure(size_t scratch_n, unsigned int slots, size_t record_bytes, size_t windows) {
+  // moving(): called before a buffer is replaced, to drop what holds its address (a captured step).
+  template <class Moving>
+  void ensure(size_t scratch_n, unsigned int slots, size_t record_bytes, size_t windows, Moving moving) {
+    const auto grow = [&](auto& buf, size_t n) {
+      if (n <= buf.cap && buf.p) return;
+      moving();
+      buf.ensure(n);
+    };
     if (capacity < slots || !rest.p) {
       capacity = 0;
-      rest.ensure(static_cast<size_t>(slots) * record_bytes);
+      grow(rest, static_cast<size_t>(slots) * record_bytes);
       capacity = slots;
     }
-    scratch.ensure(scratch_n);
-    counts.ensure(windows);
+    grow(scratch, scratch_n);
+    grow(counts, windows);
   }
   void release() {
     capacity = 0;

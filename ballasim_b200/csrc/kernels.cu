@@ -1340,6 +1340,14 @@ StepShape step_shape(uint32_t total_tiles, int sms, int most_warps) {
           static_cast<int>(warps)};
 }
 
+// Lets `kernel` take `most` bytes of dynamic shared memory, the most of any of its launches and not this one's: the limit
+// belongs to the kernel, so engines of different sizes on different threads have to set the same. false: refused (the
+// error is left for cudaGetLastError).
+template <class... P>
+bool allow_shared(void (*kernel)(P...), size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)) == cudaSuccess;
+}
+
 // The fused engine with the cascade's noise lattice. A cell's look-ahead needs the cell's input up to its end, so
 // the window's samples are buffered from the last one at or before the current time to the first one at or after
 // the cell's end, and the cell then runs on that buffer. A window's last sample is at its end, so each window is
@@ -2437,10 +2445,9 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
     const bool alone = at_most_per_sm(total_tiles, sms, kCascadeApart);
     const StepShape c =
         alone ? StepShape{static_cast<int>(total_tiles), 1} : step_shape(total_tiles, sms, kCascadeWarps);
-    const int bytes = c.warps * static_cast<int>(sizeof(CascadeWarpShared));
     const auto kernel = alone ? engine_cascade_kernel<1, kCascadeApart> : engine_cascade_kernel<kCascadeWarps, 1>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a);
+    if (!allow_shared(kernel, (alone ? 1 : kCascadeWarps) * sizeof(CascadeWarpShared))) return;
+    kernel<<<c.blocks, c.warps * 32, c.warps * sizeof(CascadeWarpShared), stream>>>(a);
   } else if (cascade == 2 && stage != 0) {
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
@@ -2499,10 +2506,10 @@ void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint3
   const bool alone = at_most_per_sm(total_tiles, sms, kLearnedApart);
   const StepShape c =
       alone ? StepShape{static_cast<int>(total_tiles), 1} : step_shape(total_tiles, sms, kLearnedWarps);
-  const int bytes = static_cast<int>(kMlpSharedBytes) + c.warps * static_cast<int>(sizeof(LearnedWarpShared));
+  const auto bytes = [](int warps) { return kMlpSharedBytes + warps * sizeof(LearnedWarpShared); };
   const auto kernel = alone ? learned_engine_kernel<1, kLearnedApart> : learned_engine_kernel<kLearnedWarps, 1>;
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  kernel<<<c.blocks, c.warps * 32, static_cast<size_t>(bytes), stream>>>(a, l);
+  if (!allow_shared(kernel, bytes(alone ? 1 : kLearnedWarps))) return;
+  kernel<<<c.blocks, c.warps * 32, bytes(c.warps), stream>>>(a, l);
 }
 
 int learned_engine_max_blocks_per_sm(int warps_per_block) {

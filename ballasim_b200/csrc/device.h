@@ -176,10 +176,10 @@ int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
 // launch), and split_end_kernel. The state passes from S.in to S.out (carried_in to carried_out). tile0: the sensors'
 // first tiles (host memory); scratch: split_scratch_bytes(), 128-byte aligned.
 constexpr int kStageSplit = 1;
-size_t split_scratch_bytes(uint32_t total_tiles, uint32_t total_blobs);
+size_t split_scratch_bytes(uint32_t total_tiles, size_t total_blobs);
 size_t split_record_bytes();
 void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,
-                         uint32_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
+                         size_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
                          void* rest, unsigned int* rest_counts, unsigned int rest_capacity, int blocks,
                          int warps_per_block, int tile_lw, int rest_blocks, bool solo, cudaStream_t stream);
 int split_solo_blocks_per_sm(int warps_per_block);

@@ -85,7 +85,6 @@ struct SplitArgs {
   int32_t w, windows;
   SamplerRules r;
   uint32_t tile_lw;
-  uint32_t total_blobs;
   unsigned long long minus_zero2;  // two fp32 -0 (mul2)
   uint32_t block_tiles;  // split_solo_kernel: the tiles of a block
   QuickPlanes q;
@@ -1133,7 +1132,7 @@ __global__ void __launch_bounds__(128, 4) split_solo_kernel(const __grid_constan
 
 }  // namespace
 
-size_t split_scratch_bytes(uint32_t total_tiles, uint32_t total_blobs) {
+size_t split_scratch_bytes(uint32_t total_tiles, size_t total_blobs) {
   const size_t slots = static_cast<size_t>(total_tiles) * 32u;
   return slots * (sizeof(SplitPixel) + sizeof(float4) + sizeof(float2) + sizeof(float)) +
          2u * total_blobs * sizeof(float4);
@@ -1141,7 +1140,7 @@ size_t split_scratch_bytes(uint32_t total_tiles, uint32_t total_blobs) {
 size_t split_record_bytes() { return sizeof(RestRecord) + sizeof(RestTimes); }
 
 void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,
-                         uint32_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
+                         size_t total_blobs, const int64_t* t0, int32_t windows, const SamplerRules& r, void* scratch,
                          void* rest, unsigned int* rest_counts, unsigned int rest_capacity, int blocks,
                          int warps_per_block, int tile_lw, int rest_blocks, bool solo, cudaStream_t stream) {
   const size_t slots = static_cast<size_t>(total_tiles) * 32u;
@@ -1153,7 +1152,6 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   a.windows = windows;
   a.r = r;
   a.tile_lw = static_cast<uint32_t>(tile_lw);
-  a.total_blobs = total_blobs;
   a.minus_zero2 = 0x8000000080000000ull;
   a.px = static_cast<SplitPixel*>(scratch);
   float4* boxes = reinterpret_cast<float4*>(a.px + slots);
@@ -1174,8 +1172,8 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   split_begin_kernel<<<(total_tiles + 3) / 4, 128, 0, stream>>>(a);
   for (int32_t w = 0; w < windows; ++w) {
     a.w = w;
-    a.boxes = boxes + (w & 1) * static_cast<size_t>(total_blobs);
-    a.boxes_next = boxes + (1 - (w & 1)) * static_cast<size_t>(total_blobs);
+    a.boxes = boxes + (w & 1) * total_blobs;
+    a.boxes_next = boxes + (1 - (w & 1)) * total_blobs;
     const RestList rl{records, times, rest_counts + w, rest_capacity};
     split_window_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a, rl);
     split_rest_kernel<<<rest_blocks, 128, 0, stream>>>(a, rl);

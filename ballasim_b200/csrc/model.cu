@@ -1123,7 +1123,7 @@ struct FieldHolder {
     f.c = h.c;
     f.speed = h.speed;
     f.width_px = h.width_px;
-    f.n_blobs = h.kind == kFieldBlobs ? h.n_blobs : 0;
+    f.n_blobs = h.kind == kFieldBlobs ? std::max(h.n_blobs, 0) : 0;  // a negative count is an empty table
     f.blobs = nullptr;
     if (f.n_blobs > 0) {
       blobs.ensure(static_cast<size_t>(f.n_blobs) * kBlobWords);
@@ -1589,7 +1589,7 @@ struct Engine {
   size_t rec_cap = 0;
   unsigned long long rec_n[2] = {0, 0};
   SplitBufs<DevBuf<float4>, DevBuf<unsigned char>, DevBuf<unsigned int>> split;  // stage kStageSplit's
-  uint32_t total_blobs = 0;
+  size_t total_blobs = 0;
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
   // 0 the instantaneous response, 1 the cascade, 2 the cascade with its noise lattice (every sensor alike).
@@ -1628,8 +1628,8 @@ struct Engine {
       e.tiles_x = (m->width + 7) / 8;
       e.tiles_y = (m->height + 3) / 4;
       e.tile0 = tile0;
-      e.blob0 = total_blobs;
-      total_blobs += static_cast<uint32_t>(fields.back()->f.n_blobs);
+      e.blob0 = static_cast<uint32_t>(total_blobs);  // read by the split engine, which refuses totals past 32 bits
+      total_blobs += static_cast<size_t>(fields.back()->f.n_blobs);
       tile0 += e.tiles_x * e.tiles_y;
       host.push_back(e);
     }
@@ -1790,6 +1790,7 @@ struct Engine {
   bool split_solo() const { return total_tiles <= 2u * 16u * static_cast<uint32_t>(sm_count()); }
   void ensure_split(int32_t windows) {
     if (total_tiles > (1u << 26)) throw BudgetError("the split engine: too many pixels for its records");
+    if (total_blobs > (size_t{1} << 31)) throw BudgetError("the split engine: too many blobs for its boxes");
     split.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4),
                  total_tiles * 32u, split_record_bytes(), static_cast<size_t>(std::max(windows, 1)),
                  [&] { release_graph(); });

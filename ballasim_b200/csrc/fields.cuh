@@ -37,10 +37,13 @@ struct BlobList {
 };
 
 // Bounds of the field's values over all pixels and times, from the parameters and the blob table in host memory: the
-// base with every term of either sign, widened by the sums' rounding (a blob term lies between 0 and its
-// amplitude, tanh between -1 and 1). Parameters that are not finite give the widest bounds.
+// base with every term of either sign, widened by the sums' rounding. tanh lies between -1 and 1, and a blob's term
+// between 0 and its amplitude where that is finite and 1 / (2 r^2) is neither negative (the exponential would grow with
+// the distance) nor infinite (infinity times the 0 at the centre). Anything else gives the widest bounds.
 inline void field_bounds(FieldDev& f, const float* blobs_host) {
+  const float inf = __builtin_huge_valf();
   double lo = f.base, hi = f.base, mag = lo < 0 ? -lo : lo;
+  bool known = true, falling = true;  // falling: some term may be below 0 (terms >= 0 never round below the base)
   const auto span = [&](double below, double above) {
     lo -= below;
     hi += above;
@@ -51,19 +54,19 @@ inline void field_bounds(FieldDev& f, const float* blobs_host) {
     const double a = f.amp < 0 ? -f.amp : f.amp;
     span(a, a);
   } else {
-    bool negative = false;
+    falling = false;
     for (int32_t k = 0; k < f.n_blobs; ++k) {
       const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
-      negative = negative || !(b[0] >= 0.0f);
+      known = known && b[0] > -inf && b[0] < inf && b[5] >= 0.0f && b[5] < inf;
+      falling = falling || b[0] < 0.0f;
       span(b[0] < 0.0f ? -b[0] : 0.0f, b[0] > 0.0f ? b[0] : 0.0f);
       if (!(b[5] >= 0.0f && b[5] * b[6] <= 79.0f)) f.listable = 0;
     }
-    if (!negative) mag = 0.0;  // adding terms >= 0 never rounds below the base
   }
   const double rounding = 1e-7 * (64.0 + f.n_blobs);  // each sum rounds by at most 2^-24 of the terms so far
-  lo -= rounding * mag;
-  hi += rounding * (mag + hi);
-  if (!(lo > -3e38 && hi < 3e38 && mag < 3e38)) {
+  if (falling) lo -= rounding * mag;
+  hi += rounding * mag;
+  if (!(known && lo > -3e38 && hi < 3e38 && mag < 3e38)) {
     lo = -3e38;
     hi = 3e38;
   }

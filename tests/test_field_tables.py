@@ -1,5 +1,7 @@
 """Blob tables that the fields' own generator does not make, as the C ABI takes them."""
 import ctypes as C
+import subprocess
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -8,6 +10,7 @@ from ballasim_b200 import fields as F
 from ballasim_b200 import workloads as W
 from ballasim_b200.params import resolve
 
+ROOT = Path(__file__).resolve().parents[1]
 RULES = W.Rules()
 
 
@@ -68,3 +71,43 @@ def test_a_negative_count_is_an_empty_table(cuda_lib, sizes):
     assert sum(len(e["p"]) for e in got[1][0]) > 0
     same(got[0], got[1])
     same(got[2], got[1])
+
+
+# name: (word of the blob row, its value) on the first blob of the first sensor
+TABLES = {
+    "an amplitude of NaN": {0: np.nan},
+    "an infinite amplitude": {0: -np.inf},
+    "a term that grows": {0: -5.0, 5: -0.01, 6: 1600.0},  # below 0 from 15 px out to its rim at 40
+    "a NaN falloff": {5: np.nan},
+    "an infinite falloff": {5: np.inf},
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(TABLES))
+def test_noise_under_a_table_out_of_the_ordinary(cuda_lib, name):
+    """The shot candidates that the bound on the field's values lets the split engine skip are ones that the model
+    rejects, whatever the table holds: the streaming engine (which skips none) gives the same events and states."""
+    from ballasim_b200.sampling import field_struct
+
+    rows = {**W.MISMATCH, **W.NOISE, "noise_shot_rate_hz": 60.0}
+    got = []
+    for stage in (1, 0):
+        f = F.blobs(48, 32, 90, 4)
+        b = f.blobs.copy()
+        b[0, 1:5] = (24.0, 16.0, 60.0, -40.0)
+        for k, v in TABLES[name].items():
+            b[0, k] = np.float32(v)
+        f.blobs = b
+        got.append(play(sensors([(48, 32)], rows), [field_struct(f)], stage, [np.full(48 * 32, f.base, np.float32)], (4, 12)))
+    assert sum(np.count_nonzero(e["label"] == 1) for e in got[1][0]) > 20
+    same(got[0], got[1])
+
+
+def test_bounds_hold_every_sample(tmp_path):
+    """field_bounds on the CPU over random fields (tests/native/field_bounds.cc)."""
+    exe = tmp_path / "field_bounds"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", f"-I{ROOT / 'ballasim_b200' / 'csrc'}",
+                    str(ROOT / "tests" / "native" / "field_bounds.cc"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr

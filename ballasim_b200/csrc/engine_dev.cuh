@@ -411,6 +411,18 @@ struct RegFeed {
 // ---------------------------------------------------------------------------------------------
 // Quiet windows and noise stops (the split engine's header comment says what they are for)
 // ---------------------------------------------------------------------------------------------
+// The extremes of a window's samples: a NaN stays in both, so no bound holds for it.
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // The quick record's bounds from the state. Delta = ln(I / i_scale) - s3 - n3 + (leak (t - t_ref) 1e-9 + dr), so it
 // stays below theta_on while log2 I < upper - leak log2(e) (t - T0), and above -theta_off alike. The slack, 2e-5 of the
 // sum of the terms' magnitudes, is over 20 times what the roundings of Delta (four fp32 operations, log_f, the

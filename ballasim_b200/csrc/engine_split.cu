@@ -294,17 +294,6 @@ __device__ __forceinline__ F2 exp_neg2(F2 x, F2 z) {
                __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23)));
 }
 
-__device__ __forceinline__ float min_nan(float a, float b) {
-  float r;
-  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float max_nan(float a, float b) {
-  float r;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
-  return r;
-}
-
 // exceeds() with the quotient formed only near the tolerance (tol_lo: the tolerance less 2^-20 of it, below which the
 // rounded quotient cannot exceed it; a NaN or a denominator that is not positive takes the quotient).
 __device__ __forceinline__ bool exceeds_fast(const SamplerRules& r, float tol_lo, float a, float m, float b) {

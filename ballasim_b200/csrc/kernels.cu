@@ -2198,7 +2198,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks) learned_engine_kernel(En
       uint32_t staged = 0, n_seg = 0;  // samples in the stage, segments of the window
       bool fed = false;                // the pixel model has taken the window's first samples
       FeedPos pos{t_w, clamp_irr(carried, S.consts.irr_max), 0.0f};
-      float v_lo = carried, v_hi = carried, last = carried;
+      float v_lo = carried, v_hi = carried, last = carried;  // a NaN among the samples stays in both extremes
       const auto flush = [&]() {
         PixelRegs ts = s;
         PixelMapRegs tm = m;
@@ -2217,10 +2217,8 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks) learned_engine_kernel(En
         my_v[staged * 32u] = v;
         ++staged;
         ++n_seg;
-        v_lo = fminf(v_lo, v);
-        v_hi = fmaxf(v_hi, v);
-        // A NaN never reaches the extremes: it takes the window out of the quick test.
-        if (v != v) v_lo = -1.0f;
+        v_lo = min_nan(v_lo, v);
+        v_hi = max_nan(v_hi, v);
         last = v;
         if (rec_s) rec_push(l.rec_samples, t_w + dt, tag, v);
       };

@@ -1736,6 +1736,9 @@ struct Engine {
   }
 
   int block_warps() const { return mlp ? 4 : warps_per_block; }
+  // The stage that set_launch takes back: with a proposal the split engine is refused and no stage matters, so 0 stands
+  // for it there.
+  int reported_stage() const { return mlp && stage == kStageSplit ? 0 : stage; }
   static int sm_count() {
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
@@ -2002,8 +2005,10 @@ struct Engine {
     if (lw != 0 && (lw < 2 || lw > 5)) throw std::invalid_argument("engine: tile width 4, 8, 16 or 32");
     warps_per_block = warps ? warps : 4;
     blocks_per_sm = per_sm;
-    stage = stg;
-    stage_chosen = true;
+    if (!mlp || stg != reported_stage()) {  // with a proposal the reported stage leaves the plain sampler's as it is
+      stage = stg;
+      stage_chosen = true;
+    }
     tile_lw = lw ? lw : 3;
     retile();
   }
@@ -2551,7 +2556,7 @@ bs_status bs_engine_get_launch(const bs_engine* e, int32_t out[4]) {
     NEED(out);
     out[0] = e->warps_per_block;
     out[1] = e->blocks_per_sm;
-    out[2] = e->stage;
+    out[2] = e->reported_stage();
     out[3] = 1 << e->tile_lw;
   });
 }

@@ -1687,6 +1687,7 @@ struct Engine {
   void set_proposal(const Mlp* p, float mg) {
     if (p && !std::isfinite(mg)) throw std::invalid_argument("engine: margin must be finite");
     if (p && cascade()) throw std::invalid_argument("engine: the learned proposal runs with the instantaneous response");
+    release_graph();  // it holds the old network's buffers, and a new one can stand at the old one's address
     mlp = p;
     margin = mg;
     if (p) {

@@ -45,3 +45,31 @@ def test_a_replay_finds_its_buffers(cuda_lib, name):
         for k in a:
             assert np.asarray(a[k]).tobytes() == np.asarray(b[k]).tobytes(), k
     assert state == want_state
+
+
+def test_a_network_in_place_of_another(cuda_lib):
+    """Each network dies before the next one is made, which may then stand at its address. Their last biases differ by
+    a step's length (log2), so that each proposes other steps than the one before."""
+    from ballasim_b200.engine import Engine
+    from ballasim_b200.learned import StepMLP
+    from ballasim_b200.sensor import SensorModel
+
+    r, got = W.Rules(), []
+    for graph in (True, False):
+        m = SensorModel(resolve("ideal", {**W.MISMATCH, **W.NOISE}), 48, 32, 5, [{"type": "constant"}], 0)
+        eng = Engine([(m, F.blobs(48, 32, 5, 6))], tol=r.tol, dark=r.dark, min_dt_ns=r.min_dt_ns,
+                     max_refine_levels=r.max_refine_levels, l_min=r.l_min, l_max=r.l_max)
+        eng.set_graph(graph)
+        eng.start(0)
+        rows = []
+        for seed in range(6):
+            eng.set_proposal(None)
+            net = StepMLP(seed=seed)
+            net.params = np.append(net.params[:-1], np.float32(seed + 6))
+            eng.set_proposal(net, margin=0.0)
+            del net
+            eng.start(0)
+            rows.append((eng.run(5), m.take_events(with_pixel=True)["t_cross_ns"].tobytes(), m.save_state()))
+        got.append(rows)
+    assert got[0] == got[1]
+    assert len({samples for (samples, _), _, _ in got[1]}) > 1  # the networks do propose other steps

@@ -271,8 +271,7 @@ struct Model {
   DevBuf<SensorConsts> k_dev;  // a device copy of k (the row-major kernel's out-of-line calls read it)
   DevBuf<unsigned long long> counters;
   PinBuf<unsigned long long> counters_h;
-  DevBuf<RawEvent> events;
-  size_t event_cap = 0;
+  DevBuf<RawEvent> events;     // room for events.cap of them
   size_t last_events = 0;      // events of the last device call (on the device)
   int64_t events_lo = 0, events_hi = -1;  // the times `events` holds (of the last call that wrote it)
   std::vector<RawEvent> kept;  // host-kept events (advance_runs, engine runs)
@@ -463,10 +462,11 @@ struct Model {
     map.shot_max = mapd.p + n;
   }
 
+  // Growing drops the events there were, also where the new buffer is refused: there is room for none then.
   void ensure_events(size_t cap) {
-    if (cap <= event_cap) return;
+    if (cap <= events.cap) return;
+    last_events = 0;
     events.ensure(cap);
-    event_cap = cap;
   }
 
   void read_counters(cudaStream_t s) {
@@ -618,7 +618,7 @@ struct Model {
     if (r.n > n) throw std::invalid_argument("SensorModel.advance: more runs than pixels");
     for (int attempt = 0;; ++attempt) {
       CK(cudaMemsetAsync(counters.p, 0, kCntWords * sizeof(unsigned long long), s));
-      const EventBuf evb{events.p, static_cast<unsigned long long>(event_cap)};
+      const EventBuf evb{events.p, static_cast<unsigned long long>(events.cap)};
       if (!k.cascade && (block == 0 || block == 1)) {
         // The instantaneous response: row-major over the runs, long runs walked by the whole warp; split (block 0):
         // a row stopped at its first segment that is not clean is finished by a second kernel, one thread per row.
@@ -658,7 +658,7 @@ struct Model {
       launch_ms_max = std::max(launch_ms_max, static_cast<double>(ms));
       const unsigned long long* c = counters_h.p;
       if (c[kCntErrors] != 0) throw std::invalid_argument(error_text(c[kCntErrors]));
-      if (c[kCntEvents] > event_cap) {
+      if (c[kCntEvents] > events.cap) {
         ++stat_reruns;
         ensure_events(static_cast<size_t>(c[kCntEvents] + c[kCntEvents] / 4 + 1024));
         continue;
@@ -1777,7 +1777,7 @@ struct Engine {
       e.map = m->map;
       e.carried_in = carried[2 * i + carried_cur[i]]->p;
       e.carried_out = carried[2 * i + 1 - carried_cur[i]]->p;
-      e.ev = EventBuf{m->events.p, static_cast<unsigned long long>(m->event_cap)};
+      e.ev = EventBuf{m->events.p, static_cast<unsigned long long>(m->events.cap)};
       e.counters = m->counters.p;
       if (mlp) {
         e.lin = lbufs[2 * i + lcur[i]]->soa(m->n);
@@ -1910,7 +1910,7 @@ struct Engine {
       bool rerun = false;
       for (Model* m : models) {
         const unsigned long long ev = m->counters_h.p[kCntEvents];
-        if (ev > m->event_cap) {
+        if (ev > m->events.cap) {
           m->ensure_events(static_cast<size_t>(ev + ev / 4 + 1024));
           ++m->stat_reruns;
           rerun = true;

@@ -1700,8 +1700,7 @@ struct Engine {
     rec_cap = cap;
     rec_n[0] = rec_n[1] = 0;
     if (cap) {
-      rec[0].ensure(cap);
-      rec[1].ensure(cap);
+      with_room<BudgetError>([&] { rec[0].ensure(cap), rec[1].ensure(cap); }, [&] { return give_way(); });
     }
     rec_count.ensure(2);
   }
@@ -1800,6 +1799,18 @@ struct Engine {
                  [&] { release_graph(); });
   }
 
+  bool split_runs() const { return stage == kStageSplit && !mlp; }
+  // Frees the split engine's records (about 300 bytes a pixel) where memory is short: where they are not in use, and
+  // where the constructor chose that engine, which then gives way to the streaming one (it needs none). false: nothing
+  // to free.
+  bool give_way() {
+    if (split_runs() ? stage_chosen : split.empty()) return false;
+    release_graph();
+    split.release();
+    if (split_runs()) stage = 0;
+    return true;
+  }
+
   // One step's device work, in stream order (what the CUDA graph holds): counters cleared, descriptors and the
   // model time uploaded from pinned memory, the persistent kernel between two timing events, counters read back.
   void enqueue(int32_t windows, int blocks, cudaStream_t st, bool capturing) {
@@ -1819,7 +1830,7 @@ struct Engine {
                               RecBuf{rec[0].p, rec_count.p, rec_cap}, RecBuf{rec[1].p, rec_count.p + 1, rec_cap}};
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
                               rules, l, tile_counter.p, blocks, block_warps(), tile_lw, st);
-      } else if (stage == kStageSplit) {
+      } else if (split_runs()) {
         CK(cudaMemsetAsync(split.counts.p, 0, static_cast<size_t>(windows) * sizeof(unsigned int), st));
         const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());
         std::vector<uint32_t> tile0;
@@ -1859,21 +1870,12 @@ struct Engine {
       if ((t0 & (kWindowNs - 1)) != 0) throw std::invalid_argument("engine: the model time must be a window start");
     }
     if (mlp && lcur.size() != models.size()) throw std::logic_error("engine: call start() after set_proposal()");
-    if (stage == kStageSplit && !mlp && !stage_chosen) {
-      try {
-        ensure_split(windows);
-      } catch (const BudgetError&) {  // its records (about 300 bytes a pixel) do not fit: the streaming engine's need none
-        release_graph();
-        split.release();
-        stage = 0;
-      }
-    }
-    const int blocks = grid_blocks();
     t0_pin.ensure(1);
     rec_n_pin.ensure(2);
     for (;;) {
+      with_room<BudgetError>([&] { if (split_runs()) ensure_split(windows); }, [&] { return give_way(); });
+      const int blocks = grid_blocks();
       describe(t0);
-      if (stage == kStageSplit && !mlp) ensure_split(windows);
       if (use_graph && rec_cap == 0) {
         const uint64_t key[8] = {static_cast<uint64_t>(windows), static_cast<uint64_t>(blocks),
                                  static_cast<uint64_t>(block_warps()), static_cast<uint64_t>(stage),
@@ -1911,7 +1913,8 @@ struct Engine {
       for (Model* m : models) {
         const unsigned long long ev = m->counters_h.p[kCntEvents];
         if (ev > m->events.cap) {
-          m->ensure_events(static_cast<size_t>(ev + ev / 4 + 1024));
+          with_room<BudgetError>([&] { m->ensure_events(static_cast<size_t>(ev + ev / 4 + 1024)); },
+                                 [&] { return give_way(); });
           ++m->stat_reruns;
           rerun = true;
         }

@@ -31,6 +31,7 @@ struct SplitBufs {
     grow(scratch, scratch_n);
     grow(counts, windows);
   }
+  bool empty() const { return !rest.p && !scratch.p && !counts.p; }
   void release() {
     capacity = 0;
     rest.release();
@@ -38,5 +39,17 @@ struct SplitBufs {
     counts.release();
   }
 };
+
+// need(), which allocates; where memory is short (it throws Short) and give_way() could free some, once more.
+template <class Short, class Need, class GiveWay>
+void with_room(Need need, GiveWay give_way) {
+  try {
+    need();
+    return;
+  } catch (const Short&) {
+    if (!give_way()) throw;
+  }
+  need();
+}
 
 }  // namespace bs

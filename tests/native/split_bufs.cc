@@ -115,12 +115,42 @@ void captured_addresses() {
   CHECK(moves == 0);  // nothing moves for a call that fits
 }
 
+// A need that does not fit beside the buffers: they give way once, and what is refused after that is refused.
+void gives_way() {
+  Bufs b;
+  most = 1000;
+  b.ensure(10, 8, 100, 2, [] {});
+  CHECK(!b.empty());
+  FakeBuf events;
+  int tries = 0, given = 0;
+  const auto need = [&](size_t n) {
+    return [&, n] {
+      ++tries;
+      most = b.empty() ? 2000 : 1000;
+      events.ensure(n);
+    };
+  };
+  const auto give = [&] {
+    if (b.empty()) return false;
+    b.release();
+    ++given;
+    return true;
+  };
+  bs::with_room<Refused>(need(900), give);
+  CHECK(tries == 1 && given == 0 && events.cap == 900);
+  bs::with_room<Refused>(need(1500), give);
+  CHECK(tries == 3 && given == 1 && events.cap == 1500 && b.empty());
+  CHECK(refused([&] { bs::with_room<Refused>(need(3000), give); }));
+  CHECK(tries == 4 && given == 1 && events.p == nullptr);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const char* name = argc > 1 ? argv[1] : "";
   if (!std::strcmp(name, "refused_list")) refused_list();
   else if (!std::strcmp(name, "captured_addresses")) captured_addresses();
+  else if (!std::strcmp(name, "gives_way")) gives_way();
   else return 2;
   return failures ? 1 : 0;
 }

@@ -16,7 +16,7 @@ def exe(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("check", ["refused_list", "captured_addresses"])
+@pytest.mark.parametrize("check", ["refused_list", "captured_addresses", "gives_way"])
 def test_split_buffers(exe, check):
     r = subprocess.run([str(exe), check], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -1697,12 +1697,13 @@ struct Engine {
   }
 
   void set_record(size_t cap) {
-    rec_cap = cap;
+    rec_cap = 0;  // also where the rows do not fit
     rec_n[0] = rec_n[1] = 0;
+    rec_count.ensure(2);
     if (cap) {
       with_room<BudgetError>([&] { rec[0].ensure(cap), rec[1].ensure(cap); }, [&] { return give_way(); });
     }
-    rec_count.ensure(2);
+    rec_cap = cap;
   }
 
   // Copies up to cap rows of record `which` (0 samples, 1 proposed steps) of the last run; n gets the rows recorded

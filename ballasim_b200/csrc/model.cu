@@ -2020,33 +2020,52 @@ struct Engine {
 
   // Times each candidate launch shape on trial steps of `windows` windows from the current state (the models keep
   // their state) and keeps the fastest. Candidates: tile width 4, 8, 16 px (height 8, 4, 2) x warps per block 2, 4 x
-  // staging depth 0, 16, 64 (32 deep with the warp-cooperative search; the learned engine: tile widths only; the
-  // cascade: stage 0; the lattice: 0 or 32). Returns the candidates tried (ms of the second of
-  // two trial steps each); rows are {tile_lw, warps, stage, ms}.
+  // stage 0, 1 (split), 16, 64 (32 deep with the warp-cooperative search); the learned engine: tile widths only; the
+  // cascade: stage 0; the lattice: stage 0 or 32. A candidate whose buffers do not fit
+  // is left out; where none fits or a trial fails, the shape is what it was. Returns the candidates tried (ms of the
+  // second of two trial steps each); rows are {tile_lw, warps, stage, ms}.
   std::vector<std::array<double, 4>> autotune(int32_t windows, cudaStream_t s) {
     if (windows < 1) throw std::invalid_argument("engine.autotune: windows >= 1");
     std::vector<std::array<double, 4>> rows;
     const int keep[4] = {tile_lw, warps_per_block, stage, blocks_per_sm};
+    const bool keep_chosen = stage_chosen;
     double best = 1e300;
     int bl = keep[0], bw = keep[1], bs = keep[2];
-    for (int lw : {2, 3, 4}) {
-      for (int w : {2, 4}) {
-        for (int st : {0, kStageSplit, 16, 64}) {
-          if ((mlp && (w != 4 || st != 0)) || (cascade() == 1 && st != 0)) continue;
-          if (cascade() == 2 && (st == 64 || st == kStageSplit)) continue;
-          if (cascade() == 2 && st != 0) st = 32;
-          set_launch(w, 0, st, lw);
-          step(windows, s, false, nullptr, nullptr);
-          step(windows, s, false, nullptr, nullptr);
-          rows.push_back({static_cast<double>(lw), static_cast<double>(w), static_cast<double>(st), last_ms});
-          if (last_ms < best) {
-            best = last_ms;
-            bl = lw;
-            bw = w;
-            bs = st;
+    std::string refused;
+    try {
+      for (int lw : {2, 3, 4}) {
+        for (int w : {2, 4}) {
+          for (int st : {0, kStageSplit, 16, 64}) {
+            if ((mlp && (w != 4 || st != 0)) || (cascade() == 1 && st != 0)) continue;
+            if (cascade() == 2 && (st == 64 || st == kStageSplit)) continue;
+            if (cascade() == 2 && st != 0) st = 32;
+            set_launch(w, 0, st, lw);
+            try {
+              step(windows, s, false, nullptr, nullptr);
+              step(windows, s, false, nullptr, nullptr);
+            } catch (const BudgetError& e) {
+              refused = e.what();
+              continue;
+            }
+            rows.push_back({static_cast<double>(lw), static_cast<double>(w), static_cast<double>(st), last_ms});
+            if (last_ms < best) {
+              best = last_ms;
+              bl = lw;
+              bw = w;
+              bs = st;
+            }
           }
         }
       }
+      if (rows.empty()) throw BudgetError(refused);
+    } catch (...) {
+      tile_lw = keep[0];
+      warps_per_block = keep[1];
+      stage = keep[2];
+      blocks_per_sm = keep[3];
+      stage_chosen = keep_chosen;
+      retile();
+      throw;
     }
     set_launch(bw, keep[3], bs, bl);
     return rows;

@@ -38,3 +38,25 @@ def test_launch_goes_back_in(cuda_lib, kind):
     assert eng.launch == before
     eng.start(0)
     assert eng.run(2)[0] > 0
+
+
+@pytest.mark.parametrize("kind, shapes", [("learned", 3), ("lattice", 12)])
+def test_the_autotuner_tries_a_shape_once(cuda_lib, kind, shapes):
+    from ballasim_b200.learned import StepMLP
+
+    eng, _ = engine("ideal" if kind == "learned" else "prophesee_gen3", {**W.MISMATCH, "noise": kind == "lattice"})
+    if kind == "learned":
+        eng.set_proposal(StepMLP(seed=1))
+    eng.start(0)
+    rows = eng.autotune(2)
+    assert len(rows) == shapes == len({(r["tile_width"], r["warps_per_block"], r["stage"]) for r in rows})
+    assert eng.launch["tile_width"] == min(rows, key=lambda r: r["ms"])["tile_width"]
+
+
+def test_a_failed_autotune_leaves_the_shape(cuda_lib):
+    eng, m = engine("ideal", {**W.MISMATCH, "noise": False})
+    eng.set_launch(2, 3, 16, 16)
+    shape = eng.launch
+    with pytest.raises(RuntimeError):  # before start()
+        eng.autotune(2)
+    assert eng.launch == shape

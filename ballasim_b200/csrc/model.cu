@@ -2020,8 +2020,8 @@ struct Engine {
 
   // Times each candidate launch shape on trial steps of `windows` windows from the current state (the models keep
   // their state) and keeps the fastest. Candidates: tile width 4, 8, 16 px (height 8, 4, 2) x warps per block 2, 4 x
-  // stage 0, 1 (split), 16, 64 (32 deep with the warp-cooperative search); the learned engine: tile widths only; the
-  // cascade: stage 0; the lattice: stage 0 or 32. A candidate whose buffers do not fit
+  // stage 0, 1 (split), 16, 64 (32 deep with the warp-cooperative search); the learned engine and the cascade, whose
+  // blocks have a shape of their own: tile widths only; the lattice: stage 0 or 32. A candidate whose buffers do not fit
   // is left out; where none fits or a trial fails, the shape is what it was. Returns the candidates tried (ms of the
   // second of two trial steps each); rows are {tile_lw, warps, stage, ms}.
   std::vector<std::array<double, 4>> autotune(int32_t windows, cudaStream_t s) {
@@ -2036,7 +2036,7 @@ struct Engine {
       for (int lw : {2, 3, 4}) {
         for (int w : {2, 4}) {
           for (int st : {0, kStageSplit, 16, 64}) {
-            if ((mlp && (w != 4 || st != 0)) || (cascade() == 1 && st != 0)) continue;
+            if ((mlp || cascade() == 1) && (w != 4 || st != 0)) continue;
             if (cascade() == 2 && (st == 64 || st == kStageSplit)) continue;
             if (cascade() == 2 && st != 0) st = 32;
             set_launch(w, 0, st, lw);

@@ -40,7 +40,7 @@ def test_launch_goes_back_in(cuda_lib, kind):
     assert eng.run(2)[0] > 0
 
 
-@pytest.mark.parametrize("kind, shapes", [("learned", 3), ("lattice", 12)])
+@pytest.mark.parametrize("kind, shapes", [("learned", 3), ("cascade", 3), ("lattice", 12)])
 def test_the_autotuner_tries_a_shape_once(cuda_lib, kind, shapes):
     from ballasim_b200.learned import StepMLP
 

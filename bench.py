@@ -353,7 +353,7 @@ def run_ours(args, rank: int, world: int) -> dict | None:
                                                  clocks.get("sm_mhz"))},
     }
     if world == 1 and not (args.no_cpu_baseline or args.profile):
-        out["cpu_baseline"] = cpu_baseline(wl, cpu_windows(args))
+        out.update(beside(lambda: cpu_baseline(wl, cpu_windows(args))))
     if rank == 0 and not (args.no_learned or args.profile):
         out["learned_vs_plain"] = learned_comparison(steps=args.learned_steps)
     return out
@@ -599,8 +599,25 @@ def run_sink(args, rank: int, world: int) -> dict | None:
                      "traffic": None, "algorithmic_bytes_per_launch": alg, "avg_launch_ms": kms},
     }
     if world == 1 and not (args.no_cpu_baseline or args.profile):
-        out["cpu_baseline"] = sink_reference(fmt, es, 8 << 20)
+        out.update(beside(lambda: sink_reference(fmt, es, 8 << 20)))
     return out
+
+
+def no_reference() -> str | None:
+    """Why the reference's own CPU path cannot run here (its library, oracle/_ref, is built from its sources), or None."""
+    from oracle.oracle import Ref
+
+    try:
+        Ref.lib()
+    except (OSError, RuntimeError) as e:
+        return " ".join(str(e).split())
+    return None
+
+
+def beside(measure) -> dict:
+    """The reference's figure for the result line; null, with the reason, where it cannot run."""
+    why = no_reference()
+    return {"cpu_baseline": None, "cpu_baseline_unavailable": why} if why else {"cpu_baseline": measure()}
 
 
 def sink_reference(fmt: str, es, n: int) -> dict:
@@ -713,6 +730,9 @@ def cpu_baseline(wl: W.Workload, windows: int) -> dict:
 def run_reference(args, rank: int) -> dict | None:
     if rank != 0:
         return None
+    why = no_reference()
+    if why:
+        return {"impl": "reference", "unavailable": why}
     if args.workload in SINKS:
         es = W.event_stream()
         vals, cb = [], None

@@ -1325,8 +1325,8 @@ struct StepShape {
 // warps share few fetches, and each would wait for the slowest. Cascade, in step / apart: 97x61 (1.4 tiles) 6.16 / 5.59
 // ms, 160x120 (4.1) 13.7 / 15.2. Learned: 160x120 14.2 / 6.1 ms, 200x150 (6.4) 8.7 / 6.0, 300x220 (14) 9.7 / 10.0.
 constexpr int kCascadeApart = 2, kLearnedApart = 8;
-// The staged lattice kernel's cap pays once the blocks it makes room for are there; uncapped / capped: 64x48 23.3 / 33.6
-// ms, 240x180 (9.1 tiles) 77.6 / 91.0, 300x220 (14) alike within 1 %, 346x260 (19) 95.2 / 89.9.
+// The staged lattice kernel's cap pays once the blocks it makes room for are there; uncapped / capped: 64x48 22.5 / 34.2
+// ms, 240x180 (9.1 tiles) 75.7 / 90.9, 300x220 (14) 90.1 / 92.5, 320x240 (16) 84.9 / 81.6, 346x260 (19) 94.7 / 89.0.
 constexpr int kLatticeFew = 16;
 bool at_most_per_sm(uint32_t total_tiles, int sms, int tiles) {
   return total_tiles <= static_cast<uint32_t>(tiles) * static_cast<uint32_t>(sms);
@@ -1574,9 +1574,10 @@ struct LatticeStageFeed {
   }
 };
 
-// kBlocks 5: at most 102 registers, 87.6 against 92.6 ms at 168 (kBlocks 3) on 346x260, 8 windows (a form that kept the
-// block's warps in step, as engine_cascade_kernel does, with the tree walks put off until an eighth of the lanes wait for
-// one, took 133: some pixels need a walk in nearly every cell).
+// kBlocks 5: at most 102 registers, 89.0 against 94.7 ms at 168 (kBlocks 0, the compiler's own; asking for the 3 blocks
+// that fit there gave the same 168 by another allocation, 77.4 against 75.7 ms on 240x180) on 346x260, 8 windows. A form
+// that kept the block's warps in step, as engine_cascade_kernel does, with the tree walks put off until an eighth of the
+// lanes wait for one, took 133 where this one took 88: some pixels need a walk in nearly every cell.
 template <int kBlocks>
 __global__ void __launch_bounds__(128, kBlocks) engine_lattice_kernel_staged(EngineArgs a) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -2450,7 +2451,7 @@ void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t tota
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const auto kernel = at_most_per_sm(total_tiles, sms, kLatticeFew) ? engine_lattice_kernel_staged<3>
+    const auto kernel = at_most_per_sm(total_tiles, sms, kLatticeFew) ? engine_lattice_kernel_staged<0>
                                                                       : engine_lattice_kernel_staged<5>;
     kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);
   } else if (cascade == 2) engine_lattice_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a);

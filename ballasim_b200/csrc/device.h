@@ -172,7 +172,7 @@ int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
 // The split engine (stage kStageSplit). solo: the whole call in split_solo_kernel, up to `blocks` blocks. Else
 // split_begin_kernel, then per window split_window_kernel (blocks x
 // warps_per_block warps over the tiles) and split_rest_kernel (rest_blocks x 128 threads) over the pixels that the first
-// posted to `rest` (rest_capacity records of split_record_bytes(); rest_counts: a word per window, zero before the
+// posted to `rest` (rest_capacity records of split_record_bytes(); rest_counts: two words per window, zero before the
 // launch), and split_end_kernel. The state passes from S.in to S.out (carried_in to carried_out). tile0: the sensors'
 // first tiles (host memory); scratch: split_scratch_bytes(), 128-byte aligned.
 constexpr int kStageSplit = 1;

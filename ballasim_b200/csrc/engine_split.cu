@@ -74,6 +74,7 @@ struct RestList {
   RestRecord* rec;
   RestTimes* times;
   unsigned int* count;
+  unsigned int* taken;  // the records that warps have taken after their first ones
   unsigned int capacity;
 };
 
@@ -89,6 +90,8 @@ struct SplitArgs {
   uint32_t block_tiles;  // split_solo_kernel: the tiles of a block
   QuickPlanes q;
   SplitPixel* px;
+  uint16_t* lists;   // of a tile with pixels posted whole: its blob list (kMaxListed entries a tile) and
+  int32_t* list_n;   // that list's length (< 0: none)
   float4* boxes;  // this window's blob boxes (total_blobs), and the next one's (written by the rest kernel)
   float4* boxes_next;
   uint32_t tile0[kTile0Args];
@@ -494,10 +497,14 @@ __device__ __forceinline__ void window_tile(const SplitArgs& a, const RestList& 
     n_clean += n - 1u;
     a.q.c[slot] = last;
   }
-  // One record per posted pixel, the warp's records reserved together.
+  // One record per posted pixel, the warp's records reserved together; with a pixel posted whole, the tile's blob list.
   const bool post = have && !quiet;
   const unsigned posting = __ballot_sync(full, post);
   if (posting != 0u) {
+    if (__any_sync(full, post && !staged)) {
+      for (int i = static_cast<int>(lane); i < n_list; i += 32) a.lists[static_cast<size_t>(tile) * kMaxListed + i] = w.list[i];
+      if (lane == 0u) a.list_n[tile] = n_list;
+    }
     const int leader = __ffs(posting) - 1;
     unsigned int base = 0;
     if (static_cast<int>(lane) == leader) base = atomicAdd(rl.count, static_cast<unsigned int>(__popc(posting)));
@@ -589,21 +596,25 @@ __global__ void __launch_bounds__(128, 6) split_window_kernel(const __grid_const
   sums.add(a);
 }
 
-// A window posted whole (more samples than the stage holds), out of line: walked from its start with every blob of the
-// field evaluated (the same values as a culled list gives) and fed to the general pixel model. Returns the samples.
-__device__ __noinline__ uint32_t rest_whole(const SplitArgs* a, const EngineSensor* S, uint32_t pixel, int level,
-                                            int64_t t_w, PixelRegs* s, const PixelMapRegs* m, PixelCounters* c,
+// A window posted whole (more samples than the stage holds), out of line: walked from its start over the tile's blob
+// list (every blob where it has none) and fed to the general pixel model. Returns the samples. (Walked by the tile's own
+// warp in the window kernel instead, its 80 registers cost the other windows 9 %.)
+__device__ __noinline__ uint32_t rest_whole(const SplitArgs* a, const EngineSensor* S, uint32_t tile, uint32_t pixel,
+                                            int level, int64_t t_w, PixelRegs* s, const PixelMapRegs* m, PixelCounters* c,
                                             float* carried) {
   const FieldDev& f = S->field;
-  const BlobList all{nullptr, f.n_blobs};
+  const int32_t n_list = a->list_n[tile];
+  const BlobList list{n_list >= 0 ? a->lists + static_cast<size_t>(tile) * kMaxListed : nullptr,
+                      n_list >= 0 ? n_list : f.n_blobs};
   const uint32_t x = pixel % S->width, y = pixel / S->width;
   const ThreadSink sink{S->ev, &S->counters[kCntEvents]};
   PixelRegs sl = *s;
+  const PixelMapRegs ml = *m;
   PixelCounters cl = *c;
-  RegFeed<true, ThreadSink> feed{sl, *m, cl, S->consts, &S->consts, pixel, sink, t_w, t_w, sl.held, *carried, 0.0f};
+  RegFeed<true, ThreadSink> feed{sl, ml, cl, S->consts, &S->consts, pixel, sink, t_w, t_w, sl.held, *carried, 0.0f};
   feed.start(*carried);
   const uint32_t n = sample_pixel_window(a->r, level, *carried, false,
-                                         [&](uint32_t dt) { return field_eval(f, all, x, y, t_w + dt); }, feed);
+                                         [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); }, feed);
   sl.held = feed.prev_v;
   *carried = feed.last_raw;
   *s = sl;
@@ -816,7 +827,7 @@ __device__ __forceinline__ void rest_pixel(const SplitArgs& a, const RestList& r
     PixelMapRegs mt = m;
     PixelCounters ct = c;
     float rt = raw;
-    const uint32_t n = rest_whole(&a, &S, pixel, level, t_w, &st, &mt, &ct, &rt);
+    const uint32_t n = rest_whole(&a, &S, slot >> 5, pixel, level, t_w, &st, &mt, &ct, &rt);
     s = st;
     c = ct;
     raw = rt;
@@ -1064,8 +1075,11 @@ __device__ __forceinline__ void rest_pixel(const SplitArgs& a, const RestList& r
 }
 
 // The posted pixels of window a.w. Where the list is shorter than the launch, each warp takes fewer records (a power of
-// two of its lanes), since what one pixel does hardly ever falls together with what its neighbour does. 128 registers (4
-// blocks per SM): 5.90 ms of engine time on 346x260, 239 windows; 6.17 at 5 blocks, 6.58 at 6.
+// two of its lanes), since what one pixel does hardly ever falls together with what its neighbour does. A longer list's
+// warps take their next records as they get to them: a window past the stage can have a hundred times its neighbour's
+// samples (1280x720, 200 blobs of 400 px/s: 20.3 ms of engine time against 49.6 by a fixed stride, and 396 with every
+// blob evaluated for those windows instead of the tile's list). 128 registers (4 blocks per SM): 5.90 ms of engine time
+// on 346x260, 239 windows; 6.17 at 5 blocks, 6.58 at 6.
 __global__ void __launch_bounds__(128, 4) split_rest_kernel(const __grid_constant__ SplitArgs a, RestList rl) {
   const WindowTimes wt(a, a.w);
   if (a.w + 1 < a.windows) write_boxes(a, wt.t_w + kWindowNs, a.boxes_next);
@@ -1075,7 +1089,15 @@ __global__ void __launch_bounds__(128, 4) split_rest_kernel(const __grid_constan
   unsigned int share = 32u;
   while (share > 1u && static_cast<uint64_t>(share / 2u) * warps >= count) share /= 2u;
   if (lane >= share) return;
-  for (unsigned int i = warp * share + lane; i < count; i += warps * share) rest_pixel(a, rl, wt, i, lane);
+  const unsigned lanes = share == 32u ? 0xffffffffu : (1u << share) - 1u;
+  for (unsigned int first = warp * share; first < count;) {
+    if (first + lane < count) rest_pixel(a, rl, wt, first + lane, lane);
+    if (warps * share >= count) break;
+    __syncwarp(lanes);
+    unsigned int next = 0;
+    if (lane == 0u) next = atomicAdd(rl.taken, share);
+    first = warps * share + __shfl_sync(lanes, next, 0);
+  }
 }
 
 // The whole call in one launch, for few tiles: a block keeps its tiles through all windows, and each window's posted
@@ -1124,7 +1146,7 @@ __global__ void __launch_bounds__(128, 4) split_solo_kernel(const __grid_constan
 size_t split_scratch_bytes(uint32_t total_tiles, size_t total_blobs) {
   const size_t slots = static_cast<size_t>(total_tiles) * 32u;
   return slots * (sizeof(SplitPixel) + sizeof(float4) + sizeof(float2) + sizeof(float)) +
-         2u * total_blobs * sizeof(float4);
+         total_tiles * (kMaxListed * sizeof(uint16_t) + sizeof(int32_t)) + 2u * total_blobs * sizeof(float4);
 }
 size_t split_record_bytes() { return sizeof(RestRecord) + sizeof(RestTimes); }
 
@@ -1147,6 +1169,8 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   a.q.a = boxes + 2u * total_blobs;
   a.q.b = reinterpret_cast<float2*>(a.q.a + slots);
   a.q.c = reinterpret_cast<float*>(a.q.b + slots);
+  a.list_n = reinterpret_cast<int32_t*>(a.q.c + slots);
+  a.lists = reinterpret_cast<uint16_t*>(a.list_n + total_tiles);
   RestRecord* records = static_cast<RestRecord*>(rest);
   RestTimes* times = reinterpret_cast<RestTimes*>(records + rest_capacity);
   for (int i = 0; i < n_sensors && i < kTile0Args; ++i) a.tile0[i] = tile0[i];
@@ -1154,7 +1178,7 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
   if (solo) {
     const uint32_t most = static_cast<uint32_t>(blocks);
     a.block_tiles = (total_tiles + most - 1) / most;
-    const RestList rl{records, times, nullptr, rest_capacity};
+    const RestList rl{records, times, nullptr, nullptr, rest_capacity};
     split_solo_kernel<<<(total_tiles + a.block_tiles - 1) / a.block_tiles, warps_per_block * 32, 0, stream>>>(a, rl);
     return;
   }
@@ -1163,7 +1187,7 @@ void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0,
     a.w = w;
     a.boxes = boxes + (w & 1) * total_blobs;
     a.boxes_next = boxes + (1 - (w & 1)) * total_blobs;
-    const RestList rl{records, times, rest_counts + w, rest_capacity};
+    const RestList rl{records, times, rest_counts + 2 * w, rest_counts + 2 * w + 1, rest_capacity};
     split_window_kernel<<<blocks, warps_per_block * 32, 0, stream>>>(a, rl);
     split_rest_kernel<<<rest_blocks, 128, 0, stream>>>(a, rl);
   }

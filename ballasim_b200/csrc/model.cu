@@ -1796,7 +1796,7 @@ struct Engine {
     if (total_tiles > (1u << 26)) throw BudgetError("the split engine: too many pixels for its records");
     if (total_blobs > (size_t{1} << 31)) throw BudgetError("the split engine: too many blobs for its boxes");
     split.ensure((split_scratch_bytes(total_tiles, total_blobs) + sizeof(float4) - 1) / sizeof(float4),
-                 total_tiles * 32u, split_record_bytes(), static_cast<size_t>(std::max(windows, 1)),
+                 total_tiles * 32u, split_record_bytes(), 2 * static_cast<size_t>(std::max(windows, 1)),
                  [&] { release_graph(); });
   }
 
@@ -1832,7 +1832,7 @@ struct Engine {
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
                               rules, l, tile_counter.p, blocks, block_warps(), tile_lw, st);
       } else if (split_runs()) {
-        CK(cudaMemsetAsync(split.counts.p, 0, static_cast<size_t>(windows) * sizeof(unsigned int), st));
+        CK(cudaMemsetAsync(split.counts.p, 0, 2 * static_cast<size_t>(windows) * sizeof(unsigned int), st));
         const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());
         std::vector<uint32_t> tile0;
         for (const EngineSensor& e : host) tile0.push_back(e.tile0);

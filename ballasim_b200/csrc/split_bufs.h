@@ -1,5 +1,5 @@
 // The split engine's device buffers: its scratch (the pixel and quick records, the blob boxes), the posted-pixel list (a
-// record for every slot of the tiles) and a list count per window. Host code over any buffer type with a pointer p, a
+// record for every slot of the tiles) and the list's counts per window. Host code over any buffer type with a pointer p, a
 // capacity cap, ensure(n) (which frees the old allocation before it makes the new one, and throws where that fails) and
 // release(), so that the CPU tests run it over buffers that fail.
 #pragma once

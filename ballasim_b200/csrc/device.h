@@ -176,6 +176,7 @@ int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
 // launch), and split_end_kernel. The state passes from S.in to S.out (carried_in to carried_out). tile0: the sensors'
 // first tiles (host memory); scratch: split_scratch_bytes(), 128-byte aligned.
 constexpr int kStageSplit = 1;
+constexpr int kSplitStageLog2 = 4;  // log2 of the samples a pixel's window stages
 size_t split_scratch_bytes(uint32_t total_tiles, size_t total_blobs);
 size_t split_record_bytes();
 void launch_engine_split(const EngineSensor* sensors_dev, const uint32_t* tile0, int n_sensors, uint32_t total_tiles,

@@ -31,7 +31,7 @@ namespace bs {
 
 namespace {
 
-constexpr int kSplitStage = 16;       // samples after slot 0 that a posted pixel takes along (lattice level 4)
+constexpr int kSplitStage = 1 << kSplitStageLog2;  // samples after slot 0 that a posted pixel takes along
 constexpr uint32_t kRestWhole = 0xFF;  // the samples of a window that has more: walked again by the rest kernel
 constexpr int kCentres = 64;          // blobs a warp holds, and centres (one blob at two lattice slots) at a time
 constexpr int kTile0Args = 16;        // sensors whose first tiles travel as kernel arguments

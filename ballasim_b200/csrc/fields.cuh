@@ -164,6 +164,34 @@ BS_HD int32_t field_level(const FieldDev& f, const BlobList& l, uint32_t x, uint
   return level_of_speed(v, l_min, l_max);
 }
 
+// Whether the windows of a field are expected to hold at most 2^most_log2 samples by its motion: for a blob, the lattice
+// level of its speed and the halvings after which the chord over a step of its path deviates by no more than the sampler's
+// tolerance (step^2 / (8 r^2) of the value, a quarter of it per halving); an edge that crosses no more than its width
+// per step. Host side; parameters that are not numbers count as still.
+inline bool windows_expected_within(const FieldDev& f, const float* blobs_host, int32_t l_min, int32_t l_max, bool midpoint,
+                                    float tol, int32_t max_refine, int most_log2) {
+  if (l_min > most_log2) return false;
+  const auto step_of = [](float speed, int32_t level) {
+    return static_cast<double>(speed) * 1e-9 * static_cast<double>(kWindowNs >> level);
+  };
+  if (f.kind == kFieldTanhEdge) {
+    const double step = step_of(f.speed, l_min);
+    return !((step < 0 ? -step : step) > f.width_px) || !midpoint;
+  }
+  for (int32_t k = 0; k < f.n_blobs; ++k) {
+    const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
+    int32_t level = level_of_speed(b[8], l_min, l_max);
+    const double dx = step_of(b[3], level), dy = step_of(b[4], level);
+    double deviation = 0.25 * (dx * dx + dy * dy) * b[5];
+    for (int32_t i = 0; midpoint && i < max_refine && level <= most_log2 && deviation > tol; ++i) {
+      deviation *= 0.25;
+      ++level;
+    }
+    if (level > most_log2) return false;
+  }
+  return true;
+}
+
 #if defined(__CUDACC__)
 // Builds the calling warp's candidate list for [t_a, t_b] in `list` (kMaxListed entries of shared memory): blob k
 // is listed when its 6 r disc, swept from t_a to t_b, can reach the bounding box of the active lanes' pixel

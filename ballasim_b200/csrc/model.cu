@@ -1600,6 +1600,7 @@ struct Engine {
     if (cnt < 1) throw std::invalid_argument("engine: at least one sensor");
     if (cnt > 65535) throw std::invalid_argument("engine: at most 65535 sensors");
     rules = make_rules(r);
+    bool within = true;  // every sensor's windows are expected to fit the split engine's stage
     uint32_t tile0 = 0;
     for (int32_t i = 0; i < cnt; ++i) {
       Model* m = reinterpret_cast<Model*>(ms[i]);
@@ -1617,6 +1618,9 @@ struct Engine {
       auto f = std::make_unique<FieldHolder>();
       f->set(fs[i]);
       fields.push_back(std::move(f));
+      within = within && windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max,
+                                                 rules.midpoint != 0, rules.tol, rules.max_refine_levels,
+                                                 kSplitStageLog2);
       for (int b = 0; b < 2; ++b) {
         carried.push_back(std::make_unique<DevBuf<float>>());
         carried.back()->ensure(m->n);
@@ -1634,10 +1638,14 @@ struct Engine {
       host.push_back(e);
     }
     total_tiles = tile0;
-    // The launch shape until set_launch or the autotuner: the split engine for the instantaneous response. From the
-    // first frame on (64x48 to 640x480, 1 to 160 windows, with and without noise) it takes 0.24 to 0.93 of the streaming
-    // engine's time, and 0.37 of it on 1280x720.
-    if (cascade() == 0) {
+    // The launch shape until set_launch or the autotuner: the split engine for the instantaneous response, where the
+    // windows are expected to fit its stage or there are few tiles; else the streaming engine. Within the stage (64x48
+    // to 1280x720, 1 to 160 windows, blobs of 60 and 120 px/s, edges up to 120, tolerances 1e-2 and 1e-4, with and
+    // without noise) it takes 0.14 to 0.93 of the streaming engine's time. Past it (blobs of 300 to 2,000 px/s, or 60
+    // with a tolerance of 1e-5, 346x260 to 1280x720) 0.75 to 2.5, but up to two tiles a multiprocessor (97x61, 128x72)
+    // 0.6 to 0.98; with a lattice past the stage already 1.0 to 1.08 there and 1.3 to 1.7 on larger frames.
+    const bool few = total_tiles <= 2u * static_cast<uint32_t>(sm_count()) && rules.l_min <= kSplitStageLog2;
+    if (cascade() == 0 && (within || few)) {
       stage = kStageSplit;
       stage_chosen = false;
     }

@@ -1,4 +1,6 @@
 """An engine's launch shape: what launch reports is what set_launch takes, and the autotuner leaves the engine whole."""
+from dataclasses import replace
+
 import pytest
 
 from ballasim_b200 import fields as F
@@ -8,13 +10,12 @@ from ballasim_b200.params import resolve
 pytestmark = pytest.mark.gpu
 
 
-def engine(preset, rows, w=60, h=40):
+def engine(preset, rows, w=60, h=40, field=None, r=W.Rules()):
     from ballasim_b200.engine import Engine
     from ballasim_b200.sensor import SensorModel
 
-    r = W.Rules()
     m = SensorModel(resolve(preset, rows), w, h, 9, [{"type": "constant"}], 0)
-    eng = Engine([(m, F.blobs(w, h, 9, 5))], tol=r.tol, dark=r.dark, min_dt_ns=r.min_dt_ns,
+    eng = Engine([(m, field or F.blobs(w, h, 9, 5))], tol=r.tol, dark=r.dark, min_dt_ns=r.min_dt_ns,
                  max_refine_levels=r.max_refine_levels, l_min=r.l_min, l_max=r.l_max)
     return eng, m
 
@@ -60,3 +61,40 @@ def test_a_failed_autotune_leaves_the_shape(cuda_lib):
     with pytest.raises(RuntimeError):  # before start()
         eng.autotune(2)
     assert eng.launch == shape
+
+
+@pytest.mark.parametrize("size, field, rules, stage", [
+    ((346, 260), dict(), dict(), 1),
+    ((346, 260), dict(v_sigma=600.0), dict(), 0),  # levels past 4
+    ((346, 260), dict(v_sigma=600.0), dict(l_max=4), 1),  # 0.8 px a step: within the tolerance
+    ((346, 260), dict(v_sigma=600.0), dict(l_max=4, tol=1e-4), 0),
+    ((346, 260), dict(), dict(tol=1e-5), 0),  # refined past the stage
+    ((346, 260), dict(), dict(tol=1e-5, max_refine_levels=0), 1),
+    ((346, 260), dict(), dict(l_min=5), 0),
+    ((97, 61), dict(v_sigma=600.0), dict(), 1),  # few tiles
+    ((97, 61), dict(), dict(l_min=5), 0),
+])
+def test_the_stage_an_engine_starts_with(cuda_lib, size, field, rules, stage):
+    """The split engine where the windows are expected to fit its stage or the tiles are few, and the streaming engine's
+    events whichever it is."""
+    w, h = size
+    r = replace(W.Rules(), **rules)
+    f = F.blobs(w, h, 9, 12, **field)
+    got = []
+    for chosen in (None, 0):
+        eng, m = engine("ideal", {**W.MISMATCH, **W.NOISE}, w, h, f, r)
+        if chosen is None:
+            assert eng.launch["stage"] == stage
+        else:
+            eng.set_launch(stage=chosen)
+        eng.start(0)
+        got.append((eng.run(3), m.take_events(with_pixel=True), m.save_state()))
+    assert got[0][0] == got[1][0] and got[0][2] == got[1][2]
+    for k in got[0][1]:
+        assert got[0][1][k].tobytes() == got[1][1][k].tobytes(), k
+
+
+@pytest.mark.parametrize("speed, stage", [(40.0, 1), (-40.0, 1), (600.0, 0), (-600.0, 0)])
+def test_the_stage_of_an_edge(cuda_lib, speed, stage):
+    eng, _ = engine("ideal", W.MISMATCH, 346, 260, replace(F.tanh_edge(346, 260, 3), speed=speed))
+    assert eng.launch["stage"] == stage

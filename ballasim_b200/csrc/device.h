@@ -163,11 +163,11 @@ void launch_field_frame(const FieldDev& f, int64_t t, uint32_t n_pixels, float* 
 // counter (work stealing) by a persistent grid. stage 0: the sampler feeds the pixel model sample by sample;
 // 16 or 32: per window the samples are staged in shared memory (that many per lane) between the two phases.
 // t0: the model time in device memory; tiles of 2^tile_lw x 2^(5 - tile_lw) pixels (tile_lw in [2, 5]).
-// cascade: 0 the instantaneous response; 1 every sensor runs the cascade photoreceptor, 2 with its noise lattice
-// (streaming form; stage is ignored).
+// cascade: 0 the instantaneous response; 1 every sensor runs the cascade photoreceptor (in_step: the block's warps take
+// their sub-steps together, in a launch shape of its own; else they run freely), 2 with its noise lattice (stage 0 or 32).
 void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                    int32_t w0, int32_t w1, const SamplerRules& r, unsigned int* tile_counter, int blocks,
-                   int warps_per_block, int stage, int tile_lw, int cascade, cudaStream_t stream);
+                   int warps_per_block, int stage, int tile_lw, int cascade, bool in_step, cudaStream_t stream);
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade);
 // The split engine (stage kStageSplit). solo: the whole call in split_solo_kernel, up to `blocks` blocks. Else
 // split_begin_kernel, then per window split_window_kernel (blocks x

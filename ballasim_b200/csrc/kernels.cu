@@ -1193,6 +1193,71 @@ struct CascadeFeed {
   }
 };
 
+// The cascade with its warps running freely: tiles as they come, each lane's samples fed as they are walked. Where windows of
+// very different lengths stand side by side (blobs past the staged form's 16 samples) or every window is past them, a
+// block in step waits for its longest and walks such windows twice: 346x260, 40 blobs of 400 px/s 7.9 against 12.7 ms in
+// step, 640x480 with 90 of 1,500 px/s 37.7 against 56.3, a lattice of 128 samples 18.4 against 27.0. At most 128
+// registers (168 uncapped): on 346x260, 60 windows of 2 s, 36.6 against 38.2 ms per step, spills included.
+__global__ void __launch_bounds__(128, 4) engine_cascade_kernel_free(EngineArgs a) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const int64_t t0 = *a.t0;
+  for (;;) {
+    uint32_t tile = 0;
+    if (lane == 0) tile = atomicAdd(a.tile_counter, 1u);
+    tile = __shfl_sync(0xffffffffu, tile, 0);
+    if (tile >= a.total_tiles) break;
+    int si = 0;
+    while (si + 1 < a.n_sensors && a.sensors[si + 1].tile0 <= tile) ++si;
+    const EngineSensor& S = a.sensors[si];
+    const uint32_t local = tile - S.tile0;
+    uint32_t x, y;
+    tile_xy(local, S.tiles_x, a.tile_lw, lane, x, y);
+    const bool have = x < S.width && y < S.height;
+    const uint32_t p = have ? y * S.width + x : 0u;
+    PixelRegs s;
+    CascadeRegs q;
+    PixelMapRegs m;
+    float carried = 0.0f;
+    if (have) {
+      load_state(S.in, p, false, s);
+      load_cascade(S.in, p, q);
+      load_map(S.map, p, m);
+      carried = S.carried_in[p];
+    }
+    PixelCounters c;
+    CascadeCounters cn;
+    unsigned long long samples = 0;
+    GlobalSink sink{S.ev, &S.counters[kCntEvents]};
+    CascadeProc<GlobalSink> proc{s, q, m, S.consts, S.cc, p, sink, c, cn};
+    const FieldDev& f = S.field;
+    __shared__ uint16_t lists[4][kMaxListed];
+    uint16_t* my_list = lists[threadIdx.x >> 5];
+    for (int32_t w = a.w0; w < a.w1; ++w) {
+      const int64_t t_w = t0 + static_cast<int64_t>(w) * kWindowNs;
+      const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, my_list);
+      if (have) {
+        const int level = field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
+        CascadeFeed feed{&proc, t_w, S.consts.irr_max, t_w, s.held, carried};
+        feed.start(carried);
+        auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
+        samples += sample_pixel_window(a.r, level, carried, false, render, feed);
+        s.held = feed.prev_v;
+        carried = feed.last_raw;
+      }
+      __syncwarp();
+    }
+    if (have) {
+      store_state(S.out, p, false, s);
+      store_cascade(S.out, p, q);
+      S.carried_out[p] = carried;
+    }
+    warp_add(&S.counters[kCntPieces], c.pieces);
+    warp_add(&S.counters[kCntLeaves], c.leaves);
+    warp_add(&S.counters[kCntSamples], samples);
+    warp_add(&S.counters[kCntSubsteps], cn.substeps);
+  }
+}
+
 // The block's warps take one sub-step a turn together, a barrier between turns. A sub-step is some thousands of
 // instructions that run once (two stage-1 solves, logarithms, residual exponentials, the crossing search), more than the
 // instruction caches next to the schedulers hold: warps that drift apart each fetch it for themselves (10.7 of the 16
@@ -2435,9 +2500,11 @@ void launch_field_frame(const FieldDev& f, int64_t t, uint32_t n_pixels, float* 
 
 void launch_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                    int32_t w0, int32_t w1, const SamplerRules& r, unsigned int* tile_counter, int blocks,
-                   int warps_per_block, int stage, int tile_lw, int cascade, cudaStream_t stream) {
+                   int warps_per_block, int stage, int tile_lw, int cascade, bool in_step, cudaStream_t stream) {
   EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w0, w1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
-  if (cascade == 1) {
+  if (cascade == 1 && !in_step) {
+    engine_cascade_kernel_free<<<blocks, warps_per_block * 32, 0, stream>>>(a);
+  } else if (cascade == 1) {
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2470,8 +2537,8 @@ int rows_rest_blocks_per_sm() {
 
 int engine_max_blocks_per_sm(int warps_per_block, int stage, int cascade) {
   int n = 0;
-  if (cascade == 1) {
-    n = 1;  // launch_engine takes a shape of its own (step_shape)
+  if (cascade == 1) {  // in step launch_engine takes a shape of its own (step_shape)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_cascade_kernel_free, warps_per_block * 32, 0);
   } else if (cascade == 2 && stage != 0) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, engine_lattice_kernel_staged<5>, warps_per_block * 32, 0);
   } else if (cascade == 2) {

@@ -1590,6 +1590,7 @@ struct Engine {
   unsigned long long rec_n[2] = {0, 0};
   SplitBufs<DevBuf<float4>, DevBuf<unsigned char>, DevBuf<unsigned int>> split;  // stage kStageSplit's
   size_t total_blobs = 0;
+  bool within = true;  // every sensor's windows are expected to hold no more samples than the engines' stages (16)
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
   // 0 the instantaneous response, 1 the cascade, 2 the cascade with its noise lattice (every sensor alike).
@@ -1600,7 +1601,6 @@ struct Engine {
     if (cnt < 1) throw std::invalid_argument("engine: at least one sensor");
     if (cnt > 65535) throw std::invalid_argument("engine: at most 65535 sensors");
     rules = make_rules(r);
-    bool within = true;  // every sensor's windows are expected to fit the split engine's stage
     uint32_t tile0 = 0;
     for (int32_t i = 0; i < cnt; ++i) {
       Model* m = reinterpret_cast<Model*>(ms[i]);
@@ -1744,6 +1744,8 @@ struct Engine {
     total_tiles = tile0;
   }
 
+  // The cascade's warps go in step where their windows are alike (engine_cascade_kernel_free says why).
+  bool in_step() const { return cascade() == 1 && within; }
   int block_warps() const { return mlp ? 4 : warps_per_block; }
   // The stage that set_launch takes back: with a proposal the split engine is refused and no stage matters, so 0 stands
   // for it there.
@@ -1849,7 +1851,7 @@ struct Engine {
                             warps_per_block, tile_lw, rest_blocks, split_solo(), st);
       } else {
         launch_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows, rules,
-                      tile_counter.p, blocks, warps_per_block, stage, tile_lw, cascade(), st);
+                      tile_counter.p, blocks, warps_per_block, stage, tile_lw, cascade(), in_step(), st);
       }
     }
     CK(cudaGetLastError());
@@ -2028,10 +2030,10 @@ struct Engine {
 
   // Times each candidate launch shape on trial steps of `windows` windows from the current state (the models keep
   // their state) and keeps the fastest. Candidates: tile width 4, 8, 16 px (height 8, 4, 2) x warps per block 2, 4 x
-  // stage 0, 1 (split), 16, 64 (32 deep with the warp-cooperative search); the learned engine and the cascade, whose
-  // blocks have a shape of their own: tile widths only; the lattice: stage 0 or 32. A candidate whose buffers do not fit
-  // is left out; where none fits or a trial fails, the shape is what it was. Returns the candidates tried (ms of the
-  // second of two trial steps each); rows are {tile_lw, warps, stage, ms}.
+  // stage 0, 1 (split), 16, 64 (32 deep with the warp-cooperative search); the learned engine and the cascade in step,
+  // whose blocks have a shape of their own: tile widths only; the other cascade: stage 0; the lattice: 0 or 32. A
+  // candidate whose buffers do not fit is left out; where none fits or a trial fails, the shape is what it was. Returns
+  // the candidates tried (ms of the second of two trial steps each); rows are {tile_lw, warps, stage, ms}.
   std::vector<std::array<double, 4>> autotune(int32_t windows, cudaStream_t s) {
     if (windows < 1) throw std::invalid_argument("engine.autotune: windows >= 1");
     std::vector<std::array<double, 4>> rows;
@@ -2044,7 +2046,8 @@ struct Engine {
       for (int lw : {2, 3, 4}) {
         for (int w : {2, 4}) {
           for (int st : {0, kStageSplit, 16, 64}) {
-            if ((mlp || cascade() == 1) && (w != 4 || st != 0)) continue;
+            if ((mlp || in_step()) && (w != 4 || st != 0)) continue;
+            if (cascade() == 1 && st != 0) continue;
             if (cascade() == 2 && (st == 64 || st == kStageSplit)) continue;
             if (cascade() == 2 && st != 0) st = 32;
             set_launch(w, 0, st, lw);

@@ -198,9 +198,7 @@ struct LearnedLaunch {
 };
 void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                            int32_t w0, int32_t w1, const SamplerRules& r, const LearnedLaunch& l,
-                           unsigned int* tile_counter, int blocks, int warps_per_block, int tile_lw,
-                           cudaStream_t stream);
-int learned_engine_max_blocks_per_sm(int warps_per_block);
+                           unsigned int* tile_counter, int tile_lw, bool in_step, cudaStream_t stream);
 // Resets the walk state of n pixels from their initial irradiance.
 void launch_learned_reset(LearnedSoA st, uint32_t n, const float* irr0, cudaStream_t stream);
 

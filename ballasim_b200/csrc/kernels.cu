@@ -2150,6 +2150,119 @@ __global__ void learned_reset_kernel(LearnedSoA st, uint32_t n, const float* irr
   store_learned(st, p, n, L);
 }
 
+// The learned engine with its warps running freely, every sample fed to the pixel model as it is taken: where windows of
+// very different lengths stand side by side on many tiles. Per window and warp, as learned_engine_kernel below. 640x480,
+// 90 blobs of 400 px/s 11.0 against 15.0 ms in step, of 1,500 px/s 33.0 against 56.0 (learned_engine_kernel's stage and
+// quiet test with free warps 11.9 and 37.7). At most 64 registers (8 blocks per SM; 128 uncapped held it to 4): on the
+// 1280x720 held-out field 170.5 against 198.7 ms.
+__global__ void __launch_bounds__(128, 8) learned_engine_kernel_free(EngineArgs a, LearnedLaunch l) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const int64_t t0 = *a.t0;
+  __shared__ MlpShared W;
+  __shared__ __align__(16) uint16_t rows[4][32 * kSF];
+  __shared__ float ys[4][32];
+  __shared__ uint16_t lists[4][kMaxListed];
+  mlp_load_shared(W, l.ops, l.params);
+  uint16_t* my_list = lists[warp];
+  uint16_t* my_rows = rows[warp];
+  float* my_y = ys[warp];
+  const bool rec_s = l.rec_samples.capacity > 0, rec_p = l.rec_steps.capacity > 0;
+  for (;;) {
+    uint32_t tile = 0;
+    if (lane == 0) tile = atomicAdd(a.tile_counter, 1u);
+    tile = __shfl_sync(0xffffffffu, tile, 0);
+    if (tile >= a.total_tiles) break;
+    int si = 0;
+    while (si + 1 < a.n_sensors && a.sensors[si + 1].tile0 <= tile) ++si;
+    const EngineSensor& S = a.sensors[si];
+    const uint32_t local = tile - S.tile0;
+    uint32_t x, y;
+    tile_xy(local, S.tiles_x, a.tile_lw, lane, x, y);
+    const bool have = x < S.width && y < S.height;
+    const uint32_t np = S.width * S.height;
+    const uint32_t p = have ? y * S.width + x : 0u;
+    const uint32_t tag = (static_cast<uint32_t>(si) << 24) | p;
+    const bool noise = S.consts.noise != 0;
+    PixelRegs s;
+    PixelMapRegs m;
+    LearnedPixel L;
+    float carried = 0.0f;
+    if (have) {
+      load_state(S.in, p, noise, s);
+      load_map(S.map, p, m);
+      load_learned(S.lin, p, np, L);
+      carried = S.carried_in[p];
+    }
+    PixelCounters c;
+    unsigned long long samples = 0;
+    GlobalSink sink{S.ev, &S.counters[kCntEvents]};
+    PixelProc<GlobalSink> proc{s, m, S.consts, p, sink, c};
+    const FieldDev& f = S.field;
+    for (int32_t w = a.w0; w < a.w1; ++w) {
+      const int64_t t_w = t0 + static_cast<int64_t>(w) * kWindowNs;
+      const BlobList list = warp_blob_list(f, have, x, y, t_w, t_w + kWindowNs, my_list);
+      auto render = [&](uint32_t dt) { return field_eval(f, list, x, y, t_w + dt); };
+      WindowFeed feed{&proc, t_w, S.consts.irr_max, t_w, s.held, carried, 0.0f};
+      int s_floor = kWindowLog2;
+      uint32_t cur = 0;
+      float v_cur = carried, x_cur = 0.0f;
+      if (have) {
+        s_floor = kWindowLog2 - field_level(f, list, x, y, t_w, a.r.l_min, a.r.l_max);
+        feed.start(carried);
+        x_cur = log_f(carried);
+      }
+      auto emit = [&](uint32_t dt, float v) {
+        feed(dt, v);
+        if (rec_s) rec_push(l.rec_samples, t_w + dt, tag, v);
+      };
+      for (;;) {
+        const bool act = have && cur < static_cast<uint32_t>(kWindowNs);
+        if (!__any_sync(0xffffffffu, act)) break;
+        float feat[16];
+        if (act) {
+          step_features(L.hx, L.gaps, x_cur, feat);
+        } else {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) feat[k] = 0.0f;
+        }
+        uint32_t packed[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) packed[k] = pack2(feat[2 * k], feat[2 * k + 1]);
+        uint4* dst = reinterpret_cast<uint4*>(my_rows + lane * kSF);
+        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+        __syncwarp();
+        mlp_forward_warp(W, my_rows, my_y);
+        if (act) {
+          const int sl = proposal_log2(my_y[lane], l.margin, l.sh, s_floor, cur);
+          if (rec_p) rec_push(l.rec_steps, t_w + cur, tag, static_cast<float>(sl));
+          float v_end = 0.0f;
+          samples += learned_step(a.r, cur, sl, v_cur, x_cur, L, v_end, render, emit);
+          cur += 1u << sl;
+          v_cur = v_end;
+          x_cur = log_f(v_end);
+        }
+        __syncwarp();
+      }
+      if (have) {
+        ++samples;  // the carried slot, as in the plain engine's count
+        s.held = feed.prev_v;
+        carried = feed.last_raw;
+      }
+      __syncwarp();
+    }
+    if (have) {
+      store_state(S.out, p, noise, s);
+      store_learned(S.lout, p, np, L);
+      S.carried_out[p] = carried;
+    }
+    warp_add(&S.counters[kCntPieces], c.pieces);
+    warp_add(&S.counters[kCntLeaves], c.leaves);
+    warp_add(&S.counters[kCntSamples], samples);
+    warp_add(&S.counters[kCntNoise], c.noise_candidates);
+  }
+}
+
 // Samples of a window not yet taken by the pixel model (entry i at dt[32 i], v[32 i]), fed to it out of line, on copies:
 // few windows come here. pos: where the feed stands.
 constexpr uint32_t kLearnedStage = 8;
@@ -2561,26 +2674,25 @@ namespace bs {
 
 void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                            int32_t w0, int32_t w1, const SamplerRules& r, const LearnedLaunch& l,
-                           unsigned int* tile_counter, int blocks, int warps_per_block, int tile_lw,
-                           cudaStream_t stream) {
+                           unsigned int* tile_counter, int tile_lw, bool in_step, cudaStream_t stream) {
   EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w0, w1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
-  (void)warps_per_block;  // a shape of its own
-  (void)blocks;
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool alone = at_most_per_sm(total_tiles, sms, kLearnedApart);
+  if (!alone && !in_step) {
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, learned_engine_kernel_free, 128, 0);
+    const uint32_t blocks = std::min(static_cast<uint32_t>(sms * std::max(1, per_sm)), (total_tiles + 3u) / 4u);
+    learned_engine_kernel_free<<<blocks, 128, 0, stream>>>(a, l);
+    return;
+  }
   const StepShape c =
       alone ? StepShape{static_cast<int>(total_tiles), 1} : step_shape(total_tiles, sms, kLearnedWarps);
   const auto bytes = [](int warps) { return kMlpSharedBytes + warps * sizeof(LearnedWarpShared); };
   const auto kernel = alone ? learned_engine_kernel<1, kLearnedApart> : learned_engine_kernel<kLearnedWarps, 1>;
   if (!allow_shared(kernel, bytes(alone ? 1 : kLearnedWarps))) return;
   kernel<<<c.blocks, c.warps * 32, bytes(c.warps), stream>>>(a, l);
-}
-
-int learned_engine_max_blocks_per_sm(int warps_per_block) {
-  (void)warps_per_block;
-  return 1;  // launch_learned_engine takes a shape of its own (step_shape)
 }
 
 void launch_learned_reset(LearnedSoA st, uint32_t n, const float* irr0, cudaStream_t stream) {

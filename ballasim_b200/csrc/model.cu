@@ -1591,6 +1591,7 @@ struct Engine {
   SplitBufs<DevBuf<float4>, DevBuf<unsigned char>, DevBuf<unsigned int>> split;  // stage kStageSplit's
   size_t total_blobs = 0;
   bool within = true;  // every sensor's windows are expected to hold no more samples than the engines' stages (16)
+  bool alike = true;   // the same, or no more than every window's lattice has
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
   // 0 the instantaneous response, 1 the cascade, 2 the cascade with its noise lattice (every sensor alike).
@@ -1618,9 +1619,12 @@ struct Engine {
       auto f = std::make_unique<FieldHolder>();
       f->set(fs[i]);
       fields.push_back(std::move(f));
-      within = within && windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max,
-                                                 rules.midpoint != 0, rules.tol, rules.max_refine_levels,
-                                                 kSplitStageLog2);
+      const auto expected = [&](int most_log2) {
+        return windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max, rules.midpoint != 0,
+                                       rules.tol, rules.max_refine_levels, most_log2);
+      };
+      within = within && expected(kSplitStageLog2);
+      alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
       for (int b = 0; b < 2; ++b) {
         carried.push_back(std::make_unique<DevBuf<float>>());
         carried.back()->ensure(m->n);
@@ -1746,7 +1750,6 @@ struct Engine {
 
   // The cascade's warps go in step where their windows are alike (engine_cascade_kernel_free says why).
   bool in_step() const { return cascade() == 1 && within; }
-  int block_warps() const { return mlp ? 4 : warps_per_block; }
   // The stage that set_launch takes back: with a proposal the split engine is refused and no stage matters, so 0 stands
   // for it there.
   int reported_stage() const { return mlp && stage == kStageSplit ? 0 : stage; }
@@ -1760,15 +1763,15 @@ struct Engine {
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int wpb = block_warps();
+    const int wpb = warps_per_block;
+    if (mlp || in_step()) return 0;  // their launches have a shape of their own
     const int per_sm = blocks_per_sm > 0 ? blocks_per_sm
-                                         : std::max(1, mlp ? learned_engine_max_blocks_per_sm(wpb)
-                                                       : stage == kStageSplit
+                                         : std::max(1, stage == kStageSplit
                                                            ? (split_solo() ? split_solo_blocks_per_sm(wpb)
                                                                            : split_window_blocks_per_sm(wpb))
                                                            : engine_max_blocks_per_sm(wpb, stage, cascade()));
     // One tile per block is enough for the split engine in one launch (its block's warps share a tile's posted pixels).
-    const uint64_t needed = !mlp && stage == kStageSplit && split_solo() ? total_tiles : (total_tiles + wpb - 1) / wpb;
+    const uint64_t needed = stage == kStageSplit && split_solo() ? total_tiles : (total_tiles + wpb - 1) / wpb;
     return static_cast<int>(std::min<uint64_t>(static_cast<uint64_t>(sms) * per_sm, needed));
   }
 
@@ -1840,7 +1843,7 @@ struct Engine {
         const LearnedLaunch l{mlp->ops.p, mlp->params.p, margin, sh,
                               RecBuf{rec[0].p, rec_count.p, rec_cap}, RecBuf{rec[1].p, rec_count.p + 1, rec_cap}};
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
-                              rules, l, tile_counter.p, blocks, block_warps(), tile_lw, st);
+                              rules, l, tile_counter.p, tile_lw, alike, st);
       } else if (split_runs()) {
         CK(cudaMemsetAsync(split.counts.p, 0, 2 * static_cast<size_t>(windows) * sizeof(unsigned int), st));
         const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());
@@ -1889,7 +1892,7 @@ struct Engine {
       describe(t0);
       if (use_graph && rec_cap == 0) {
         const uint64_t key[8] = {static_cast<uint64_t>(windows), static_cast<uint64_t>(blocks),
-                                 static_cast<uint64_t>(block_warps()), static_cast<uint64_t>(stage),
+                                 static_cast<uint64_t>(warps_per_block), static_cast<uint64_t>(stage),
                                  static_cast<uint64_t>(tile_lw), reinterpret_cast<uint64_t>(mlp),
                                  (static_cast<uint64_t>(f2u(margin)) << 32) | total_tiles, 1};
         if (!exec || std::memcmp(key, graph_key, sizeof(key)) != 0) {

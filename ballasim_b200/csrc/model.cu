@@ -1602,6 +1602,8 @@ struct Engine {
     if (cnt < 1) throw std::invalid_argument("engine: at least one sensor");
     if (cnt > 65535) throw std::invalid_argument("engine: at most 65535 sensors");
     rules = make_rules(r);
+    bool lattice_within = true;  // every sensor's lattice is expected to hold at most half the samples that the staged
+                                 // form has room for (32: the other half for refinement)
     uint32_t tile0 = 0;
     for (int32_t i = 0; i < cnt; ++i) {
       Model* m = reinterpret_cast<Model*>(ms[i]);
@@ -1625,6 +1627,8 @@ struct Engine {
       };
       within = within && expected(kSplitStageLog2);
       alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
+      lattice_within = lattice_within && windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max,
+                                                                 false, 0.0f, 0, 4);
       for (int b = 0; b < 2; ++b) {
         carried.push_back(std::make_unique<DevBuf<float>>());
         carried.back()->ensure(m->n);
@@ -1653,8 +1657,10 @@ struct Engine {
       stage = kStageSplit;
       stage_chosen = false;
     }
-    // The lattice's staged form: 87.9 against 102.1 ms streaming on 346x260, 8 windows.
-    if (cascade() == 2) stage = 32;
+    // The lattice's staged form: 89.0 against 102 ms streaming on 346x260, 8 windows, and 0.6 to 0.7 of it under a
+    // tolerance of 1e-5; with motion past its stage (blobs of 400 px/s) 54.7 against 42.5 there and 92.8 against 75 on
+    // 640x480, with a lattice of 32 samples 1.03 times the streaming form's time, so those stream.
+    if (cascade() == 2 && lattice_within) stage = 32;
     retile();
     sensors_dev.ensure(host.size());
     tile_counter.ensure(1);

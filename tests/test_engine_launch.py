@@ -98,3 +98,12 @@ def test_the_stage_an_engine_starts_with(cuda_lib, size, field, rules, stage):
 def test_the_stage_of_an_edge(cuda_lib, speed, stage):
     eng, _ = engine("ideal", W.MISMATCH, 346, 260, replace(F.tanh_edge(346, 260, 3), speed=speed))
     assert eng.launch["stage"] == stage
+
+
+@pytest.mark.parametrize("field, rules, stage", [
+    (dict(), dict(), 32), (dict(), dict(tol=1e-5), 32), (dict(), dict(l_min=4), 32), (dict(), dict(l_min=5), 0),
+    (dict(v_sigma=1500.0), dict(), 0), (dict(v_sigma=1500.0), dict(l_max=4), 32),
+])
+def test_the_stage_of_the_lattice(cuda_lib, field, rules, stage):
+    eng, _ = engine("prophesee_gen3", W.MISMATCH, 60, 40, F.blobs(60, 40, 9, 5, **field), replace(W.Rules(), **rules))
+    assert eng.launch["stage"] == stage

@@ -10,6 +10,8 @@ namespace bs {
 
 namespace cg = cooperative_groups;
 
+namespace {  // each including file's own: the compiler fits an internal function's calls to it
+
 // Appends events to one sensor's buffer; the lanes of a warp that push together share one atomic, so every lane of
 // the warp must push to the same buffer (a warp works on one tile of one sensor).
 struct GlobalSink {
@@ -475,5 +477,7 @@ __device__ __forceinline__ void skip_rejected(const SensorConsts& k, uint32_t pi
     t = noise_after(w, t, rate_hz);
   }
 }
+
+}  // namespace
 
 }  // namespace bs

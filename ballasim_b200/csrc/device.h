@@ -196,9 +196,12 @@ struct LearnedLaunch {
   int32_t sh;  // log2 min_dt_ns
   RecBuf rec_samples, rec_steps;
 };
+// How its warps run: in step on many tiles and one to a block on few; freely on many and one to a block on few (windows of
+// very different lengths side by side); freely always (windows whose lanes' lengths differ as much).
+enum class LearnedForm { kInStep, kApartOrFree, kFree };
 void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                            int32_t w0, int32_t w1, const SamplerRules& r, const LearnedLaunch& l,
-                           unsigned int* tile_counter, int tile_lw, bool in_step, cudaStream_t stream);
+                           unsigned int* tile_counter, int tile_lw, LearnedForm form, cudaStream_t stream);
 // Resets the walk state of n pixels from their initial irradiance.
 void launch_learned_reset(LearnedSoA st, uint32_t n, const float* irr0, cudaStream_t stream);
 

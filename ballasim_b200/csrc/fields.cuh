@@ -164,32 +164,43 @@ BS_HD int32_t field_level(const FieldDev& f, const BlobList& l, uint32_t x, uint
   return level_of_speed(v, l_min, l_max);
 }
 
+// The lattice level at which the chord over a step deviates by no more than the sampler's tolerance: a quarter of
+// `deviation` (at `level`) per halving, at most max_refine of them; past most_log2 only that it is.
+inline int32_t refined_level(int32_t level, double deviation, float tol, int32_t max_refine, int most_log2) {
+  for (int32_t i = 0; i < max_refine && level <= most_log2 && deviation > tol; ++i) {
+    deviation *= 0.25;
+    ++level;
+  }
+  return level;
+}
+// A speed's way in a step of the lattice, px.
+inline double lattice_step(float speed, int32_t level) {
+  return static_cast<double>(speed) * 1e-9 * static_cast<double>(kWindowNs >> level);
+}
 // Whether the windows of a field are expected to hold at most 2^most_log2 samples by its motion: for a blob, the lattice
-// level of its speed and the halvings after which the chord over a step of its path deviates by no more than the sampler's
-// tolerance (step^2 / (8 r^2) of the value, a quarter of it per halving); an edge that crosses no more than its width
-// per step. Host side; parameters that are not numbers count as still.
+// level of its speed refined to the tolerance (the chord deviates by step^2 / (8 r^2) of the value); an edge that crosses
+// no more than its width per step (its refined windows are few whatever the tolerance). Host side; parameters that are
+// not numbers count as still.
 inline bool windows_expected_within(const FieldDev& f, const float* blobs_host, int32_t l_min, int32_t l_max, bool midpoint,
                                     float tol, int32_t max_refine, int most_log2) {
   if (l_min > most_log2) return false;
-  const auto step_of = [](float speed, int32_t level) {
-    return static_cast<double>(speed) * 1e-9 * static_cast<double>(kWindowNs >> level);
-  };
   if (f.kind == kFieldTanhEdge) {
-    const double step = step_of(f.speed, l_min);
+    const double step = lattice_step(f.speed, l_min);
     return !((step < 0 ? -step : step) > f.width_px) || !midpoint;
   }
   for (int32_t k = 0; k < f.n_blobs; ++k) {
     const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
-    int32_t level = level_of_speed(b[8], l_min, l_max);
-    const double dx = step_of(b[3], level), dy = step_of(b[4], level);
-    double deviation = 0.25 * (dx * dx + dy * dy) * b[5];
-    for (int32_t i = 0; midpoint && i < max_refine && level <= most_log2 && deviation > tol; ++i) {
-      deviation *= 0.25;
-      ++level;
-    }
-    if (level > most_log2) return false;
+    const int32_t level = level_of_speed(b[8], l_min, l_max);
+    const double dx = lattice_step(b[3], level), dy = lattice_step(b[4], level);
+    const double deviation = 0.25 * (dx * dx + dy * dy) * b[5];
+    if (refined_level(level, deviation, tol, midpoint ? max_refine : 0, most_log2) > most_log2) return false;
   }
   return true;
+}
+// The same for the windows at an edge, refined to the tolerance (step^2 / (8 width^2)).
+inline bool edge_expected_within(const FieldDev& f, int32_t l_min, float tol, int32_t max_refine, int most_log2) {
+  const double step = lattice_step(f.speed, l_min) / f.width_px;
+  return refined_level(l_min, 0.125 * step * step, tol, max_refine, most_log2) <= most_log2;
 }
 
 #if defined(__CUDACC__)

@@ -1276,13 +1276,26 @@ struct CascadeWarpShared {
   float v[kCascadeStage][32];
 };
 
+// The next tiles of a block in step, as many as it has warps, after its first ones (blockIdx.x's): the blocks take them as
+// they get to them: heavy tiles can come back every so many (a fixed stride of 148 groups of 20 met the same blocks with
+// a 640x480 frame's edge in every row of tiles: 1.01 ms of the cascade's time, 0.80 so). All of its threads call it.
+__device__ __forceinline__ uint32_t next_tiles(const EngineArgs& a, uint32_t warps) {
+  const uint32_t firsts = gridDim.x * warps;
+  if (firsts >= a.total_tiles) return a.total_tiles;
+  __shared__ uint32_t next;
+  __syncthreads();
+  if (threadIdx.x == 0u) next = firsts + atomicAdd(a.tile_counter, warps);
+  __syncthreads();
+  return next;
+}
+
 template <int kWarps, int kBlocks>
 __global__ void __launch_bounds__(32 * kWarps, kBlocks) engine_cascade_kernel(EngineArgs a) {
   extern __shared__ CascadeWarpShared cascade_shared[];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   CascadeWarpShared& sh = cascade_shared[warp];
   const int64_t t0 = *a.t0;
-  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first += gridDim.x * warps) {
+  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first = next_tiles(a, warps)) {
     const uint32_t tile = first + warp < a.total_tiles ? first + warp : a.total_tiles - 1u;
     const bool real = first + warp < a.total_tiles;  // a warp past the last tile only keeps the barriers
     int si = 0;
@@ -2315,7 +2328,7 @@ __global__ void __launch_bounds__(32 * kWarps, kBlocks) learned_engine_kernel(En
   float* my_y = sh.y;
   const bool rec_s = l.rec_samples.capacity > 0, rec_p = l.rec_steps.capacity > 0;
   const uint32_t warps = blockDim.x >> 5;
-  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first += gridDim.x * warps) {
+  for (uint32_t first = blockIdx.x * warps; first < a.total_tiles; first = next_tiles(a, warps)) {
     const uint32_t tile = first + warp < a.total_tiles ? first + warp : a.total_tiles - 1u;
     const bool real = first + warp < a.total_tiles;  // a warp past the last tile only keeps the barriers
     int si = 0;
@@ -2674,13 +2687,13 @@ namespace bs {
 
 void launch_learned_engine(const EngineSensor* sensors_dev, int n_sensors, uint32_t total_tiles, const int64_t* t0,
                            int32_t w0, int32_t w1, const SamplerRules& r, const LearnedLaunch& l,
-                           unsigned int* tile_counter, int tile_lw, bool in_step, cudaStream_t stream) {
+                           unsigned int* tile_counter, int tile_lw, LearnedForm form, cudaStream_t stream) {
   EngineArgs a{sensors_dev, n_sensors, total_tiles, t0, w0, w1, r, tile_counter, static_cast<uint32_t>(tile_lw)};
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool alone = at_most_per_sm(total_tiles, sms, kLearnedApart);
-  if (!alone && !in_step) {
+  if (form == LearnedForm::kFree || (!alone && form != LearnedForm::kInStep)) {
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, learned_engine_kernel_free, 128, 0);
     const uint32_t blocks = std::min(static_cast<uint32_t>(sms * std::max(1, per_sm)), (total_tiles + 3u) / 4u);

@@ -1592,6 +1592,7 @@ struct Engine {
   size_t total_blobs = 0;
   bool within = true;  // every sensor's windows are expected to hold no more samples than the engines' stages (16)
   bool alike = true;   // the same, or no more than every window's lattice has
+  bool any_edge = false, fine_edge = false;  // an edge; one that the tolerance is expected to refine past the stages
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
   // 0 the instantaneous response, 1 the cascade, 2 the cascade with its noise lattice (every sensor alike).
@@ -1627,6 +1628,10 @@ struct Engine {
       };
       within = within && expected(kSplitStageLog2);
       alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
+      any_edge = any_edge || fs[i].kind == kFieldTanhEdge;
+      fine_edge = fine_edge || (fs[i].kind == kFieldTanhEdge && rules.midpoint != 0 &&
+                                !edge_expected_within(fields.back()->f, rules.l_min, rules.tol, rules.max_refine_levels,
+                                                      kSplitStageLog2));
       lattice_within = lattice_within && windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max,
                                                                  false, 0.0f, 0, 4);
       for (int b = 0; b < 2; ++b) {
@@ -1754,8 +1759,15 @@ struct Engine {
     total_tiles = tile0;
   }
 
-  // The cascade's warps go in step where their windows are alike (engine_cascade_kernel_free says why).
-  bool in_step() const { return cascade() == 1 && within; }
+  // The cascade's warps go in step where their windows are alike (engine_cascade_kernel_free says why). An edge leaves most
+  // tiles still: in step up to a round of tiles (20 a multiprocessor; 346x260 0.48 to 1.04 times the free form's time over
+  // 40 and 120 px/s and tolerances of 1e-2 to 1e-6; 640x480 0.55 to 1.52, 1280x720 0.84 to 2.04).
+  bool in_step() const {
+    return cascade() == 1 && within && (!any_edge || total_tiles <= 20u * static_cast<uint32_t>(sm_count()));
+  }
+  LearnedForm learned_form() const {
+    return fine_edge ? LearnedForm::kFree : alike ? LearnedForm::kInStep : LearnedForm::kApartOrFree;
+  }
   // The stage that set_launch takes back: with a proposal the split engine is refused and no stage matters, so 0 stands
   // for it there.
   int reported_stage() const { return mlp && stage == kStageSplit ? 0 : stage; }
@@ -1849,7 +1861,7 @@ struct Engine {
         const LearnedLaunch l{mlp->ops.p, mlp->params.p, margin, sh,
                               RecBuf{rec[0].p, rec_count.p, rec_cap}, RecBuf{rec[1].p, rec_count.p + 1, rec_cap}};
         launch_learned_engine(sensors_dev.p, static_cast<int>(host.size()), total_tiles, t0_dev.p, 0, windows,
-                              rules, l, tile_counter.p, tile_lw, alike, st);
+                              rules, l, tile_counter.p, tile_lw, learned_form(), st);
       } else if (split_runs()) {
         CK(cudaMemsetAsync(split.counts.p, 0, 2 * static_cast<size_t>(windows) * sizeof(unsigned int), st));
         const int rest_blocks = sm_count() * std::max(1, split_rest_blocks_per_sm());

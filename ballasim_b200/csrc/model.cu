@@ -1628,12 +1628,14 @@ struct Engine {
       };
       within = within && expected(kSplitStageLog2);
       alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
-      any_edge = any_edge || fs[i].kind == kFieldTanhEdge;
-      fine_edge = fine_edge || (fs[i].kind == kFieldTanhEdge && rules.midpoint != 0 &&
+      const bool edge = fs[i].kind == kFieldTanhEdge;
+      any_edge = any_edge || edge;
+      fine_edge = fine_edge || (edge && rules.midpoint != 0 &&
                                 !edge_expected_within(fields.back()->f, rules.l_min, rules.tol, rules.max_refine_levels,
                                                       kSplitStageLog2));
-      lattice_within = lattice_within && windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min, rules.l_max,
-                                                                 false, 0.0f, 0, 4);
+      lattice_within = lattice_within && (edge ? within && !fine_edge
+                                               : windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min,
+                                                                         rules.l_max, false, 0.0f, 0, 4));
       for (int b = 0; b < 2; ++b) {
         carried.push_back(std::make_unique<DevBuf<float>>());
         carried.back()->ensure(m->n);
@@ -1664,7 +1666,8 @@ struct Engine {
     }
     // The lattice's staged form: 89.0 against 102 ms streaming on 346x260, 8 windows, and 0.6 to 0.7 of it under a
     // tolerance of 1e-5; with motion past its stage (blobs of 400 px/s) 54.7 against 42.5 there and 92.8 against 75 on
-    // 640x480, with a lattice of 32 samples 1.03 times the streaming form's time, so those stream.
+    // 640x480, with a lattice of 32 samples 1.03 times the streaming form's time, an edge of 2,000 px/s or 1e-6 up to 1.17
+    // times, so those stream.
     if (cascade() == 2 && lattice_within) stage = 32;
     retile();
     sensors_dev.ensure(host.size());

@@ -107,3 +107,10 @@ def test_the_stage_of_an_edge(cuda_lib, speed, stage):
 def test_the_stage_of_the_lattice(cuda_lib, field, rules, stage):
     eng, _ = engine("prophesee_gen3", W.MISMATCH, 60, 40, F.blobs(60, 40, 9, 5, **field), replace(W.Rules(), **rules))
     assert eng.launch["stage"] == stage
+
+
+@pytest.mark.parametrize("speed, tol, stage", [(40.0, 1e-2, 32), (40.0, 1e-4, 32), (40.0, 1e-6, 0), (2000.0, 1e-2, 0)])
+def test_the_stage_of_the_lattice_at_an_edge(cuda_lib, speed, tol, stage):
+    eng, _ = engine("prophesee_gen3", W.MISMATCH, 60, 40, replace(F.tanh_edge(60, 40, 3), speed=speed),
+                    replace(W.Rules(), tol=tol))
+    assert eng.launch["stage"] == stage

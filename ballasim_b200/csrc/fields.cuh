@@ -177,10 +177,23 @@ inline int32_t refined_level(int32_t level, double deviation, float tol, int32_t
 inline double lattice_step(float speed, int32_t level) {
   return static_cast<double>(speed) * 1e-9 * static_cast<double>(kWindowNs >> level);
 }
-// Whether the windows of a field are expected to hold at most 2^most_log2 samples by its motion: for a blob, the lattice
-// level of its speed refined to the tolerance (the chord deviates by step^2 / (8 r^2) of the value); an edge that crosses
-// no more than its width per step (its refined windows are few whatever the tolerance). Host side; parameters that are
-// not numbers count as still.
+// How many of a field's blobs are expected to take some window past 2^most_log2 samples by their motion: the lattice level
+// of their speed refined to the tolerance (the chord deviates by step^2 / (8 r^2) of the value). Host side; parameters that
+// are not numbers count as still.
+inline int32_t blobs_expected_past(const FieldDev& f, const float* blobs_host, int32_t l_min, int32_t l_max, bool midpoint,
+                                   float tol, int32_t max_refine, int most_log2) {
+  int32_t past = 0;
+  for (int32_t k = 0; k < f.n_blobs; ++k) {
+    const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
+    const int32_t level = level_of_speed(b[8], l_min, l_max);
+    const double dx = lattice_step(b[3], level), dy = lattice_step(b[4], level);
+    const double deviation = 0.25 * (dx * dx + dy * dy) * b[5];
+    if (refined_level(level, deviation, tol, midpoint ? max_refine : 0, most_log2) > most_log2) ++past;
+  }
+  return past;
+}
+// Whether the windows of a field are expected to hold at most 2^most_log2 samples: no such blob, or an edge that crosses
+// no more than its width per step (its refined windows are few whatever the tolerance).
 inline bool windows_expected_within(const FieldDev& f, const float* blobs_host, int32_t l_min, int32_t l_max, bool midpoint,
                                     float tol, int32_t max_refine, int most_log2) {
   if (l_min > most_log2) return false;
@@ -188,14 +201,7 @@ inline bool windows_expected_within(const FieldDev& f, const float* blobs_host, 
     const double step = lattice_step(f.speed, l_min);
     return !((step < 0 ? -step : step) > f.width_px) || !midpoint;
   }
-  for (int32_t k = 0; k < f.n_blobs; ++k) {
-    const float* b = blobs_host + static_cast<size_t>(k) * kBlobWords;
-    const int32_t level = level_of_speed(b[8], l_min, l_max);
-    const double dx = lattice_step(b[3], level), dy = lattice_step(b[4], level);
-    const double deviation = 0.25 * (dx * dx + dy * dy) * b[5];
-    if (refined_level(level, deviation, tol, midpoint ? max_refine : 0, most_log2) > most_log2) return false;
-  }
-  return true;
+  return blobs_expected_past(f, blobs_host, l_min, l_max, midpoint, tol, max_refine, most_log2) == 0;
 }
 // The same for the windows at an edge, refined to the tolerance (step^2 / (8 width^2)).
 inline bool edge_expected_within(const FieldDev& f, int32_t l_min, float tol, int32_t max_refine, int most_log2) {

@@ -1592,6 +1592,7 @@ struct Engine {
   size_t total_blobs = 0;
   bool within = true;  // every sensor's windows are expected to hold no more samples than the engines' stages (16)
   bool alike = true;   // the same, or no more than every window's lattice has
+  bool mostly_short = true;  // at most a quarter of any sensor's blobs past half of that (or past every window's lattice)
   bool any_edge = false, fine_edge = false;  // an edge; one that the tolerance is expected to refine past the stages
 
   static int32_t models_cascade(bs_model* m) { return m ? reinterpret_cast<Model*>(m)->mode() : 0; }
@@ -1629,13 +1630,18 @@ struct Engine {
       within = within && expected(kSplitStageLog2);
       alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
       const bool edge = fs[i].kind == kFieldTanhEdge;
+      const FieldDev& fd = fields.back()->f;
+      mostly_short = mostly_short && 4 * static_cast<int64_t>(blobs_expected_past(
+                                             fd, fs[i].blobs, rules.l_min, rules.l_max, rules.midpoint != 0, rules.tol,
+                                             rules.max_refine_levels, std::max(kSplitStageLog2 - 1, rules.l_min))) <=
+                                         fd.n_blobs;
       any_edge = any_edge || edge;
       fine_edge = fine_edge || (edge && rules.midpoint != 0 &&
-                                !edge_expected_within(fields.back()->f, rules.l_min, rules.tol, rules.max_refine_levels,
+                                !edge_expected_within(fd, rules.l_min, rules.tol, rules.max_refine_levels,
                                                       kSplitStageLog2));
       lattice_within = lattice_within && (edge ? within && !fine_edge
-                                               : windows_expected_within(fields.back()->f, fs[i].blobs, rules.l_min,
-                                                                         rules.l_max, false, 0.0f, 0, 4));
+                                               : windows_expected_within(fd, fs[i].blobs, rules.l_min, rules.l_max,
+                                                                         false, 0.0f, 0, kSplitStageLog2));
       for (int b = 0; b < 2; ++b) {
         carried.push_back(std::make_unique<DevBuf<float>>());
         carried.back()->ensure(m->n);
@@ -1764,9 +1770,11 @@ struct Engine {
 
   // The cascade's warps go in step where their windows are alike (engine_cascade_kernel_free says why). An edge leaves most
   // tiles still: in step up to a round of tiles (20 a multiprocessor; 346x260 0.48 to 1.04 times the free form's time over
-  // 40 and 120 px/s and tolerances of 1e-2 to 1e-6; 640x480 0.55 to 1.52, 1280x720 0.84 to 2.04).
+  // 40 and 120 px/s and tolerances of 1e-2 to 1e-6; 640x480 0.55 to 1.52, 1280x720 0.84 to 2.04). Blobs past half the
+  // stage beside slow ones do not pay either (160x120, speeds of 200 px/s, half of them past it: 1.10; of 120 px/s, a
+  // seventh: 0.94).
   bool in_step() const {
-    return cascade() == 1 && within && (!any_edge || total_tiles <= 20u * static_cast<uint32_t>(sm_count()));
+    return cascade() == 1 && within && mostly_short && (!any_edge || total_tiles <= 20u * static_cast<uint32_t>(sm_count()));
   }
   LearnedForm learned_form() const {
     return fine_edge ? LearnedForm::kFree : alike ? LearnedForm::kInStep : LearnedForm::kApartOrFree;

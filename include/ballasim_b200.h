@@ -343,28 +343,34 @@ bs_status bs_engine_run(bs_engine* e, int32_t windows, void* stream, uint64_t* p
  * sensor's copies into the caller's arrays run while the device works on the sensors after it. No counterpart in the
  * reference, whose engine takes one camera's events at a time; the columns and the order are bs_model_take_events'. */
 bs_status bs_engine_take_events(bs_engine* e, bs_event_columns* out);
-/* Launch shape: warps per block and blocks per SM of the persistent grid (0: the defaults, 4 and as many as fit),
- * the staging depth (0: the sampler feeds the pixel model sample by sample; 16 or 32: per window each lane's samples
- * are staged in shared memory between a sampling phase and a sensing phase; 64: staged 32 deep with the crossing
- * search taken by the whole warp; 1: the split engine, two launches per window, the first running the staged phases
- * and the pixel model's clean segments for every pixel and posting each pixel at its first other segment, the second
- * finishing the posted pixels' windows one thread per pixel, or one launch per call for few pixels; the instantaneous
- * response only, and the stage an engine of such sensors starts with; an engine with the noise lattice starts with 32)
- * and the tile width in
- * pixels (4, 8, 16 or 32; the tile is 32 / width pixels high, one warp per tile; 0: 8). The learned engine and the
- * cascade without the lattice run one block per SM with as many warps as their tiles need. */
+/* Launch shape: warps per block and blocks per SM of the persistent grid (0: the defaults, 4 and as many as fit), the
+ * stage and the tile width in pixels (4, 8, 16 or 32; the tile is 32 / width pixels high, one warp per tile; 0: 8).
+ * Stages: 0, the sampler feeds the pixel model sample by sample; 16 or 32, per window each lane's samples are staged in
+ * shared memory between a sampling phase and a sensing phase; 64, staged 32 deep with the crossing search taken by the
+ * whole warp; 1, the split engine: per window one launch samples every pixel and keeps those that two bounds show to
+ * fire nothing, and a second one runs the others, whole windows, through the pixel model, one thread per pixel (few
+ * pixels: the whole call in one launch). 64 and 1 are the instantaneous response's; the cascade takes 0, its noise
+ * lattice 0 or 32, and with a learned proposal the stage has no effect (1 and 64 are refused).
+ * An engine starts with 1 (instantaneous response) or 32 (lattice) where its fields' motion is expected to leave a
+ * pixel's window within 16 samples, or with 1 on few tiles, else with 0; where the split engine's records (about 300
+ * bytes a pixel) do not fit, it changes from 1 to 0.
+ * The learned engine, and the cascade without the lattice where such windows are expected, run in a shape of their own:
+ * one block per SM with as many warps as their tiles need, or on few tiles one warp per block. Warps per block and blocks
+ * per SM have no effect on them, though get_launch reports them. */
 bs_status bs_engine_set_launch(bs_engine* e, int32_t warps_per_block, int32_t blocks_per_sm, int32_t stage,
                                int32_t tile_width);
-/* The current launch shape: warps per block, blocks per SM, staging depth, tile width. */
+/* The current launch shape, as set_launch takes it: warps per block, blocks per SM, stage (0 for 1 while a proposal is
+ * set), tile width. */
 bs_status bs_engine_get_launch(const bs_engine* e, int32_t out[4]);
 /* Runs each step as a CUDA graph (on, the default) or as separate stream operations (off). The graph holds the
- * counter resets, the descriptor and model-time uploads, the persistent kernel and the counter read-back; it is
- * rebuilt when the window count, launch shape or proposal changes. */
+ * counter resets, the descriptor and model-time uploads, the engine's kernels and the counter read-back; it is
+ * rebuilt when the window count, launch shape or proposal changes, or a buffer that it holds moves. */
 bs_status bs_engine_set_graph(bs_engine* e, int32_t on);
 /* The autotuner: times trial steps of `windows` windows from the current state for each candidate launch shape
- * (tile width 4, 8, 16 x warps per block 2, 4 x stage 0, 1, 16, 64; the learned engine: tile widths) without
- * moving the models, and keeps the fastest. rows (cap x 4 doubles: tile width, warps, stage, ms) receives the
- * candidates tried, *n their number. */
+ * (tile width 4, 8, 16 x warps per block 2, 4 x stage 0, 1, 16, 64; the lattice: stage 0, 32; the cascade: stage 0;
+ * tile widths alone where the engine has a shape of its own) without moving the models, and keeps the fastest. A shape
+ * whose buffers do not fit is left out; where none fits or a trial fails, the shape stays as it was. rows (cap x 4
+ * doubles: tile width, warps, stage, ms) receives the candidates tried, *n their number. */
 bs_status bs_engine_autotune(bs_engine* e, int32_t windows, void* stream, double* rows, size_t cap, size_t* n);
 /* Kernel time of the last bs_engine_run's launches (ms, CUDA events on its stream). */
 bs_status bs_engine_last_ms(const bs_engine* e, double* ms);

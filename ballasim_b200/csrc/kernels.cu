@@ -1264,8 +1264,8 @@ __global__ void __launch_bounds__(128, 4) engine_cascade_kernel_free(EngineArgs 
 // cycles between a warp's issues waited for instructions; 0.7 in step). So the samples of a window are staged first (as
 // engine_kernel_staged does), and every turn each lane runs its next sub-step, whichever segment it stands in. One block
 // per multiprocessor with as many warps as the registers allow (at most 102 each). What is left is the wait at the
-// barrier for the turn's longest sub-step. 346x260, 60 windows: 12.0 ms against 16.4 free-running, 640x480 17.3 against
-// 23.5; 2 or 4 turns between barriers 13.4 and 14.9, a barrier before the comparator too 12.9, two blocks of 10 warps
+// barrier for the turn's longest sub-step. 346x260, 60 windows: 12.0 ms against 16.4 free-running, 640x480 16.3 against
+// 23.3; 2 or 4 turns between barriers 13.4 and 14.9, a barrier before the comparator too 12.9, two blocks of 10 warps
 // 11.4 and 19.4, warps free to go on to their next window 14.1.
 constexpr int kCascadeStage = 16;
 constexpr int kCascadeWarps = 20;
@@ -2304,7 +2304,8 @@ __device__ __noinline__ void feed_samples(PixelRegs* s, const PixelMapRegs* m, c
 // it. The shot chain stands at its next candidate that may be accepted, as there.
 // The block's warps take their trips in step (engine_cascade_kernel says why: 19 of the 28 cycles between a warp's issues
 // waited for instructions). 640x360 with noise, 30 windows: 12.6 ms with blocks of 32 warps (64 registers), 13.5 with
-// two of 12, 15.7 with one of 16 (free-running 15.7, and 17.6 with every sample fed to the pixel model).
+// two of 12, 15.7 with one of 16 (free-running 15.7, and 17.6 with every sample fed to the pixel model); over four seeds
+// 11.3 ms by a fixed stride of tiles, 10.6 with tiles taken as the blocks get to them (next_tiles).
 constexpr int kLearnedWarps = 32;
 struct alignas(16) LearnedWarpShared {
   uint16_t rows[32 * kSF];

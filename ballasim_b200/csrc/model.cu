@@ -1604,6 +1604,7 @@ struct Engine {
     if (cnt < 1) throw std::invalid_argument("engine: at least one sensor");
     if (cnt > 65535) throw std::invalid_argument("engine: at most 65535 sensors");
     rules = make_rules(r);
+    bool unlisted = false;  // some sensor's table is evaluated whole outside the split engine
     bool lattice_within = true;  // every sensor's lattice is expected to hold at most half the samples that the staged
                                  // form has room for (32: the other half for refinement)
     uint32_t tile0 = 0;
@@ -1629,6 +1630,7 @@ struct Engine {
       };
       within = within && expected(kSplitStageLog2);
       alike = alike && expected(std::max(kSplitStageLog2, rules.l_min));
+      unlisted = unlisted || fields.back()->f.n_blobs > kMaxListed;
       const bool edge = fs[i].kind == kFieldTanhEdge;
       const FieldDev& fd = fields.back()->f;
       mostly_short = mostly_short && 4 * static_cast<int64_t>(blobs_expected_past(
@@ -1660,13 +1662,15 @@ struct Engine {
     }
     total_tiles = tile0;
     // The launch shape until set_launch or the autotuner: the split engine for the instantaneous response, where the
-    // windows are expected to fit its stage or there are few tiles; else the streaming engine. Within the stage (64x48
+    // windows are expected to fit its stage, there are few tiles or very many blobs; else the streaming engine. Within the stage (64x48
     // to 1280x720, 1 to 160 windows, blobs of 60 and 120 px/s, edges up to 120, tolerances 1e-2 and 1e-4, with and
     // without noise) it takes 0.14 to 0.93 of the streaming engine's time. Past it (blobs of 300 to 2,000 px/s, or 60
     // with a tolerance of 1e-5, 346x260 to 1280x720) 0.75 to 2.5, but up to two tiles a multiprocessor (97x61, 128x72)
-    // 0.6 to 0.98; with a lattice past the stage already 1.0 to 1.08 there and 1.3 to 1.7 on larger frames.
+    // 0.6 to 0.98; with a lattice past the stage already 1.0 to 1.08 there and 1.3 to 1.7 on larger frames. A table of more
+    // blobs than the other engines list (256), which they evaluate whole: 0.02 to 0.7 past the stage (346x260 with 300
+    // to 1920x1080 with 3,000 blobs).
     const bool few = total_tiles <= 2u * static_cast<uint32_t>(sm_count()) && rules.l_min <= kSplitStageLog2;
-    if (cascade() == 0 && (within || few)) {
+    if (cascade() == 0 && (within || few || unlisted)) {
       stage = kStageSplit;
       stage_chosen = false;
     }

@@ -352,8 +352,8 @@ bs_status bs_engine_take_events(bs_engine* e, bs_event_columns* out);
  * pixels: the whole call in one launch). 64 and 1 are the instantaneous response's; the cascade takes 0, its noise
  * lattice 0 or 32, and with a learned proposal the stage has no effect (1 and 64 are refused).
  * An engine starts with 1 (instantaneous response) or 32 (lattice) where its fields' motion is expected to leave a
- * pixel's window within 16 samples, or with 1 on few tiles, else with 0; where the split engine's records (about 300
- * bytes a pixel) do not fit, it changes from 1 to 0.
+ * pixel's window within 16 samples, or with 1 on few tiles or under more than 256 blobs, else with 0; where the split
+ * engine's records (about 300 bytes a pixel) do not fit, it changes from 1 to 0.
  * The learned engine, and the cascade without the lattice where such windows are expected, run in a shape of their own:
  * one block per SM with as many warps as their tiles need, or on few tiles one warp per block. Warps per block and blocks
  * per SM have no effect on them, though get_launch reports them. */

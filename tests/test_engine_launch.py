@@ -73,13 +73,15 @@ def test_a_failed_autotune_leaves_the_shape(cuda_lib):
     ((346, 260), dict(), dict(l_min=5), 0),
     ((97, 61), dict(v_sigma=600.0), dict(), 1),  # few tiles
     ((97, 61), dict(), dict(l_min=5), 0),
+    ((346, 260), dict(n_blobs=256, v_sigma=600.0), dict(), 0),
+    ((346, 260), dict(n_blobs=257, v_sigma=600.0), dict(), 1),  # more blobs than the streaming engine lists
 ])
 def test_the_stage_an_engine_starts_with(cuda_lib, size, field, rules, stage):
     """The split engine where the windows are expected to fit its stage or the tiles are few, and the streaming engine's
     events whichever it is."""
     w, h = size
     r = replace(W.Rules(), **rules)
-    f = F.blobs(w, h, 9, 12, **field)
+    f = F.blobs(w, h, 9, **{"n_blobs": 12, **field})
     got = []
     for chosen in (None, 0):
         eng, m = engine("ideal", {**W.MISMATCH, **W.NOISE}, w, h, f, r)

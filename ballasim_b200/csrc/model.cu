@@ -1834,7 +1834,8 @@ struct Engine {
     t0_pin.p[0] = t0;
   }
 
-  // The split engine in one launch (split_solo_kernel) up to two tiles per resident warp (16 a multiprocessor): 346x260
+  // The split engine in one launch (split_solo_kernel) up to two tiles per resident warp (16 a multiprocessor by its
+  // registers; the line stays there when set_launch asks for fewer): 346x260
   // (2,811 tiles, 239 windows) 4.44 against 5.88 ms of engine time with two launches per window, 333x187 with noise
   // (1,974 tiles, 37 windows) 1.25 against 1.60, 640x480 (9,600 tiles) 3.33 against 3.37, 1280x720 12.5 against 11.8.
   bool split_solo() const { return total_tiles <= 2u * 16u * static_cast<uint32_t>(sm_count()); }
